@@ -59,34 +59,29 @@ constexpr int kRA2 = JHTB_RA2;  // adjoint, spin 2
 #endif
 constexpr int kTcMaps = JHTB_TC_MAPS;  // maps per tensor-core pass (N = 4 * maps per GEMM)
 
-// FFT: largest power-of-two length handled in one CTA's shared memory.
-constexpr int kFftMax = 8192;    // largest power-of-two ring handled by the direct path per piece plan
-constexpr int kTwLen = 32768;    // twiddle table length: every FFT and split length divides it
-constexpr int kFftPiece = 4096;  // largest FFT held in shared memory; longer ones run in pieces
-constexpr int kFftLogMax = 13;
+// Azimuthal stage (ringfft.cu).
+constexpr int kTwLen = 32768;      // twiddle table length: every FFT length divides it
+constexpr int kFftPiece = 4096;    // points of one FFT of the 256-thread kernels
+constexpr int kRingThreads = 256;  // threads of a ring CTA
+constexpr int kSmallRing = 128;    // rings up to this length run as a plain sum
 
-// Ring FFT modes: kDirect (N a power of two), kBluestein (chirp-z of length N), kSplit4
-// (N = 4 i: four chirp-z transforms of length i and a radix-4 combination).
-enum RingMode : int { kDirect = 0, kBluestein = 1, kSplit4 = 2 };
+// Classes of work units: kClsSmall, or kClsDirect / kClsChirp plus the FFT's log2 length.
+enum RingClass : int { kClsSmall = 0, kClsDirect = 0x100, kClsChirp = 0x200 };
+// One CTA's work: rings [ring, ring + n) (n > 1 where several fit), its first piece.
+struct RingUnit {
+    int cls, ring, piece, n;
+};
+// Columns of i factors each per chirp length i = N / 4 (ring_table_kernel)
+enum RingCol : int { kColAdjIn = 0, kColSynth = 4, kColAdjOut = 8, kRingCols = 12 };
 
 struct RingDesc {
-    int N;          // pixels in the ring
-    int mode;       // RingMode
-    int P;          // FFT length: N (direct), Bluestein length (power of two >= 2N-1), or for
-                    // kSplit4 the Bluestein length of the quarter ring (power of two >= N/2-1)
-    int Q;          // pieces of P / Q <= kFftPiece points (1, 2, 4 or 8) in the piecewise path
-    long long start;   // first pixel
-    long long bh_off;  // offset (complex units) of this length's chirp spectrum
-    double phi0;       // azimuth of the first pixel
+    int N;               // pixels in the ring
+    int shifted;         // azimuth of the first pixel: pi / N (1) or 0
+    long long start;     // first pixel
+    long long mirror;    // first pixel of the mirror ring (spin 0 pairs), -1 for the equator
+    long long ctab_off;  // offset (complex units) of this chirp length's factor columns
+    long long bh_off;    // offset (complex units) of its chirp spectrum
 };
-
-// Pieces a ring's transform runs in, one CTA each (1: the whole ring in one CTA): a
-// power-of-two ring above kFftPiece points in N / kFftPiece pieces, a kSplit4 ring in 4.
-__host__ __device__ __forceinline__ int ring_pieces(const RingDesc &rd) {
-    if (rd.mode == kSplit4) return 4;
-    if (rd.mode == kDirect && rd.N > kFftPiece && 2 * rd.N <= kTwLen) return rd.N / kFftPiece;
-    return 1;
-}
 
 // Per-m seed parameters.  Spin 0: lf = theta-independent log|lambda_mm|,
 // sign = (-1)^m, pc = ps = 0.  Spin +-2: log|d^{lmin}_{-m,+-2}| = lf + pc log cos(t/2)
@@ -126,8 +121,10 @@ struct Plan {
     double *d_logsh;    // [T] log sin(theta/2)
     RingDesc *d_rings;  // [nrings]
     double2 *d_tw;      // [kTwLen] exp(-2 pi i k / kTwLen)
-    double2 *d_bh;      // Bluestein chirp spectra, FFT_P(conj(w))/P, per distinct length
-    long long bh_len;
+    double2 *d_bh;      // chirp spectra, FFT_P(conj(w))/P, per distinct chirp length
+    double2 *d_ctab;    // chirp, piece and ring-phase factors per distinct chirp length
+    double2 *d_belt;    // [2 belt_n] e^{i pi a / belt_n} of a power-of-two belt
+    int belt_n;         // points of the belt rings where they run as power-of-two FFTs, else 0
 
     // recursion tables (device), packed like the alm
     SeedParam *d_seed;  // [M]
@@ -200,18 +197,14 @@ struct Plan {
     int ring_t0, ring_t1;
     int nsynth;           // entries of d_synth_order (items inside the range)
     int tc_norder;        // entries of d_tc_order
-    // rings of the plan's range by kernel: ring_small (one 256-thread CTA per ring, pieces
-    // through global scratch above kFftPiece points) and ring_piece ((ring << 3 | piece)
-    // work units of the rings that run in pieces, ring_pieces() > 1)
-    int *d_ring_small, *d_ring_piece;
-    int nring_small, nring_piece;
-    std::vector<unsigned char> h_ring_pieces;  // [ring] pieces of its transform (1: the one-CTA kernel)
+    // work units of the plan's range in launch order, then those of the 512-thread kernel
+    RingUnit *d_ring_units;
+    int nunit, nunit_long;
+    std::vector<int> h_ring_n;               // [ring] pixels (empty for a ring-set plan)
     std::vector<int> h_lw, h_a_lw, h_tc_lw;  // start l per item, kept for re-sorting
 
     // workspace
     double2 *d_F;       // [chunk][nchan][nrings][M] ring spectra
-    double2 *d_W;       // [chunk][npix] ring scratch rows of the split transforms
-    double2 *d_W2;      // [chunk][npix] second scratch row (phased input / piece sums)
     double *d_scratch;  // small reduction scratch
     int chunk;          // maps per workspace pass
     size_t bytes;
@@ -232,23 +225,26 @@ constexpr int kInjectStall = JHTB_FAULT_STALL;
 enum Stage : int { kStageLegSynth = 0, kStageRingSynth = 1, kStageRingAdj = 2, kStageLegAdj = 3, kNumStages = 4 };
 
 // kernels launchers (return 0 or a jhtb status)
-int launch_legendre_synth(const Plan &p, const double2 *alm, double2 *F, int nb, cudaStream_t s);
-int launch_legendre_adjoint(const Plan &p, const double2 *F, double2 *alm, int nb, cudaStream_t s);
+// `paired` (spin 0): the ring spectra of a northern ring and its mirror are exchanged as
+// P = north + i south (row t) and M = north - i south (the mirror's row), the form the
+// azimuthal stage transforms; otherwise as the two rings' own coefficients
+int launch_legendre_synth(const Plan &p, const double2 *alm, double2 *F, int nb, bool paired, cudaStream_t s);
+int launch_legendre_adjoint(const Plan &p, const double2 *F, double2 *alm, int nb, bool paired, cudaStream_t s);
 int launch_ring_synth(const Plan &p, const double2 *F, double *maps, int nb, cudaStream_t s);
-int launch_ring_adjoint(const Plan &p, const double *maps, double2 *F, double2 *W, int nb,
-                        cudaStream_t s);
+int launch_ring_adjoint(const Plan &p, const double *maps, double2 *F, int nb, cudaStream_t s);
 int launch_start_states(const Plan &p, cudaStream_t s);
 int launch_start_states_r(const Plan &p, int R, int ntiles, int *lw, double2 *st, int *stsc, cudaStream_t s);
-int launch_tc_synth(const Plan &p, const double2 *alm, double2 *F, int nb, cudaStream_t s);
-int launch_tc_adjoint(const Plan &p, const double2 *F, double2 *alm, int nb, cudaStream_t s);
+int launch_tc_synth(const Plan &p, const double2 *alm, double2 *F, int nb, bool paired, cudaStream_t s);
+int launch_tc_adjoint(const Plan &p, const double2 *F, double2 *alm, int nb, bool paired, cudaStream_t s);
 size_t tc_synth_chunk_bytes(int spin);
 int launch_tca_block_states(const Plan &p, cudaStream_t s);
 constexpr int kTcaLB = 128;       // degrees per tensor-core adjoint item (= MMA M)
 constexpr int kTcaSeg = 4;        // recursion segments per item (independent chains per thread)
 constexpr int kTcaMaps = 16;      // maps per tensor-core adjoint group
 constexpr int kTcaBStage = 12288; // bytes of one ring chunk's BF16x3 tiles (2 x 3 x 64 x 16 x 2)
-int launch_bluestein_setup(const Plan &p, const int *lengths, const long long *offs, int nlen,
-                           cudaStream_t s);
+// chirp lengths sorted by their FFT length, count[log2 P] of each (device arrays)
+int launch_ring_tables(const Plan &p, const int *lens, const long long *ctab_offs, const long long *bh_offs,
+                       const int (&count)[14], cudaStream_t s);
 constexpr int kRingGranule = 256;  // alignment of ring ranges: a multiple of every tile width
 
 __host__ __device__ inline long long alm_index(long long l, long long m, long long lmax) {

@@ -61,6 +61,7 @@ constexpr unsigned kFull = 0xffffffffu;
 
 struct LegParams {
     int lmax, T, nrings, M, nside;
+    int paired;               // spin 0: rows exchanged as P = north + i south, M = north - i south
     long long K;
     const double *x, *logsin, *logch, *logsh;
     const SeedParam *seed;
@@ -85,6 +86,7 @@ LegParams make_params(const Plan &p) {
     q.nrings = p.nrings;
     q.M = p.M;
     q.nside = p.nside;
+    q.paired = 0;
     q.K = p.K;
     q.x = p.d_x;
     q.logsin = p.d_logsin;
@@ -329,9 +331,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) synth0_kernel(LegParams p
         for (int r = 0; r < R; ++r) {
             const int t = tile * 32 * R + r * 32 + lane;
             if (t < p.T && JHTB_IN((long long)(p.nrings - 1 - t) * p.M + m, (long long)p.nrings * p.M, 202)) {
-                F[(size_t)t * p.M + m] = make_double2(Ar[r] + Br[r], Ai[r] + Bi[r]);
-                if (t < p.T - 1)
-                    F[(size_t)(p.nrings - 1 - t) * p.M + m] = make_double2(Ar[r] - Br[r], Ai[r] - Bi[r]);
+                double2 n = make_double2(Ar[r] + Br[r], Ai[r] + Bi[r]);
+                double2 sth = make_double2(Ar[r] - Br[r], Ai[r] - Bi[r]);
+                if (p.paired) spin0_pair(n, sth, m == 0, t < p.T - 1);
+                F[(size_t)t * p.M + m] = n;
+                if (t < p.T - 1) F[(size_t)(p.nrings - 1 - t) * p.M + m] = sth;
             }
         }
     }
@@ -579,7 +583,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj0MinBlocks) adj0_kern
                 if (t < p.T && JHTB_IN((long long)(p.nrings - 1 - t) * p.M + m, (long long)p.nrings * p.M, 203)) {
                     x[r] = p.x[t];
                     vn = V[(size_t)t * p.M + m];
-                    if (t < p.T - 1) vs = V[(size_t)(p.nrings - 1 - t) * p.M + m];
+                    if (t < p.T - 1) {
+                        vs = V[(size_t)(p.nrings - 1 - t) * p.M + m];
+                        if (p.paired) spin0_unpair(vn, vs);
+                    }
                 }
                 // b_l = sum_t lambda (Vn + (-1)^l (-1)^m V_south)  (_recursion.py:472-497)
                 UA[r] = make_double2(vn.x + vs.x, vn.y + vs.y);
@@ -901,10 +908,11 @@ int launch_start_states_r(const Plan &p, int R, int ntiles, int *lw, double2 *st
     return JHTB_OK;
 }
 
-int launch_legendre_synth(const Plan &p, const double2 *alm, double2 *F, int nb, cudaStream_t s) {
+int launch_legendre_synth(const Plan &p, const double2 *alm, double2 *F, int nb, bool paired, cudaStream_t s) {
     if (nb <= 0) return JHTB_OK;
     JHTB_CUDA_TRY(cudaMemsetAsync(p.d_counter, 0, sizeof(unsigned), s));
     LegParams q = make_params(p);
+    q.paired = paired;
     if (p.spin == 0) {
         auto k = synth0_kernel<kR0>;
         k<<<leg_grid(p, k), kWarpsPerBlock * 32, 0, s>>>(q, alm, F, nb);
@@ -916,10 +924,11 @@ int launch_legendre_synth(const Plan &p, const double2 *alm, double2 *F, int nb,
     return JHTB_OK;
 }
 
-int launch_legendre_adjoint(const Plan &p, const double2 *F, double2 *alm, int nb, cudaStream_t s) {
+int launch_legendre_adjoint(const Plan &p, const double2 *F, double2 *alm, int nb, bool paired, cudaStream_t s) {
     if (nb <= 0) return JHTB_OK;
     JHTB_CUDA_TRY(cudaMemsetAsync(p.d_counter, 0, sizeof(unsigned), s));
     LegParams q = make_params(p);
+    q.paired = paired;
     q.ntiles = p.a_ntiles;
     q.lw = p.d_a_lw;
     q.st = p.d_a_st;

@@ -44,12 +44,6 @@ namespace {
 
 bool is_pow2(long long n) { return n > 0 && (n & (n - 1)) == 0; }
 
-long long next_pow2(long long n) {
-    long long p = 1;
-    while (p < n) p <<= 1;
-    return p;
-}
-
 // Compensated sum, for the theta-independent log of the sectoral seed.
 double kahan_log_const(int m) {
     double s = -0.5 * std::log(4.0 * M_PI), c = 0.0;
@@ -89,8 +83,8 @@ void free_plan(Plan *p) {
     if (!p) return;
     void *ptrs[] = {p->d_x,     p->d_logsin, p->d_logch, p->d_logsh,   p->d_rings, p->d_tw,
                     p->d_bh,    p->d_seed,   p->d_alpha, p->d_gamma,   p->d_cnorm, p->d_F,
-                    p->d_W,     p->d_W2,     p->d_scratch, p->d_lw, p->d_st, p->d_stsc, p->d_synth_order,
-                    p->d_adj_order, p->d_adj_tiles, p->d_counter, p->d_part, p->d_err, p->d_ring_small, p->d_ring_piece};
+                    p->d_ctab,  p->d_belt,   p->d_scratch, p->d_lw, p->d_st, p->d_stsc, p->d_synth_order,
+                    p->d_adj_order, p->d_adj_tiles, p->d_counter, p->d_part, p->d_err, p->d_ring_units};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (p->a_owns_tables) {
@@ -220,36 +214,77 @@ int build_orders(Plan *p) {
         p->d_tca_items = nullptr;
         if ((rc = upload(&p->d_tca_items, items, bytes))) return rc;
     }
-    if (!p->h_ring_pieces.empty() && (rc = build_ring_lists(p, bytes))) return rc;
+    if (!p->h_ring_n.empty() && (rc = build_ring_lists(p, bytes))) return rc;
     return JHTB_OK;
 }
 
-// Azimuthal stage: the range's northern rings and their southern mirrors, split by the
-// kernel that transforms them (whole rings in one CTA; (ring << 3 | piece) units of the
-// rings that run in pieces, a ring's pieces adjacent so that they read its data from L2
-// together); within each list the rings keep their order.
+// log2 of the chirp-z length of a ring of N = 4 i points: P >= 2 i - 1 and at least 128.
+int chirp_log2(int n) {
+    int lg = 7;
+    while ((1LL << lg) < 2LL * (n / 4) - 1) ++lg;
+    return lg;
+}
+
+// Azimuthal stage: the work units (ringfft.cu) of the range's rings.  Spin 2 transforms every
+// northern ring and its southern mirror, spin 0 one pair per half-grid ring.  A ring's pieces
+// are adjacent, so that they read its data from L2 together; rings of the same class that
+// share a CTA are consecutive.  Launch order: the short chirp rings first (few CTAs whose
+// threads each fold many aliases), then by falling FFT length, the small rings last.
 int build_ring_lists(Plan *p, size_t &bytes) {
     const int T = p->T, t0 = p->ring_t0, t1 = p->ring_t1;
-    int rc;
-    for (int **q : {&p->d_ring_small, &p->d_ring_piece})
-        if (*q) cudaFree(*q);
-    p->d_ring_small = p->d_ring_piece = nullptr;
-    std::vector<int> small, whole;
-    auto add = [&](int r) { (p->h_ring_pieces[r] > 1 ? whole : small).push_back(r); };
+    if (p->d_ring_units) cudaFree(p->d_ring_units);
+    p->d_ring_units = nullptr;
+    std::vector<int> list;
     for (int t = t0; t < t1; ++t) {
-        add(t);
-        if (t < T - 1) add(p->nrings - 1 - t);
+        list.push_back(t);
+        if (p->spin && t < T - 1) list.push_back(p->nrings - 1 - t);
     }
-    std::sort(small.begin(), small.end());
-    std::sort(whole.begin(), whole.end());
-    std::vector<int> pieces;
-    for (int r : whole)
-        for (int s = 0; s < p->h_ring_pieces[r]; ++s) pieces.push_back(r << 3 | s);
-    p->nring_small = (int)small.size();
-    p->nring_piece = (int)pieces.size();
-    if ((rc = upload(&p->d_ring_small, small, bytes))) return rc;
-    if ((rc = upload(&p->d_ring_piece, pieces, bytes))) return rc;
-    return JHTB_OK;
+    std::sort(list.begin(), list.end());
+    std::vector<RingUnit> units, longs;
+    for (size_t q = 0; q < list.size();) {
+        const int r = list[q], n = p->h_ring_n[r];
+        RingUnit u{kClsSmall, r, 0, 1};
+        int pieces = 1, step = 1, group = 1;  // units per ring, pieces per unit, rings per unit
+        if (n > kSmallRing && n == p->belt_n) {
+            const int len = std::min(n, kFftPiece);
+            int lg = 0;
+            while ((1 << lg) < len) ++lg;
+            u.cls = kClsDirect + lg;
+            pieces = n / len;
+            group = pieces > 1 ? 1 : kFftPiece / len;
+        } else if (n > kSmallRing) {
+            const int lg = chirp_log2(n);
+            u.cls = kClsChirp + lg;
+            pieces = 4;
+            step = lg <= 10 ? 4 : (lg == 11 ? 2 : 1);
+            group = lg <= 10 ? 1024 >> lg : 1;
+        }
+        size_t e = q + 1;
+        auto same = [&](int r2) {
+            const int n2 = p->h_ring_n[r2];
+            if (u.cls == kClsSmall || n2 <= kSmallRing) return false;
+            if (u.cls < kClsChirp) return n2 == n;
+            return n2 != p->belt_n && kClsChirp + chirp_log2(n2) == u.cls;
+        };
+        while (e < list.size() && (int)(e - q) < group && list[e] == list[e - 1] + 1 && same(list[e])) ++e;
+        u.n = (int)(e - q);
+        for (int s = 0; s < pieces; s += step) {
+            u.piece = s;
+            (u.cls == kClsChirp + 13 ? longs : units).push_back(u);
+        }
+        q = e;
+    }
+    auto key = [](const RingUnit &u) {
+        if (u.cls == kClsSmall) return 100;
+        const int lg = u.cls & 0xff;
+        if (u.cls >= kClsChirp) return lg <= 8 ? lg - 7 : 20 - lg;
+        return 50 - lg;
+    };
+    std::stable_sort(units.begin(), units.end(), [&](const RingUnit &a, const RingUnit &b) { return key(a) < key(b); });
+    p->nunit = (int)units.size();
+    p->nunit_long = (int)longs.size();
+    units.insert(units.end(), longs.begin(), longs.end());
+    return upload(&p->d_ring_units, units, bytes);
 }
 
 int build_plan(Plan *p, const jhtb_host_tables *ht) {
@@ -516,59 +551,42 @@ int build_plan(Plan *p, const jhtb_host_tables *ht) {
     p->ring_t1 = T;
     if ((rc = build_orders(p))) return rc;
 
-    // ---- ring FFT descriptors (HEALPix plans; a ring-set plan stops at the ring spectra) ----
+    // ---- ring descriptors (HEALPix plans; a ring-set plan stops at the ring spectra) --------
     std::vector<RingDesc> rings(p->rings_only ? 0 : nr);
-    std::map<long long, long long> bh_offset;  // Bluestein length -> offset
-    std::vector<int> blens;
-    std::vector<long long> boffs;
-    long long bh_len = 0;
+    std::vector<int> clens;           // distinct chirp lengths, sorted (so also by FFT length)
+    std::vector<long long> coffs, boffs;
+    int ccount[14] = {};
     if (!p->rings_only) {
+        p->belt_n = is_pow2(nside) && 4 * nside > kSmallRing ? 4 * nside : 0;
+        for (int r = 0; r < nr; ++r)
+            if (npr[r] > kSmallRing && npr[r] != p->belt_n) clens.push_back((int)npr[r] / 4);
+        std::sort(clens.begin(), clens.end());
+        clens.erase(std::unique(clens.begin(), clens.end()), clens.end());
+        long long co = 0, bo = 0;
+        std::map<int, int> at;
+        for (int i : clens) {
+            at[i] = (int)coffs.size();
+            coffs.push_back(co);
+            boffs.push_back(bo);
+            const int lg = chirp_log2(4 * i);
+            ++ccount[lg];
+            co += (long long)kRingCols * i;
+            bo += 1LL << lg;
+        }
+        p->h_ring_n.resize(nr);
         for (int r = 0; r < nr; ++r) {
             RingDesc &d = rings[r];
             d.N = (int)npr[r];
+            d.shifted = phi0[r] != 0.0;
             d.start = start[r];
-            d.phi0 = phi0[r];
-            if (is_pow2(d.N) && d.N <= 8 * kFftPiece) {
-                d.mode = kDirect;
-                d.P = d.N;
-                d.Q = std::max(1, d.N / kFftPiece);
-                d.bh_off = 0;
-            } else if (d.N % 4 == 0 && 2LL * d.N - 1 > kFftPiece && 2LL * (d.N / 4) - 1 <= kFftPiece) {
-                // too long for one shared-memory chirp-z: four of length N / 4 (polar cap rings)
-                const int qn = d.N / 4;
-                d.mode = kSplit4;
-                d.P = (int)next_pow2(2LL * qn - 1);
-                d.Q = 1;
-                auto it = bh_offset.find(qn);
-                if (it == bh_offset.end()) {
-                    bh_offset[qn] = bh_len;
-                    blens.push_back(qn);
-                    boffs.push_back(bh_len);
-                    d.bh_off = bh_len;
-                    bh_len += d.P;
-                } else {
-                    d.bh_off = it->second;
-                }
-            } else {
-                d.mode = kBluestein;
-                d.P = (int)next_pow2(2LL * d.N - 1);
-                d.Q = std::max(1, d.P / kFftPiece);
-                if (d.Q > 8) return fail(JHTB_ERR_UNSUPPORTED, "ring length too large (nside > 4096)");
-                auto it = bh_offset.find(d.N);
-                if (it == bh_offset.end()) {
-                    bh_offset[d.N] = bh_len;
-                    blens.push_back(d.N);
-                    boffs.push_back(bh_len);
-                    d.bh_off = bh_len;
-                    bh_len += d.P;
-                } else {
-                    d.bh_off = it->second;
-                }
-            }
+            d.mirror = r < T - 1 ? start[nr - 1 - r] : -1;
+            const auto it = at.find(d.N / 4);
+            const bool chirp = d.N > kSmallRing && d.N != p->belt_n && it != at.end();
+            d.ctab_off = chirp ? coffs[it->second] : 0;
+            d.bh_off = chirp ? boffs[it->second] : 0;
+            p->h_ring_n[r] = d.N;
         }
         if ((rc = upload(&p->d_rings, rings, bytes))) return rc;
-        p->h_ring_pieces.assign(nr, 1);
-        for (int r = 0; r < nr; ++r) p->h_ring_pieces[r] = (unsigned char)ring_pieces(rings[r]);
         if ((rc = build_ring_lists(p, bytes))) return rc;
 
         std::vector<double2> tw(kTwLen);
@@ -577,10 +595,10 @@ int build_plan(Plan *p, const jhtb_host_tables *ht) {
             tw[k] = make_double2((double)cosl(a), (double)sinl(a));
         }
         if ((rc = upload(&p->d_tw, tw, bytes))) return rc;
-
-        p->bh_len = bh_len;
-        JHTB_CUDA_TRY(cudaMalloc((void **)&p->d_bh, sizeof(double2) * std::max(bh_len, 1LL)));
-        bytes += sizeof(double2) * std::max(bh_len, 1LL);
+        JHTB_CUDA_TRY(cudaMalloc((void **)&p->d_bh, sizeof(double2) * std::max(bo, 1LL)));
+        JHTB_CUDA_TRY(cudaMalloc((void **)&p->d_ctab, sizeof(double2) * std::max(co, 1LL)));
+        JHTB_CUDA_TRY(cudaMalloc((void **)&p->d_belt, sizeof(double2) * std::max(2 * p->belt_n, 1)));
+        bytes += sizeof(double2) * (std::max(bo, 1LL) + std::max(co, 1LL) + std::max(2 * p->belt_n, 1));
     }
 
     // ---- workspace --------------------------------------------------------------------------
@@ -593,30 +611,21 @@ int build_plan(Plan *p, const jhtb_host_tables *ht) {
         JHTB_CUDA_TRY(cudaMalloc((void **)&p->d_part, part));
         bytes += part;
     }
-    bool need_w = false;
-    for (int r = 0; r < (int)rings.size(); ++r) need_w |= p->h_ring_pieces[r] == 1 && rings[r].Q > 1;
-    if (need_w) {
-        JHTB_CUDA_TRY(cudaMalloc((void **)&p->d_W, sizeof(double2) * (size_t)p->npix * p->chunk));
-        JHTB_CUDA_TRY(cudaMalloc((void **)&p->d_W2, sizeof(double2) * (size_t)p->npix * p->chunk));
-        bytes += 2 * sizeof(double2) * (size_t)p->npix * p->chunk;
-    }
     JHTB_CUDA_TRY(cudaMalloc((void **)&p->d_scratch, 4096 * sizeof(double)));
     bytes += 4096 * sizeof(double);
 
-    // ---- Bluestein chirp spectra (device) -------------------------------------------------------
-    if (!blens.empty()) {
+    // ---- chirp spectra and factor columns (device) ----------------------------------------------
+    if (!p->rings_only) {
         int *d_len = nullptr;
-        long long *d_off = nullptr;
-        JHTB_CUDA_TRY(cudaMalloc((void **)&d_len, sizeof(int) * blens.size()));
-        JHTB_CUDA_TRY(cudaMalloc((void **)&d_off, sizeof(long long) * boffs.size()));
-        JHTB_CUDA_TRY(cudaMemcpy(d_len, blens.data(), sizeof(int) * blens.size(), cudaMemcpyHostToDevice));
-        JHTB_CUDA_TRY(cudaMemcpy(d_off, boffs.data(), sizeof(long long) * boffs.size(), cudaMemcpyHostToDevice));
-        rc = launch_bluestein_setup(*p, d_len, d_off, (int)blens.size(), 0);
+        long long *d_coff = nullptr, *d_boff = nullptr;
+        size_t tmp = 0;
+        if (!(rc = upload(&d_len, clens, tmp)) && !(rc = upload(&d_coff, coffs, tmp)) && !(rc = upload(&d_boff, boffs, tmp)))
+            rc = launch_ring_tables(*p, d_len, d_coff, d_boff, ccount, 0);
         cudaError_t e = cudaDeviceSynchronize();
-        cudaFree(d_len);
-        cudaFree(d_off);
+        for (void *q : {(void *)d_len, (void *)d_coff, (void *)d_boff})
+            if (q) cudaFree(q);
         if (rc) return rc;
-        if (e != cudaSuccess) return cuda_fail(e, "bluestein setup");
+        if (e != cudaSuccess) return cuda_fail(e, "ring tables");
     }
     return JHTB_OK;
 }
@@ -762,8 +771,8 @@ int jhtb_legendre_synthesis(jhtb_plan *plan, const void *alm, void *rings, int b
         const int nb = std::min(p.chunk, batch - b0);
         StageTimer t(p, s, kStageLegSynth);
         const int rc = p.precision == JHTB_PREC_BF16X3
-                           ? launch_tc_synth(p, a + (size_t)b0 * p.ncomp * p.K, F + (size_t)b0 * f_map, nb, s)
-                           : launch_legendre_synth(p, a + (size_t)b0 * p.ncomp * p.K, F + (size_t)b0 * f_map, nb, s);
+                           ? launch_tc_synth(p, a + (size_t)b0 * p.ncomp * p.K, F + (size_t)b0 * f_map, nb, false, s)
+                           : launch_legendre_synth(p, a + (size_t)b0 * p.ncomp * p.K, F + (size_t)b0 * f_map, nb, false, s);
         if (rc) return rc;
     }
     return JHTB_OK;
@@ -781,8 +790,8 @@ int jhtb_legendre_adjoint(jhtb_plan *plan, const void *rings, void *alm, int bat
         const int nb = std::min(p.chunk, batch - b0);
         StageTimer t(p, s, kStageLegAdj);
         const int rc = p.precision == JHTB_PREC_BF16X3
-                           ? launch_tc_adjoint(p, F + (size_t)b0 * f_map, a + (size_t)b0 * p.ncomp * p.K, nb, s)
-                           : launch_legendre_adjoint(p, F + (size_t)b0 * f_map, a + (size_t)b0 * p.ncomp * p.K, nb, s);
+                           ? launch_tc_adjoint(p, F + (size_t)b0 * f_map, a + (size_t)b0 * p.ncomp * p.K, nb, false, s)
+                           : launch_legendre_adjoint(p, F + (size_t)b0 * f_map, a + (size_t)b0 * p.ncomp * p.K, nb, false, s);
         if (rc) return rc;
     }
     return JHTB_OK;
@@ -813,8 +822,8 @@ int jhtb_synthesis(jhtb_plan *plan, const void *alm, void *maps, int batch, void
         int rc;
         {
             StageTimer t(p, s, kStageLegSynth);
-            rc = p.precision == JHTB_PREC_BF16X3 ? launch_tc_synth(p, a + (size_t)b0 * p.ncomp * p.K, p.d_F, nb, s)
-                                                 : launch_legendre_synth(p, a + (size_t)b0 * p.ncomp * p.K, p.d_F, nb, s);
+            rc = p.precision == JHTB_PREC_BF16X3 ? launch_tc_synth(p, a + (size_t)b0 * p.ncomp * p.K, p.d_F, nb, true, s)
+                                                 : launch_legendre_synth(p, a + (size_t)b0 * p.ncomp * p.K, p.d_F, nb, true, s);
         }
         if (rc) return rc;
         {
@@ -840,13 +849,13 @@ int jhtb_adjoint_synthesis(jhtb_plan *plan, const void *maps, void *alm, int bat
         int rc;
         {
             StageTimer t(p, s, kStageRingAdj);
-            rc = launch_ring_adjoint(p, m + (size_t)b0 * p.ncomp * p.npix, p.d_F, p.d_W, nb, s);
+            rc = launch_ring_adjoint(p, m + (size_t)b0 * p.ncomp * p.npix, p.d_F, nb, s);
         }
         if (rc) return rc;
         {
             StageTimer t(p, s, kStageLegAdj);
-            rc = p.precision == JHTB_PREC_BF16X3 ? launch_tc_adjoint(p, p.d_F, a + (size_t)b0 * p.ncomp * p.K, nb, s)
-                                                 : launch_legendre_adjoint(p, p.d_F, a + (size_t)b0 * p.ncomp * p.K, nb, s);
+            rc = p.precision == JHTB_PREC_BF16X3 ? launch_tc_adjoint(p, p.d_F, a + (size_t)b0 * p.ncomp * p.K, nb, true, s)
+                                                 : launch_legendre_adjoint(p, p.d_F, a + (size_t)b0 * p.ncomp * p.K, nb, true, s);
         }
         if (rc) return rc;
     }

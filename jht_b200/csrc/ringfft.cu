@@ -1,100 +1,70 @@
 // Azimuthal stage: per-ring phase shift, m -> k fold and length-N DFT (sm_100a).
 //
 // jht (healpix.py:280-355) groups rings by length and emits one FFT per distinct
-// length, with scatter-adds for the m -> k fold.  Here a CTA owns a ring (or a piece of one):
-//   synthesis  D[k] = sum_{m = k mod N} Fp_m e^{i m phi0} + sum_{m>=1, -m = k mod N} conj(Fm_m e^{i m phi0})
-//              out[j] = sum_k D[k] e^{+2 pi i jk/N}      (real part: spin 0; Q + iU: spin 2)
-//   adjoint    W[k] = sum_j v[j] e^{-2 pi i jk/N};  V[m] = W[m mod N] e^{-i m phi0}
-//              (spin 2 also Vm[m] = conj(W[-m mod N]) e^{-i m phi0})
-// The fold is a gather (each k collects its own m's), never a scatter.  Power-of-two
-// rings use an in-place Stockham FFT in shared memory (radix-16 passes held in
-// registers, natural order in and out, a padded layout against bank conflicts; 70 KB of
-// shared memory per CTA, two CTAs per SM); every other length uses Bluestein's chirp-z
-// with an exact (n^2 mod 2N) chirp argument (_azimuth.py:150-191) at a power-of-two length
-// P >= 2N-1.  Rings whose transform exceeds 4096 points run as independent pieces, one CTA
-// per output residue class (decimation in frequency on the input, no data exchange): the
-// power-of-two belt rings in N / 4096 pieces and the long polar-cap rings (N = 4 qn) as four
-// chirp-z pieces of length qn; only chirp-z lengths above 16384 (cap rings at nside > 2048)
-// are split inside one CTA through the ring's scratch rows.
+// length, with scatter-adds for the m -> k fold.  Here a transform takes two rows of ring
+// spectra, P and M, to two real pixel streams x, y (and back):
+//   synthesis  D[k] = sum_{m = k mod N} P_m e^{i m phi0} + sum_{m>=1, -m = k mod N} conj(M_m e^{i m phi0})
+//              x[j] + i y[j] = sum_k D[k] e^{+2 pi i jk/N}
+//   adjoint    W[k] = sum_j (x[j] + i y[j]) e^{-2 pi i jk/N}
+//              P_m = W[m mod N] e^{-i m phi0},  M_m = conj(W[-m mod N]) e^{-i m phi0}
+// Spin 2: P and M are the +2 and -2 channels of one ring, x = Q and y = U.  Spin 0: one
+// complex transform serves a northern ring and its southern mirror (same length and
+// azimuth): the rows hold P = F_north + i F_south and M = F_north - i F_south (the Legendre
+// kernels write and read that form), x is the northern ring and y the southern one, so the
+// stage runs half the transforms of one real ring each.
+//
+// On the HEALPix grid phi0 is 0 or pi / N and N = 4 i (healpix.py:107-140), so every factor is
+// e^{i pi a / N} for an integer a.  A ring runs as pieces, one transform per output residue
+// class (decimation in frequency on the input):
+//   direct   N a power of two (the belt at a power-of-two nside): Q = N / 4096 pieces (1 up
+//            to 4096 points) of one FFT each;
+//   chirp    every other ring: four pieces of length i, each a chirp-z transform
+//            (_azimuth.py:150-191) of P >= 2 i - 1 points: FFT, chirp spectrum, inverse FFT;
+//   small    N <= 128: a plain sum over k with the ring's 2 N roots of unity in shared memory.
+// An FFT keeps 16 points per thread in registers: radix-16 passes (one smaller last pass),
+// decimation in frequency forward and its transpose backward, so that neither needs a
+// reordering pass and the chirp spectrum is applied in registers between the two; a pass
+// writes back where it read, so an exchange costs one barrier.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "jhtb_internal.cuh"
 
 namespace jhtb {
 namespace {
 
-#ifndef JHTB_FFT_THREADS
-#define JHTB_FFT_THREADS 256
-#endif
-#ifndef JHTB_FFT_MINB
-#define JHTB_FFT_MINB 2
-#endif
-constexpr int kFftThreads = JHTB_FFT_THREADS;  // threads per ring CTA
-constexpr int kFftMinBlocks = JHTB_FFT_MINB;   // resident ring CTAs per SM (4096-point buffers)
-#ifndef JHTB_PIECE_MINB
-#define JHTB_PIECE_MINB 2
-#endif
-constexpr int kPieceMinBlocks = JHTB_PIECE_MINB;  // resident CTAs per SM of the piece kernels
-#ifndef JHTB_PIECE_U
-#define JHTB_PIECE_U 4
-#endif
-constexpr int kUP = JHTB_PIECE_U;  // elements per thread whose gathers the piece kernels issue together
-
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
+}
+__device__ __forceinline__ double2 cmulc(double2 a, double2 b) {  // a conj(b)
+    return make_double2(fma(a.x, b.x, a.y * b.y), fma(a.y, b.x, -a.x * b.y));
 }
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double2 conjd(double2 a) { return make_double2(a.x, -a.y); }
+__device__ __forceinline__ double2 zero2() { return make_double2(0.0, 0.0); }
 
-__device__ __forceinline__ int ilog2i(int n) { return 31 - __clz(n); }
-
-// e^{i pi (a / N + 2 c / P)} for integers a, c and P a power of two: a is reduced
-// exactly modulo 2N and c modulo P before the one rounding of the argument.  Every
-// phase of the azimuthal stage is of this form: on the HEALPix grid phi0 is 0 or
-// pi / N (healpix.py:107-140), so e^{i m phi0} = e^{i pi m / N}; the chirp-z factors are
-// e^{+-i pi n^2 / N} (_azimuth.py:150-191) and the split-length twiddles e^{+-2 pi i s k / P}.
-__device__ __forceinline__ double2 cis_pi(int a, int N, int c, int P) {
+// e^{i pi a / N}, a taken modulo 2 N and folded to the first octant in integers, so the one
+// rounding of the argument is that of a value <= 1/4.
+__device__ __forceinline__ double2 cis_pi(long long a, int N) {
     const int n2 = 2 * N;
-    int r = a % n2;
+    int r = (int)(a % n2);
     if (r < 0) r += n2;
-    int q = c % P;
-    if (q < 0) q += P;
-    double s, co;
-    sincospi((double)r / (double)N + 2.0 * (double)q / (double)P, &s, &co);
-    return make_double2(co, s);
-}
-
-// e^{i * sgn * pi * (n^2 mod 2N) / N}: the exact chirp-z argument reduction.
-__device__ __forceinline__ double2 chirp(long long n, int N, double sgn) {
-    const long long r = (n * n) % (2LL * N);
+    const bool neg = r > N;  // lower half plane
+    if (neg) r = n2 - r;
+    const bool flip = 2 * r > N;  // second quadrant
+    if (flip) r = N - r;
+    const bool swap = 4 * r > N;  // second octant: pi/2 - angle = pi (N - 2 r) / (2 N)
     double s, c;
-    sincospi(sgn * (double)r / (double)N, &s, &c);
-    return make_double2(c, s);
+    if (swap) sincospi((double)(N - 2 * r) / (double)n2, &c, &s);
+    else sincospi((double)r / (double)N, &s, &c);
+    return make_double2(flip ? -c : c, neg ? -s : s);
 }
 
-// e^{i * sgn * 2 pi a / b} for integers, via sincospi with an exact rational argument.
-__device__ __forceinline__ double2 root(long long a, long long b, double sgn) {
-    const long long r = a % b;
-    double s, c;
-    sincospi(sgn * 2.0 * (double)r / (double)b, &s, &c);
-    return make_double2(c, s);
-}
-
-// e^{-+2 pi i a / L} from the twiddle table (e^{-2 pi i j / kTwLen}), L a power of two
-// dividing kTwLen; `plus` selects the + sign.
-__device__ __forceinline__ double2 twid(const double2 *__restrict__ tw, int a, int L, bool plus) {
-    int r = a & (L - 1);
-    double2 w = JHTB_IN(r * (kTwLen / L), kTwLen, 107) ? __ldg(&tw[r * (kTwLen / L)]) : make_double2(0.0, 0.0);
-    if (plus) w.y = -w.y;
-    return w;
-}
-
-// Shared-memory layout of an FFT buffer: one pad slot every 16 and every 256 elements,
-// so the strided accesses of the Stockham passes spread over the banks.
-__device__ __forceinline__ int pidx(int i) { return i + (i >> 4) + (i >> 8); }
-constexpr int kFftBufLen = kFftPiece + kFftPiece / 16 + kFftPiece / 256;
-
+// ---------------------------------------------------------------------------------
+// register FFTs
+// ---------------------------------------------------------------------------------
 // cos and sin of k pi / 8, k < 8 (the 16th roots of unity)
 __host__ __device__ constexpr double cos16(int k) {
     return k == 0 ? 1.0 : k == 1 ? 0.9238795325112867 : k == 2 ? 0.7071067811865476 : k == 3 ? 0.3826834323650898
@@ -108,225 +78,199 @@ __host__ __device__ constexpr int brev_ct(int i, int bits) {
 }
 __host__ __device__ constexpr int ilog2_ct(int n) { return n <= 1 ? 0 : 1 + ilog2_ct(n / 2); }
 
-// R-point DFT in registers (R <= 16), natural order in and out: radix-2 DIT after a
-// bit-reversal permutation, all indices and roots fixed at compile time.
-// dir = -1: e^{-2 pi i jk/R}; +1: e^{+...}.
-template <int R, int LEN, int I, int K>
-__device__ __forceinline__ void rf_bfly(double2 (&v)[R], double dir) {
-    constexpr int h = LEN / 2, ROOT = K * (16 / LEN);  // e^{dir 2 pi i ROOT / 16}
-    const double2 a = v[I + K];
-    double2 b = v[I + K + h];
-    if constexpr (ROOT == 4) b = make_double2(-dir * b.y, dir * b.x);
-    else if constexpr (ROOT != 0) b = cmul(b, make_double2(cos16(ROOT), dir * sin16(ROOT)));
-    v[I + K] = cadd(a, b);
-    v[I + K + h] = csub(a, b);
+// R-point DFT of v[O .. O + R) in registers (R <= 16), natural order in and out: radix-2 DIT
+// after a bit reversal, all indices and roots fixed at compile time.  DIR = -1:
+// e^{-2 pi i jk/R}; +1: e^{+...}.  HALF: the upper half of the inputs is zero, so the first
+// stage copies.
+template <int R, int O, int DIR, int LEN, int I, int K>
+__device__ __forceinline__ void rf_bfly(double2 (&v)[16]) {
+    constexpr int h = LEN / 2, ROOT = K * (16 / LEN);  // e^{DIR 2 pi i ROOT / 16}
+    const double2 a = v[O + I + K];
+    double2 b = v[O + I + K + h];
+    if constexpr (ROOT == 4) b = DIR > 0 ? make_double2(-b.y, b.x) : make_double2(b.y, -b.x);
+    else if constexpr (ROOT == 2) {  // (1 + i DIR) / sqrt 2
+        constexpr double c = 0.7071067811865476;
+        b = DIR > 0 ? make_double2(c * (b.x - b.y), c * (b.x + b.y)) : make_double2(c * (b.x + b.y), c * (b.y - b.x));
+    } else if constexpr (ROOT == 6) {
+        constexpr double c = 0.7071067811865476;
+        b = DIR > 0 ? make_double2(-c * (b.x + b.y), c * (b.x - b.y)) : make_double2(c * (b.y - b.x), -c * (b.x + b.y));
+    } else if constexpr (ROOT != 0) b = cmul(b, make_double2(cos16(ROOT), DIR * sin16(ROOT)));
+    v[O + I + K] = cadd(a, b);
+    v[O + I + K + h] = csub(a, b);
 }
-template <int R, int LEN, int IDX>
-__device__ __forceinline__ void rf_stage(double2 (&v)[R], double dir) {
+template <int R, int O, int DIR, int LEN, int IDX>
+__device__ __forceinline__ void rf_stage(double2 (&v)[16]) {
     if constexpr (IDX < R / 2) {
         constexpr int h = LEN / 2;
-        rf_bfly<R, LEN, (IDX / h) * LEN, IDX % h>(v, dir);
-        rf_stage<R, LEN, IDX + 1>(v, dir);
+        rf_bfly<R, O, DIR, LEN, (IDX / h) * LEN, IDX % h>(v);
+        rf_stage<R, O, DIR, LEN, IDX + 1>(v);
     }
 }
-template <int R, int LEN>
-__device__ __forceinline__ void rf_stages(double2 (&v)[R], double dir) {
+template <int R, int O, int DIR, int LEN>
+__device__ __forceinline__ void rf_stages(double2 (&v)[16]) {
     if constexpr (LEN <= R) {
-        rf_stage<R, LEN, 0>(v, dir);
-        rf_stages<R, LEN * 2>(v, dir);
+        rf_stage<R, O, DIR, LEN, 0>(v);
+        rf_stages<R, O, DIR, LEN * 2>(v);
     }
 }
-template <int R, int I>
-__device__ __forceinline__ void rf_bitrev(double2 (&v)[R]) {
+template <int R, int O, int I>
+__device__ __forceinline__ void rf_bitrev(double2 (&v)[16]) {
     if constexpr (I < R) {
         constexpr int J = brev_ct(I, ilog2_ct(R));
         if constexpr (J > I) {
-            const double2 t = v[I];
-            v[I] = v[J];
-            v[J] = t;
+            const double2 t = v[O + I];
+            v[O + I] = v[O + J];
+            v[O + J] = t;
         }
-        rf_bitrev<R, I + 1>(v);
+        rf_bitrev<R, O, I + 1>(v);
     }
 }
-template <int R>
-__device__ __forceinline__ void reg_fft(double2 (&v)[R], double dir) {
-    rf_bitrev<R, 0>(v);
-    rf_stages<R, 2>(v, dir);
+template <int R, int DIR, bool HALF, int O = 0>
+__device__ __forceinline__ void reg_fft(double2 (&v)[16]) {  // every group of R points of v
+    if constexpr (O < 16) {
+        rf_bitrev<R, O, 0>(v);
+        if constexpr (HALF) {
+#pragma unroll
+            for (int q = 0; q < R; q += 2) v[O + q + 1] = v[O + q];
+            rf_stages<R, O, DIR, 4>(v);
+        } else {
+            rf_stages<R, O, DIR, 2>(v);
+        }
+        reg_fft<R, DIR, HALF, O + R>(v);
+    }
 }
 
-// One in-place Stockham pass of radix R over n points (Ns = product of the earlier
-// radices): every thread loads its R inputs (stride n/R), twiddles them by
-// e^{dir 2 pi i (j mod Ns) r / (Ns R)}, runs an R-point DFT in registers and, after a
-// barrier, stores them at (j / Ns) Ns R + (j mod Ns) + r Ns.  n <= kFftPiece = 4096
-// and kFftThreads threads: each thread holds at most kFftPiece / kFftThreads points.
-template <int R>
-__device__ __forceinline__ void stockham_pass(double2 *buf, int n, int Ns, double dir,
-                                              const double2 *__restrict__ tw) {
-    constexpr int JM = kFftPiece / (R * kFftThreads);
-    const int nj = n / R;
-    double2 v[JM][R];
+// ---------------------------------------------------------------------------------
+// FFT of P = 2^LOGP points by TP = P / 16 threads (thread t), 16 points each in registers
+// ---------------------------------------------------------------------------------
+template <int LOGP>
+struct Fft {
+    static constexpr int P = 1 << LOGP, TP = P / 16, NP = (LOGP + 3) / 4;
+    static constexpr int RLAST = 1 << (LOGP - 4 * (NP - 1));  // radix of the last pass
+    // shared-memory layout: pads after every P / 16 points (and every 32 at 8192) spread the
+    // strided accesses of the passes over the 16-byte bank groups
+    static constexpr int PAD = LOGP == 10 ? 5 : (LOGP == 9 ? 3 : 1);
+    static __device__ __forceinline__ int pidx(int i) {
+        int r = i + PAD * (i >> (LOGP - 4));
+        if (LOGP == 13) r += 2 * (i >> 5);
+        return r;
+    }
+    static constexpr int LEN = P + 16 * PAD + (LOGP == 13 ? P / 16 : 0);
+
+    // the output digits (k1 least significant) of butterfly c of the last pass -> its block
+    static __device__ __forceinline__ int rev(int c) {
+        if (NP <= 2) return c;
+        if (NP == 3) return ((c & 15) << 4) | (c >> 4);
+        return ((c & 15) << 8) | (((c >> 4) & 15) << 4) | (c >> 8);
+    }
+    // position of point q of this thread in pass PASS
+    template <int PASS>
+    static __device__ __forceinline__ int pos(int t, int q) {
+        constexpr int BLOG = LOGP - 4 * PASS;
+        if constexpr (PASS == NP - 1) {
+            return pidx((rev(t + TP * (q / RLAST)) * RLAST) + q % RLAST);
+        } else {
+            constexpr int SLOG = BLOG - 4;
+            return pidx(((t >> SLOG) << BLOG) + (t & ((1 << SLOG) - 1)) + (q << SLOG));
+        }
+    }
+    // multiply point q of pass PASS by e^{+-2 pi i j q / B}, B the pass's block: four table
+    // entries and products of at most three of them
+    template <int PASS, bool PLUS>
+    static __device__ __forceinline__ void twiddle(double2 (&v)[16], int t, const double2 *__restrict__ tw) {
+        constexpr int BLOG = LOGP - 4 * PASS, SLOG = BLOG - 4;
+        static_assert((1 << 15) == kTwLen && BLOG <= 15, "twiddle table");
+        const int st = (t & ((1 << SLOG) - 1)) << (15 - BLOG);
+        const double2 w1 = __ldg(&tw[st]);
+        const double2 w2 = cmul(w1, w1), w3 = cmul(w2, w1);
+        v[1] = PLUS ? cmulc(v[1], w1) : cmul(v[1], w1);
+        v[2] = PLUS ? cmulc(v[2], w2) : cmul(v[2], w2);
+        v[3] = PLUS ? cmulc(v[3], w3) : cmul(v[3], w3);
 #pragma unroll
-    for (int jj = 0; jj < JM; ++jj) {
-        const int j = threadIdx.x + jj * kFftThreads;
-        if (j < nj) {
-            const int jm = j & (Ns - 1);
+        for (int a = 4; a < 16; a += 4) {
+            const double2 wa = __ldg(&tw[a * st]);
+            v[a] = PLUS ? cmulc(v[a], wa) : cmul(v[a], wa);
+            const double2 u1 = cmul(wa, w1), u2 = cmul(wa, w2), u3 = cmul(wa, w3);
+            v[a + 1] = PLUS ? cmulc(v[a + 1], u1) : cmul(v[a + 1], u1);
+            v[a + 2] = PLUS ? cmulc(v[a + 2], u2) : cmul(v[a + 2], u2);
+            v[a + 3] = PLUS ? cmulc(v[a + 3], u3) : cmul(v[a + 3], u3);
+        }
+    }
+    template <int PASS>
+    static __device__ __forceinline__ void put(const double2 (&v)[16], double2 *buf, int t) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) v[jj][r] = buf[pidx(j + r * nj)];
-            if (Ns > 1) {
-                const int step = jm * (kTwLen / (Ns * R));
+        for (int q = 0; q < 16; ++q) buf[pos<PASS>(t, q)] = v[q];
+    }
+    template <int PASS>
+    static __device__ __forceinline__ void get(double2 (&v)[16], const double2 *buf, int t) {
 #pragma unroll
-                for (int r = 1; r < R; ++r) {
-                    double2 w = JHTB_IN(step * r, kTwLen, 107) ? __ldg(&tw[step * r]) : make_double2(0.0, 0.0);
-                    if (dir > 0) w.y = -w.y;
-                    v[jj][r] = cmul(v[jj][r], w);
-                }
+        for (int q = 0; q < 16; ++q) v[q] = buf[pos<PASS>(t, q)];
+    }
+    // forward, e^{+}: v[q] = x[t + TP q] in, v[g RLAST + q] = X[out_index(t, g RLAST + q)] out.
+    // The buffer must be free on entry; `on` is false for idle threads, which only meet the barriers.
+    template <int PASS, bool HALF>
+    static __device__ __forceinline__ void forward_from(double2 (&v)[16], double2 *buf, int t, bool on,
+                                                        const double2 *__restrict__ tw) {
+        if constexpr (PASS == NP - 1) {
+            if (on) reg_fft<RLAST, 1, HALF>(v);
+        } else {
+            if (on) {
+                reg_fft<16, 1, HALF>(v);
+                twiddle<PASS, true>(v, t, tw);
+                put<PASS>(v, buf, t);
             }
-            reg_fft<R>(v[jj], dir);
+            __syncthreads();
+            if (on) get<PASS + 1>(v, buf, t);
+            forward_from<PASS + 1, false>(v, buf, t, on, tw);
         }
     }
-    __syncthreads();
-#pragma unroll
-    for (int jj = 0; jj < JM; ++jj) {
-        const int j = threadIdx.x + jj * kFftThreads;
-        if (j < nj) {
-            const int jm = j & (Ns - 1);
-            const int d = (j - jm) * R + jm;
-#pragma unroll
-            for (int r = 0; r < R; ++r) buf[pidx(d + r * Ns)] = v[jj][r];
-        }
+    template <bool HALF>
+    static __device__ __forceinline__ void forward(double2 (&v)[16], double2 *buf, int t, bool on,
+                                                   const double2 *__restrict__ tw) {
+        forward_from<0, HALF>(v, buf, t, on, tw);
     }
-    __syncthreads();
-}
-
-// One pass as a separate function: each radix is compiled once, with its own registers.
-template <int R>
-__device__ __noinline__ void stockham_pass_call(double2 *buf, int n, int Ns, double dir,
-                                                const double2 *__restrict__ tw) {
-    stockham_pass<R>(buf, n, Ns, dir, tw);
-}
-
-// In-place FFT of length n (power of two <= kFftPiece) on a padded shared-memory buffer,
-// natural order in and out.  dir = -1: e^{-2 pi i jk/n}; +1: e^{+2 pi i jk/n}.
-// Passes of radix 16 with one smaller radix for the remaining bits.
-__device__ __forceinline__ void fft_stockham(double2 *buf, int n, double dir, const double2 *__restrict__ tw) {
-    int bits = ilog2i(n), Ns = 1;
-    for (; bits >= 4; bits -= 4, Ns <<= 4) stockham_pass_call<16>(buf, n, Ns, dir, tw);
-    if (bits == 3) stockham_pass_call<8>(buf, n, Ns, dir, tw);
-    else if (bits == 2) stockham_pass_call<4>(buf, n, Ns, dir, tw);
-    else if (bits == 1) stockham_pass_call<2>(buf, n, Ns, dir, tw);
-}
-
-// Twiddles from shared memory: e^{-2 pi i x / kFftPiece} = T[x >> 6] T[64 + (x & 63)] with
-// T[a] = e^{-2 pi i a / 64} and T[64 + b] = e^{-2 pi i b / kFftPiece} (each entry rounded once,
-// the product adds about one rounding), so the passes make no global loads.
-// Eight more entries T[128 + g] = e^{-2 pi i g / kTwLen} refine it to kTwLen points (the ring
-// phases and piece twiddles of power-of-two rings up to kTwLen / 2 points).
-constexpr int kSmTwLen = 136;
-constexpr int kSmTwFine = kTwLen / kFftPiece;  // 8
-static_assert(kFftPiece == 64 * 64, "two-level twiddle table of kFftPiece points");
-__device__ __forceinline__ void sm_tw_init(double2 *T) {
-    for (int a = threadIdx.x; a < kSmTwLen; a += blockDim.x) {
-        double s, c;
-        if (a < 64) sincospi(-2.0 * (double)a / 64.0, &s, &c);
-        else if (a < 128) sincospi(-2.0 * (double)(a - 64) / (double)kFftPiece, &s, &c);
-        else sincospi(-2.0 * (double)(a - 128) / (double)kTwLen, &s, &c);
-        T[a] = make_double2(c, s);
-    }
-}
-__device__ __forceinline__ double2 sm_tw(const double2 *T, int x, bool plus) {  // e^{-+2 pi i x / kFftPiece}
-    x &= kFftPiece - 1;
-    double2 w = cmul(T[x >> 6], T[64 + (x & 63)]);
-    if (plus) w.y = -w.y;
-    return w;
-}
-
-// e^{+i pi a / N} for a power-of-two N, kFftPiece / 2 <= N <= kTwLen / 2, from the shared
-// table: with x = a mod 2N = q y + f (q = 2N / kFftPiece), the conjugate of
-// e^{-2 pi i y / kFftPiece} e^{-2 pi i f / 2N}.
-__device__ __forceinline__ double2 sm_tw_pi(const double2 *T, long long a, int N) {
-    const int x = (int)(a & (2LL * N - 1)), q = 2 * N / kFftPiece;
-    double2 w = cmul(sm_tw(T, x / q, false), T[128 + (x % q) * (kSmTwFine / q)]);
-    w.y = -w.y;
-    return w;
-}
-
-// stockham_pass with the shared-memory twiddle table.
-template <int R>
-__device__ __forceinline__ void stockham_pass_sm(double2 *buf, int n, int Ns, double dir, const double2 *T) {
-    constexpr int JM = kFftPiece / (R * kFftThreads);
-    const int nj = n / R;
-    double2 v[JM][R];
-#pragma unroll
-    for (int jj = 0; jj < JM; ++jj) {
-        const int j = threadIdx.x + jj * kFftThreads;
-        if (j < nj) {
-            const int jm = j & (Ns - 1);
-#pragma unroll
-            for (int r = 0; r < R; ++r) v[jj][r] = buf[pidx(j + r * nj)];
-            if (Ns > 1) {
-                const int step = jm * (kFftPiece / (Ns * R));
-#pragma unroll
-                for (int r = 1; r < R; ++r) v[jj][r] = cmul(v[jj][r], sm_tw(T, step * r, dir > 0));
+    static __device__ __forceinline__ int out_index(int t, int q) { return t + TP * (q / RLAST) + (P / RLAST) * (q % RLAST); }
+    // the transpose with e^{-}: takes forward's output layout back to v[q] = x[t + TP q] (times P)
+    template <int PASS>
+    static __device__ __forceinline__ void backward_from(double2 (&v)[16], double2 *buf, int t, bool on,
+                                                         const double2 *__restrict__ tw) {
+        if (on) {
+            if constexpr (PASS == NP - 1) reg_fft<RLAST, -1, false>(v);
+            else {
+                twiddle<PASS, false>(v, t, tw);
+                reg_fft<16, -1, false>(v);
             }
-            reg_fft<R>(v[jj], dir);
+        }
+        if constexpr (PASS > 0) {
+            if (on) put<PASS>(v, buf, t);
+            __syncthreads();
+            if (on) get<PASS - 1>(v, buf, t);
+            backward_from<PASS - 1>(v, buf, t, on, tw);
         }
     }
-    __syncthreads();
-#pragma unroll
-    for (int jj = 0; jj < JM; ++jj) {
-        const int j = threadIdx.x + jj * kFftThreads;
-        if (j < nj) {
-            const int jm = j & (Ns - 1);
-            const int d = (j - jm) * R + jm;
-#pragma unroll
-            for (int r = 0; r < R; ++r) buf[pidx(d + r * Ns)] = v[jj][r];
-        }
+    static __device__ __forceinline__ void backward(double2 (&v)[16], double2 *buf, int t, bool on,
+                                                    const double2 *__restrict__ tw) {
+        backward_from<NP - 1>(v, buf, t, on, tw);
     }
-    __syncthreads();
-}
+};
 
-// The FFT with every pass inlined (no call boundary, so no register saves to the stack
-// around the passes) and shared-memory twiddles; for kernels that run one or two transforms.
-// Largest radix of the piece kernels' passes (16: fewer passes; 8: fewer registers).
-#ifndef JHTB_PIECE_RADIX
-#define JHTB_PIECE_RADIX 16
-#endif
-__device__ __forceinline__ void fft_stockham_sm(double2 *buf, int n, double dir, const double2 *T) {
-    int bits = ilog2i(n), Ns = 1;
-    if (JHTB_PIECE_RADIX >= 16) {
-        for (; bits >= 4; bits -= 4, Ns <<= 4) stockham_pass_sm<16>(buf, n, Ns, dir, T);
-        if (bits == 3) stockham_pass_sm<8>(buf, n, Ns, dir, T);
-    } else {
-        for (; bits >= 3; bits -= 3, Ns <<= 3) stockham_pass_sm<8>(buf, n, Ns, dir, T);
-    }
-    if (bits == 2) stockham_pass_sm<4>(buf, n, Ns, dir, T);
-    else if (bits == 1) stockham_pass_sm<2>(buf, n, Ns, dir, T);
-}
-
-// Bluestein spectrum for the synthesis direction: Bh+ = FFT_P(b)/P with
-// b[n] = conj(w(n)) on |n| < N, w(n) = e^{+i pi n^2 / N}.  The adjoint direction
-// uses Bh-[k] = conj(Bh+[(P - k) mod P]).
-__device__ __forceinline__ double2 bh_get(const double2 *bh, int P, int k, int sgn) {
-    if (!JHTB_IN(k, P, 108)) return make_double2(0.0, 0.0);
-    if (sgn > 0) return __ldg(&bh[k]);
-    return conjd(__ldg(&bh[(P - k) & (P - 1)]));
-}
-
-// D[k] of the synthesis fold for one ring, without its phase (spin 0 passes Fm == Fp):
-// with m = k + jN in the first sum and m = jN - k in the second,
+// ---------------------------------------------------------------------------------
+// the fold
+// ---------------------------------------------------------------------------------
+// D[k] without its ring phase: with m = k + jN in the first sum and m = jN - k in the second,
 // e^{i m phi0} = (-1)^j e^{+-i pi k / N} when phi0 = pi / N, so
-// D[k] = e^{i pi k / N} [sum_j (-1)^j Fp_{k+jN} + sum_j (-1)^j conj(Fm_{jN-k})];
+// D[k] = e^{i pi k / N} [sum_j (-1)^j P_{k+jN} + sum_j (-1)^j conj(M_{jN-k})];
 // `shifted` selects the (-1)^j signs, the caller applies e^{i pi k / N}.  Aliases
 // j = part, part + parts, ... only (the caller sums the parts in a fixed order).
-__device__ __forceinline__ double2 fold_synth(const double2 *__restrict__ Fp, const double2 *__restrict__ Fm,
-                                              int k, int N, int lmax, bool shifted, int part = 0, int parts = 1) {
-    double2 d = make_double2(0.0, 0.0);
+__device__ __forceinline__ double2 fold_sum(const double2 *__restrict__ Pr, const double2 *__restrict__ Mr, int k,
+                                            int N, int lmax, bool shifted, int part = 0, int parts = 1) {
+    double2 d = zero2();
     const double flip = (shifted && (parts & 1)) ? -1.0 : 1.0;  // sign change per step of `parts` aliases
     double sg = (shifted && (part & 1)) ? -1.0 : 1.0;
     const int step = parts * N;
 #pragma unroll 4
     for (int m = k + part * N; m <= lmax; m += step) {
-        const double2 f = JHTB_IN(m, lmax + 1, 101) ? Fp[m] : make_double2(0.0, 0.0);
+        const double2 f = JHTB_IN(m, lmax + 1, 101) ? Pr[m] : zero2();
         d.x = fma(sg, f.x, d.x);
         d.y = fma(sg, f.y, d.y);
         sg *= flip;
@@ -335,7 +279,7 @@ __device__ __forceinline__ double2 fold_synth(const double2 *__restrict__ Fp, co
     sg = (shifted && ((1 + part) & 1)) ? -1.0 : 1.0;
 #pragma unroll 4
     for (int m = (1 + part) * N - k; m <= lmax; m += step) {
-        const double2 f = JHTB_IN(m, lmax + 1, 102) ? Fm[m] : make_double2(0.0, 0.0);
+        const double2 f = JHTB_IN(m, lmax + 1, 102) ? Mr[m] : zero2();
         d.x = fma(sg, f.x, d.x);
         d.y = fma(-sg, f.y, d.y);
         sg *= flip;
@@ -343,753 +287,561 @@ __device__ __forceinline__ double2 fold_synth(const double2 *__restrict__ Fp, co
     return d;
 }
 
-// Elements per thread whose global loads are issued together in the azimuthal loops (the
-// loops are bound by L2 / HBM latency, not by arithmetic).
-constexpr int kU = 4;
-
-// The phased (and, for chirp-z, chirped) fold a[k] for k < N into dst[k] (padded shared
-// buffer or a global row).  Rings longer than lmax have at most one term per sum, loaded
-// kU elements at a time; shorter rings split each k's aliases over blockDim / N threads
-// when N < blockDim (partial sums combined in a fixed order through `part_buf`).
-template <bool PADDED>
-__device__ __forceinline__ void synth_fold(const double2 *__restrict__ Fp, const double2 *__restrict__ Fm, int N,
-                                           int lmax, bool shifted, bool blue, double2 *dst, double2 *part_buf) {
-    auto phase = [&](int k, double2 d) {
-        // e^{i pi k / N} ring phase; chirp-z: times w(k) = e^{i pi k^2 / N}
-        const int ph = (shifted ? k : 0) + (blue ? (int)(((long long)k * k) % (2 * N)) : 0);
-        return ph ? cmul(d, cis_pi(ph, N, 0, 1)) : d;
-    };
-    if (N > lmax) {
-        const double sg = shifted ? -1.0 : 1.0;
-        for (int k0 = threadIdx.x; k0 < N; k0 += kU * blockDim.x) {
-            double2 fp[kU], fm[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int k = k0 + u * blockDim.x;
-                fp[u] = (k < N && k <= lmax && JHTB_IN(k, lmax + 1, 101)) ? Fp[k] : make_double2(0.0, 0.0);
-                fm[u] = (k < N && k >= 1 && N - k <= lmax && JHTB_IN(N - k, lmax + 1, 102)) ? Fm[N - k] : make_double2(0.0, 0.0);
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int k = k0 + u * blockDim.x;
-                if (k < N) {
-                    const double2 d = make_double2(fma(sg, fm[u].x, fp[u].x), fma(-sg, fm[u].y, fp[u].y));
-                    dst[PADDED ? pidx(k) : k] = phase(k, d);
-                }
-            }
-        }
-        return;
-    }
-    const int parts = N < (int)blockDim.x ? (int)blockDim.x / N : 1;
-    if (parts == 1) {
-        for (int k = threadIdx.x; k < N; k += blockDim.x) dst[PADDED ? pidx(k) : k] = phase(k, fold_synth(Fp, Fm, k, N, lmax, shifted));
-        return;
-    }
-    if ((int)threadIdx.x < N * parts) {
-        const int k = threadIdx.x % N, part = threadIdx.x / N;
-        part_buf[threadIdx.x] = fold_synth(Fp, Fm, k, N, lmax, shifted, part, parts);
-    }
-    __syncthreads();
-    if ((int)threadIdx.x < N) {
-        double2 d = part_buf[threadIdx.x];
-        for (int q = 1; q < parts; ++q) d = cadd(d, part_buf[q * N + threadIdx.x]);
-        dst[PADDED ? pidx(threadIdx.x) : threadIdx.x] = phase(threadIdx.x, d);
-    }
+// The same for a ring longer than lmax: at most one term per sum, no loop, so that a caller's
+// unrolled loads are all issued before the first is used.
+__device__ __forceinline__ double2 fold_one(const double2 *__restrict__ Pr, const double2 *__restrict__ Mr, int k,
+                                            int N, int lmax, bool shifted) {
+    const double2 p = (k <= lmax && JHTB_IN(k, lmax + 1, 101)) ? Pr[k] : zero2();
+    const double2 q = (k >= 1 && N - k <= lmax && JHTB_IN(N - k, lmax + 1, 102)) ? Mr[N - k] : zero2();
+    const double sg = shifted ? -1.0 : 1.0;
+    return make_double2(fma(sg, q.x, p.x), fma(-sg, q.y, p.y));
 }
-
-// Scratch for the fold's partial sums of short rings (N < blockDim), past the part of the
-// padded FFT buffer such rings use (their transforms have at most 512 points).
-constexpr int kPartOff = 2048;
-
-template <int SPIN>
-__global__ void __launch_bounds__(kFftThreads, kFftMinBlocks) ring_synth_kernel(const int *__restrict__ ring_list,
-                                                                     const RingDesc *__restrict__ rings, int lmax,
-                                                                     int M, int nrings, long long npix,
-                                                                     const double2 *__restrict__ F_all,
-                                                                     double *__restrict__ maps_all,
-                                                                     double2 *__restrict__ A_all,
-                                                                     double2 *__restrict__ Y_all,
-                                                                     const double2 *__restrict__ tw,
-                                                                     const double2 *__restrict__ bh) {
-    extern __shared__ double2 buf[];
-    const int r = ring_list ? ring_list[blockIdx.x] : (int)blockIdx.x;
-    const RingDesc rd = rings[r];
-    const int N = rd.N, Q = rd.Q;
-    const bool shifted = rd.phi0 != 0.0;
-    const bool blue = rd.mode == kBluestein;
-    constexpr int nchan = SPIN ? 2 : 1;
-    const double2 *Fp = F_all + ((size_t)blockIdx.y * nchan * nrings + r) * M;
-    const double2 *Fm = SPIN ? Fp + (size_t)nrings * M : Fp;
-    double *outQ = maps_all + (size_t)blockIdx.y * nchan * npix + rd.start;
-    double *outU = outQ + npix;
-    const int bd = blockDim.x;
-    const double2 *B = bh + rd.bh_off;
-    if (Q == 1) {
-        // the whole transform in shared memory: fold (chirped for chirp-z, zero-padded to P)
-        const int L = blue ? rd.P : N;
-        synth_fold<true>(Fp, Fm, N, lmax, shifted, blue, buf, buf + kPartOff);
-        for (int k = N + threadIdx.x; k < L; k += bd) buf[pidx(k)] = make_double2(0.0, 0.0);
-        __syncthreads();
-        if (blue) {
-            fft_stockham(buf, L, -1.0, tw);
-            for (int q0 = threadIdx.x; q0 < L; q0 += kU * bd) {
-                double2 w[kU];
-#pragma unroll
-                for (int u = 0; u < kU; ++u) w[u] = q0 + u * bd < L ? bh_get(B, L, q0 + u * bd, 1) : make_double2(0.0, 0.0);
-#pragma unroll
-                for (int u = 0; u < kU; ++u)
-                    if (q0 + u * bd < L) buf[pidx(q0 + u * bd)] = cmul(buf[pidx(q0 + u * bd)], w[u]);
-            }
-            __syncthreads();
-        }
-        fft_stockham(buf, L, +1.0, tw);
-        for (int j = threadIdx.x; j < N; j += bd) {
-            double2 v = buf[pidx(j)];
-            if (blue) v = cmul(v, cis_pi((int)(((long long)j * j) % (2 * N)), N, 0, 1));
-            if (JHTB_IN(rd.start + j, npix, 104)) {
-                outQ[j] = v.x;
-                if (SPIN) outU[j] = v.y;
-            }
-        }
-        return;
-    }
-    // Transform of length L (N, or the chirp-z length P) in Q pieces of Lp points.  One
-    // pass writes the phased (and chirped) fold a[k] to the ring's scratch row; piece s
-    // then folds a[k] e^{-+2 pi i s k / L} modulo Lp with table twiddles.
-    const int L = blue ? rd.P : N, Lp = L / Q;
-    double2 *Ag = A_all + (size_t)blockIdx.y * npix + rd.start;
-    double2 *Yg = Y_all + (size_t)blockIdx.y * npix + rd.start;
-    synth_fold<false>(Fp, Fm, N, lmax, shifted, blue, Ag, buf + kPartOff);
-    __syncthreads();
-    for (int s = 0; s < Q; ++s) {
-        for (int q0 = threadIdx.x; q0 < Lp; q0 += kU * bd) {
-            double2 v[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) v[u] = make_double2(0.0, 0.0);
-            for (int t = 0; t * Lp < N; ++t) {
-                double2 a[kU], w[kU];
-#pragma unroll
-                for (int u = 0; u < kU; ++u) {
-                    const int k = q0 + u * bd + t * Lp;
-                    const bool ok = q0 + u * bd < Lp && k < N;
-                    a[u] = (ok && JHTB_IN(rd.start + k, npix, 109)) ? Ag[k] : make_double2(0.0, 0.0);
-                    // direct: inverse DFT, e^{+2 pi i s k / N}; chirp-z: FFT_P, e^{-2 pi i s k / P}
-                    w[u] = (ok && s) ? twid(tw, s * k, L, !blue) : make_double2(1.0, 0.0);
-                }
-#pragma unroll
-                for (int u = 0; u < kU; ++u) v[u] = cadd(v[u], cmul(a[u], w[u]));
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u)
-                if (q0 + u * bd < Lp) buf[pidx(q0 + u * bd)] = v[u];
-        }
-        __syncthreads();
-        if (!blue) {
-            fft_stockham(buf, Lp, +1.0, tw);
-            for (int q = threadIdx.x; q < Lp; q += bd) {
-                const double2 v = buf[pidx(q)];
-                if (JHTB_IN(rd.start + (long long)Q * q + s, npix, 104)) {
-                    outQ[Q * q + s] = v.x;
-                    if (SPIN) outU[Q * q + s] = v.y;
-                }
-            }
-            __syncthreads();
-            continue;
-        }
-        fft_stockham(buf, Lp, -1.0, tw);
-        for (int q0 = threadIdx.x; q0 < Lp; q0 += kU * bd) {
-            double2 w[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) w[u] = q0 + u * bd < Lp ? bh_get(B, L, Q * (q0 + u * bd) + s, 1) : make_double2(0.0, 0.0);
-#pragma unroll
-            for (int u = 0; u < kU; ++u)
-                if (q0 + u * bd < Lp) buf[pidx(q0 + u * bd)] = cmul(buf[pidx(q0 + u * bd)], w[u]);
-        }
-        __syncthreads();
-        fft_stockham(buf, Lp, +1.0, tw);
-        // y[j] += conv_s[j mod Lp] e^{2 pi i s j / P}; the chirp is applied once after the last piece
-        for (int j0 = threadIdx.x; j0 < N; j0 += kU * bd) {
-            double2 y[kU], w[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int j = j0 + u * bd;
-                y[u] = (s && j < N && JHTB_IN(rd.start + j, npix, 109)) ? Yg[j] : make_double2(0.0, 0.0);
-                w[u] = (s && j < N) ? twid(tw, s * j, L, true) : make_double2(1.0, 0.0);
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int j = j0 + u * bd;
-                if (j >= N) continue;
-                double2 v = cadd(y[u], cmul(buf[pidx(j & (Lp - 1))], w[u]));
-                if (s < Q - 1) {
-                    if (JHTB_IN(rd.start + j, npix, 109)) Yg[j] = v;
-                } else {
-                    v = cmul(v, cis_pi((int)(((long long)j * j) % (2 * N)), N, 0, 1));
-                    if (JHTB_IN(rd.start + j, npix, 104)) {
-                        outQ[j] = v.x;
-                        if (SPIN) outU[j] = v.y;
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// V rows for ring r from its spectrum W (padded shared-memory buffer or natural global),
-// kU orders per thread at a time so the loads of a global W overlap.
-template <int SPIN, bool PADDED>
-__device__ __forceinline__ void gather_adjoint(const double2 *W, int N, int lmax, bool shifted, double2 *Vp,
-                                               double2 *Vm) {
-    const int bd = blockDim.x;
-    for (int m0 = threadIdx.x; m0 <= lmax; m0 += kU * bd) {
-        double2 vp[kU], vm[kU];
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int m = m0 + u * bd;
-            const int k1 = m % N, k2 = (N - k1) % N;
-            vp[u] = m <= lmax ? W[PADDED ? pidx(k1) : k1] : make_double2(0.0, 0.0);
-            vm[u] = (SPIN && m <= lmax) ? conjd(W[PADDED ? pidx(k2) : k2]) : vp[u];
-        }
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int m = m0 + u * bd;
-            if (m > lmax) continue;
-            double2 p = vp[u], q = vm[u];
-            if (shifted) {  // e^{-i m phi0} = e^{-i pi m / N}
-                const double2 cph = cis_pi(-(m % (2 * N)), N, 0, 1);
-                p = cmul(p, cph);
-                q = cmul(q, cph);
-            }
-            if (JHTB_IN(m, lmax + 1, 105)) {
-                Vp[m] = p;
-                if (SPIN) Vm[m] = q;
-            }
-        }
-    }
-}
-
-template <int SPIN>
-__global__ void __launch_bounds__(kFftThreads, kFftMinBlocks) ring_adjoint_kernel(const int *__restrict__ ring_list,
-                                                                       const RingDesc *__restrict__ rings, int lmax,
-                                                                       int M, int nrings, long long npix,
-                                                                       const double *__restrict__ maps_all,
-                                                                       double2 *__restrict__ V_all,
-                                                                       double2 *__restrict__ A_all,
-                                                                       double2 *__restrict__ W_all,
-                                                                       const double2 *__restrict__ tw,
-                                                                       const double2 *__restrict__ bh) {
-    extern __shared__ double2 buf[];
-    const int r = ring_list ? ring_list[blockIdx.x] : (int)blockIdx.x;
-    const RingDesc rd = rings[r];
-    const int N = rd.N, Q = rd.Q;
-    const bool shifted = rd.phi0 != 0.0;
-    const bool blue = rd.mode == kBluestein;
-    constexpr int nchan = SPIN ? 2 : 1;
-    const double *inQ = maps_all + (size_t)blockIdx.y * nchan * npix + rd.start;
-    const double *inU = inQ + npix;
-    double2 *Vp = V_all + ((size_t)blockIdx.y * nchan * nrings + r) * M;
-    double2 *Vm = SPIN ? Vp + (size_t)nrings * M : Vp;
-    const int bd = blockDim.x;
-    const double2 *B = bh + rd.bh_off;
-    // the ring's pixels (chirped for chirp-z: a[j] = v[j] conj(w(j))), kU at a time
-    auto load_in = [&](int j0, double2 (&a)[kU]) {
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int j = j0 + u * bd;
-            a[u] = (j < N && JHTB_IN(rd.start + j, npix, 103)) ? make_double2(inQ[j], SPIN ? inU[j] : 0.0) : make_double2(0.0, 0.0);
-        }
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int j = j0 + u * bd;
-            if (blue && j < N) a[u] = cmul(a[u], cis_pi(-(int)(((long long)j * j) % (2 * N)), N, 0, 1));
-        }
-    };
-    if (Q == 1) {
-        // the whole transform in shared memory
-        const int L = blue ? rd.P : N;
-        for (int j0 = threadIdx.x; j0 < N; j0 += kU * bd) {
-            double2 a[kU];
-            load_in(j0, a);
-#pragma unroll
-            for (int u = 0; u < kU; ++u)
-                if (j0 + u * bd < N) buf[pidx(j0 + u * bd)] = a[u];
-        }
-        for (int k = N + threadIdx.x; k < L; k += bd) buf[pidx(k)] = make_double2(0.0, 0.0);
-        __syncthreads();
-        fft_stockham(buf, L, -1.0, tw);
-        if (blue) {
-            for (int q0 = threadIdx.x; q0 < L; q0 += kU * bd) {
-                double2 w[kU];
-#pragma unroll
-                for (int u = 0; u < kU; ++u) w[u] = q0 + u * bd < L ? bh_get(B, L, q0 + u * bd, -1) : make_double2(0.0, 0.0);
-#pragma unroll
-                for (int u = 0; u < kU; ++u)
-                    if (q0 + u * bd < L) buf[pidx(q0 + u * bd)] = cmul(buf[pidx(q0 + u * bd)], w[u]);
-            }
-            __syncthreads();
-            fft_stockham(buf, L, +1.0, tw);
-            // W[k] = conj(w(k)) conv[k]
-            for (int k = threadIdx.x; k < N; k += bd)
-                buf[pidx(k)] = cmul(buf[pidx(k)], cis_pi(-(int)(((long long)k * k) % (2 * N)), N, 0, 1));
-            __syncthreads();
-        }
-        gather_adjoint<SPIN, true>(buf, N, lmax, shifted, Vp, Vm);
-        return;
-    }
-    // Forward transform of length L (N, or P) in Q pieces of Lp points; the spectrum
-    // W[k], k < N, is assembled in the ring's scratch row and then gathered.
-    const int L = blue ? rd.P : N, Lp = L / Q;
-    double2 *Ag = A_all + (size_t)blockIdx.y * npix + rd.start;
-    double2 *Wg = W_all + (size_t)blockIdx.y * npix + rd.start;
-    if (blue) {  // chirped input a[j] = v[j] conj(w(j)), once
-        for (int j0 = threadIdx.x; j0 < N; j0 += kU * bd) {
-            double2 a[kU];
-            load_in(j0, a);
-#pragma unroll
-            for (int u = 0; u < kU; ++u)
-                if (j0 + u * bd < N && JHTB_IN(rd.start + j0 + u * bd, npix, 109)) Ag[j0 + u * bd] = a[u];
-        }
-        __syncthreads();
-    }
-    for (int s = 0; s < Q; ++s) {
-        for (int q0 = threadIdx.x; q0 < Lp; q0 += kU * bd) {
-            double2 v[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) v[u] = make_double2(0.0, 0.0);
-            for (int t = 0; t * Lp < N; ++t) {
-                double2 a[kU], w[kU];
-#pragma unroll
-                for (int u = 0; u < kU; ++u) {
-                    const int j = q0 + u * bd + t * Lp;
-                    const bool ok = q0 + u * bd < Lp && j < N;
-                    a[u] = !ok ? make_double2(0.0, 0.0) : blue ? Ag[j] : make_double2(inQ[j], SPIN ? inU[j] : 0.0);
-                    w[u] = (ok && s) ? twid(tw, s * j, L, false) : make_double2(1.0, 0.0);  // e^{-2 pi i s j / L}
-                }
-#pragma unroll
-                for (int u = 0; u < kU; ++u) v[u] = cadd(v[u], cmul(a[u], w[u]));
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u)
-                if (q0 + u * bd < Lp) buf[pidx(q0 + u * bd)] = v[u];
-        }
-        __syncthreads();
-        fft_stockham(buf, Lp, -1.0, tw);
-        if (!blue) {  // W[Q q + s]
-            for (int q = threadIdx.x; q < Lp; q += bd)
-                if (JHTB_IN(rd.start + (long long)Q * q + s, npix, 109)) Wg[Q * q + s] = buf[pidx(q)];
-            __syncthreads();
-            continue;
-        }
-        for (int q0 = threadIdx.x; q0 < Lp; q0 += kU * bd) {
-            double2 w[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) w[u] = q0 + u * bd < Lp ? bh_get(B, L, Q * (q0 + u * bd) + s, -1) : make_double2(0.0, 0.0);
-#pragma unroll
-            for (int u = 0; u < kU; ++u)
-                if (q0 + u * bd < Lp) buf[pidx(q0 + u * bd)] = cmul(buf[pidx(q0 + u * bd)], w[u]);
-        }
-        __syncthreads();
-        fft_stockham(buf, Lp, +1.0, tw);
-        // W[k] = conj(w(k)) sum_s conv_s[k mod Lp] e^{2 pi i s k / P}, the chirp after the last piece
-        for (int k0 = threadIdx.x; k0 < N; k0 += kU * bd) {
-            double2 y[kU], w[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int k = k0 + u * bd;
-                y[u] = (s && k < N && JHTB_IN(rd.start + k, npix, 109)) ? Wg[k] : make_double2(0.0, 0.0);
-                w[u] = (s && k < N) ? twid(tw, s * k, L, true) : make_double2(1.0, 0.0);
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int k = k0 + u * bd;
-                if (k >= N) continue;
-                double2 v = cadd(y[u], cmul(buf[pidx(k & (Lp - 1))], w[u]));
-                if (s == Q - 1) v = cmul(v, cis_pi(-(int)(((long long)k * k) % (2 * N)), N, 0, 1));
-                if (JHTB_IN(rd.start + k, npix, 109)) Wg[k] = v;
-            }
-        }
-        __syncthreads();
-    }
-    __threadfence_block();
-    gather_adjoint<SPIN, false>(Wg, N, lmax, shifted, Vp, Vm);
-}
-
-// ---------------------------------------------------------------------------------
-// Long rings in pieces: a ring of N = Q Lq points (a power of two above kFftPiece, Lq =
-// kFftPiece; or a kSplit4 polar-cap ring, N = 4 Lq with Lq not a power of two) runs as Q
-// independent CTAs of the 256-thread shared-memory kernel, one per output residue class
-// (decimation in frequency).  Piece s:
-//   synthesis  out[Q j + s] = sum_{k1 < Lq} e^{+2 pi i j k1 / Lq} a_s[k1],
-//              a_s[k1]      = sum_{k2 < Q} D[k1 + Lq k2] e^{+2 pi i s (k1 + Lq k2) / N}
-//   adjoint    W[Q k + s]   = sum_{j1 < Lq} e^{-2 pi i k j1 / Lq} b_s[j1],
-//              b_s[j1]      = sum_{j2 < Q} v[j1 + Lq j2] e^{-2 pi i s (j1 + Lq j2) / N}
-// with D the phased fold of the synthesis and v the ring's pixels.  The length-Lq
-// transform is the Stockham FFT (power of two) or a chirp-z transform at P <= kFftPiece
-// points (kSplit4).  Every piece gathers the whole ring's input itself (the Q reads of a
-// ring's data hit L2), so pieces never exchange data and several fit on an SM at once.
-// ---------------------------------------------------------------------------------
-// e^{+i pi a / N} for a power-of-two N <= kTwLen / 2, from the twiddle table (entries
-// e^{-2 pi i j / kTwLen}, each rounded once).
-__device__ __forceinline__ double2 tw_pi(const double2 *__restrict__ tw, long long a, int N) {
-    const int r = (int)(a & (2LL * N - 1));
-    double2 w = JHTB_IN(r * (kTwLen / (2 * N)), kTwLen, 107) ? __ldg(&tw[r * (kTwLen / (2 * N))]) : make_double2(0.0, 0.0);
-    w.y = -w.y;
-    return w;
-}
-// most pieces of a ring (ring_pieces: a power of two N <= kTwLen / 2 in N / kFftPiece, kSplit4 in 4)
-constexpr int kMaxPieces = 4;
-static_assert(kTwLen / 2 / kFftPiece <= kMaxPieces, "pieces of the longest power-of-two ring");
 
 // e^{i pi k / 4}, k mod 8
 __device__ __forceinline__ double2 root8(int k) {
     constexpr double h = 0.70710678118654752440;
-    switch (k & 7) {
-        case 0: return make_double2(1.0, 0.0);
-        case 1: return make_double2(h, h);
-        case 2: return make_double2(0.0, 1.0);
-        case 3: return make_double2(-h, h);
-        case 4: return make_double2(-1.0, 0.0);
-        case 5: return make_double2(-h, -h);
-        case 6: return make_double2(0.0, -1.0);
-        default: return make_double2(h, -h);
+    const int q = k & 7;
+    const double c = (q & 3) == 0 ? 1.0 : ((q & 3) == 2 ? 0.0 : h), s = (q & 3) == 0 ? 0.0 : ((q & 3) == 2 ? 1.0 : h);
+    // q = 0: (1,0) 1: (h,h) 2: (0,1) 3: (-h,h) 4: (-1,0) ...
+    const double cx = (q & 3) == 3 ? -h : c;
+    return q & 4 ? make_double2(-cx, -s) : make_double2(cx, s);
+}
+
+// ---------------------------------------------------------------------------------
+// what one CTA works on, shared by both directions
+// ---------------------------------------------------------------------------------
+struct RingArgs {
+    const RingUnit *units;
+    const RingDesc *rings;
+    int lmax, M, nrows, spin;  // nrows: rows per channel
+    long long npix;
+    const double2 *tw;     // e^{-2 pi i j / kTwLen}
+    const double2 *bh;     // chirp spectra
+    const double2 *ctab;   // per chirp length i: kRingCols columns of i factors
+    const double2 *belt;   // e^{i pi a / Nb}, a < 2 Nb, of the power-of-two belt
+    int belt_n;            // Nb
+};
+
+// the two rows and the two pixel streams of a transform
+struct Streams {
+    size_t rowP, rowM;      // element offsets of m = 0
+    long long offX, offY;   // pixel offsets; offY < 0: no second stream
+};
+__device__ __forceinline__ Streams streams_of(const RingArgs &a, int r, const RingDesc &rd) {
+    Streams s;
+    s.rowP = (size_t)r * a.M;
+    s.offX = rd.start;
+    if (a.spin) {
+        s.rowM = (size_t)(a.nrows + r) * a.M;
+        s.offY = a.npix + rd.start;
+    } else {
+        s.rowM = (size_t)(a.nrows - 1 - r) * a.M;
+        s.offY = rd.mirror;
+    }
+    return s;
+}
+
+// shared-memory slots of one ring's staged points: [class s mod 4][k] with the classes two
+// bank groups apart
+__device__ __forceinline__ int class_stride(int i) { return ((i + 5) & ~7) + 2; }  // >= i, = 2 mod 8
+
+// ring phase factor of a power-of-two ring: e^{i pi a / N} from the belt's table
+__device__ __forceinline__ double2 belt_phase(const RingArgs &a, int e, int N) {
+    const int i = (e & (2 * N - 1)) * (a.belt_n / N);
+    return JHTB_IN(i, 2 * a.belt_n, 107) ? __ldg(&a.belt[i]) : zero2();
+}
+
+// A point W'[k] = W[k] e^{-i pi k / N} (shifted) of a spectrum to every order it appears in:
+// P_{k+aN} = (-1)^a W'[k] and M_{aN-k} = (-1)^a conj(W'[k]) (a >= 1, and a = 0 for k = 0), the
+// signs for shifted rings only.
+__device__ __forceinline__ void scatter_orders(double2 *Pr, double2 *Mr, bool store_m, double2 w, int k, int N, int lmax,
+                                               bool shifted) {
+    double sg = 1.0;
+    const double flip = shifted ? -1.0 : 1.0;
+    for (int m = k; m <= lmax; m += N) {
+        if (JHTB_IN(m, lmax + 1, 105)) Pr[m] = make_double2(sg * w.x, sg * w.y);
+        sg *= flip;
+    }
+    if (!store_m) return;
+    sg = k ? flip : 1.0;
+    for (int m = k ? N - k : 0; m <= lmax; m += N) {
+        if (JHTB_IN(m, lmax + 1, 105)) Mr[m] = make_double2(sg * w.x, -sg * w.y);
+        sg *= flip;
     }
 }
 
-// D[k] of the synthesis fold without its ring phase (see fold_synth); one term per sum
-// when the ring is longer than lmax.
-__device__ __forceinline__ double2 fold_one(const double2 *__restrict__ Fp, const double2 *__restrict__ Fm, int k, int N,
-                                            int lmax, bool shifted) {
-    if (N <= lmax) return fold_synth(Fp, Fm, k, N, lmax, shifted);
-    const double2 fp = (k <= lmax && JHTB_IN(k, lmax + 1, 101)) ? Fp[k] : make_double2(0.0, 0.0);
-    const double2 fm = (k >= 1 && N - k <= lmax && JHTB_IN(N - k, lmax + 1, 102)) ? Fm[N - k] : make_double2(0.0, 0.0);
-    const double sg = shifted ? -1.0 : 1.0;
-    return make_double2(fma(sg, fm.x, fp.x), fma(-sg, fm.y, fp.y));
+// Every order of a ring from its staged spectrum W'(k), in order of m by all `nt` threads.
+template <typename Get>
+__device__ __forceinline__ void gather_orders(double2 *Pr, double2 *Mr, bool store_m, int N, int lmax, bool shifted,
+                                              int tid, int nt, Get W) {
+    const unsigned magic = (unsigned)((0x100000000ull + N - 1) / N);  // m / N = umulhi(m, magic) for m N < 2^32
+    for (int m = tid; m <= lmax; m += nt) {
+        const int a = (int)__umulhi((unsigned)m, magic), k = m - a * N;
+        const bool odd = shifted && (a & 1);
+        double2 p = W(k);
+        if (odd) p = make_double2(-p.x, -p.y);
+        if (JHTB_IN(m, lmax + 1, 105)) Pr[m] = p;
+        if (!store_m) continue;
+        double2 q = conjd(W(k ? N - k : 0));
+        if (shifted && (odd != (k != 0))) q = make_double2(-q.x, -q.y);
+        if (JHTB_IN(m, lmax + 1, 105)) Mr[m] = q;
+    }
 }
 
-template <int SPIN>
-__global__ void __launch_bounds__(kFftThreads, kPieceMinBlocks) ring_synth_piece_kernel(const int *__restrict__ piece_list,
-                                                                           const RingDesc *__restrict__ rings, int lmax,
-                                                                           int M, int nrings, long long npix,
-                                                                           const double2 *__restrict__ F_all,
-                                                                           double *__restrict__ maps_all,
-                                                                           const double2 *__restrict__ tw,
-                                                                           const double2 *__restrict__ bh) {
-    extern __shared__ double2 buf[];
-    double2 *T = buf + kFftBufLen;  // twiddle table after the FFT buffer
-    sm_tw_init(T);
-    const int code = piece_list[blockIdx.x];
-    const int r = code >> 3, s = code & 7;
-    const RingDesc rd = rings[r];
-    const int N = rd.N, Q = ring_pieces(rd), Lq = N / Q;
-    const bool split = rd.mode == kSplit4;
-    const bool shifted = rd.phi0 != 0.0;
-    const int c = (shifted ? 1 : 0) + 2 * s;  // term k carries e^{i pi c k / N} (ring phase and piece twiddle)
-    constexpr int nchan = SPIN ? 2 : 1;
-    const double2 *Fp = F_all + ((size_t)blockIdx.y * nchan * nrings + r) * M;
-    const double2 *Fm = SPIN ? Fp + (size_t)nrings * M : Fp;
-    double *outQ = maps_all + (size_t)blockIdx.y * nchan * npix + rd.start;
-    double *outU = outQ + npix;
-    const int bd = blockDim.x;
-    if (!split && Q == 2) {
-        // the belt's two-piece rings: 2 kUP values of k1 per thread and round (two loads each,
-        // all issued first), twiddles from the shared table
-        constexpr int U = 2 * kUP;
-        const double2 r1 = root8(2 * c);  // e^{i pi c / 2}: exactly +-1 or +-i
-        for (int k10 = threadIdx.x; k10 < Lq; k10 += U * bd) {
-            double2 d0[U], d1[U];
+__device__ __forceinline__ double2 load_pixel(const double *map, const Streams &s, long long npix, int nstream, int j) {
+    const double x = JHTB_IN(s.offX + j, npix * nstream, 103) ? map[s.offX + j] : 0.0;
+    const double y = s.offY >= 0 ? map[s.offY + j] : 0.0;
+    return make_double2(x, y);
+}
+__device__ __forceinline__ void store_pixel(double *map, const Streams &s, long long npix, int nstream, int j, double2 v) {
+    if (!JHTB_IN(s.offX + j, npix * nstream, 104)) return;
+    map[s.offX + j] = v.x;
+    if (s.offY >= 0) map[s.offY + j] = v.y;
+}
+
+// ---------------------------------------------------------------------------------
+// direct: power-of-two pieces of 2^LOGP points
+// ---------------------------------------------------------------------------------
+template <int LOGP, bool ADJ>
+__device__ __forceinline__ void direct_unit(const RingArgs &a, const RingUnit &u, const double2 *F, double2 *V,
+                                            const double *in, double *out, double2 *buf) {
+    using X = Fft<LOGP>;
+    const int g = threadIdx.x / X::TP, t = threadIdx.x % X::TP;  // ring of the unit, thread of its FFT
+    const bool on = g < u.n;
+    const int r = u.ring + (on ? g : 0), s = u.piece;
+    const RingDesc rd = a.rings[r];
+    const Streams st = streams_of(a, r, rd);
+    const int N = rd.N, Q = N >> LOGP, nstream = a.spin ? 2 : 1;
+    const bool sh = rd.shifted;
+    const double2 *tw = a.tw;
+    double2 v[16];
+    if (on) {
+        if constexpr (!ADJ) {
+            const double2 *Pr = F + st.rowP, *Mr = F + st.rowM;
+            const int c = (sh ? 1 : 0) + 2 * s;  // term k carries e^{i pi c k / N} (ring phase and piece twiddle)
+            // e^{i pi c (k1 + P k2) / N} = e^{i pi c k1 / N} e^{i pi c k2 / Q}
+            if (N > a.lmax) {
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int k1 = k10 + u * bd;
-                d0[u] = k1 < Lq ? fold_one(Fp, Fm, k1, N, lmax, shifted) : make_double2(0.0, 0.0);
-                d1[u] = k1 < Lq ? fold_one(Fp, Fm, k1 + Lq, N, lmax, shifted) : make_double2(0.0, 0.0);
+                for (int q = 0; q < 16; ++q) v[q] = fold_one(Pr, Mr, t + X::TP * q, N, a.lmax, sh);
+                for (int k2 = 1; k2 < Q; ++k2) {
+                    const double2 w = root8((4 / Q) * c * k2);
+#pragma unroll
+                    for (int q0 = 0; q0 < 16; q0 += 4) {
+                        double2 d[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) d[q] = fold_one(Pr, Mr, t + X::TP * (q0 + q) + X::P * k2, N, a.lmax, sh);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) v[q0 + q] = cadd(v[q0 + q], cmul(d[q], w));
+                    }
+                }
+            } else {  // aliased rings (lmax >= N) go through this thread's own buffer slots: one copy of the loop
+                double2 *fb = buf + g * X::LEN;
+#pragma unroll 1
+                for (int q = 0; q < 16; ++q) {
+                    const int k1 = t + X::TP * q;
+                    double2 d = fold_sum(Pr, Mr, k1, N, a.lmax, sh);
+#pragma unroll 1
+                    for (int k2 = 1; k2 < Q; ++k2)
+                        d = cadd(d, cmul(fold_sum(Pr, Mr, k1 + X::P * k2, N, a.lmax, sh), root8((4 / Q) * c * k2)));
+                    fb[X::template pos<0>(t, q)] = d;
+                }
+#pragma unroll
+                for (int q = 0; q < 16; ++q) v[q] = fb[X::template pos<0>(t, q)];
             }
+            if (c) {
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int k1 = k10 + u * bd;
-                if (k1 >= Lq) continue;
-                const double2 v = cmul(cadd(d0[u], cmul(d1[u], r1)), sm_tw_pi(T, (long long)c * k1, N));
-                if (JHTB_IN(pidx(k1), kFftBufLen, 106)) buf[pidx(k1)] = v;
+                for (int q = 0; q < 16; ++q) v[q] = cmul(v[q], belt_phase(a, c * (t + X::TP * q), N));
+            }
+        } else {  // the transform of the conjugate: sum_j conj(v_j) e^{+2 pi i j (Q k + s) / N} = conj(W[Q k + s])
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = conjd(load_pixel(in, st, a.npix, nstream, t + X::TP * q));
+            for (int j2 = 1; j2 < Q; ++j2) {
+                const double2 w = root8((8 / Q) * s * j2);
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+                    v[q] = cadd(v[q], cmul(conjd(load_pixel(in, st, a.npix, nstream, t + X::TP * q + X::P * j2)), w));
+            }
+            if (s) {
+#pragma unroll
+                for (int q = 0; q < 16; ++q) v[q] = cmul(v[q], belt_phase(a, 2 * s * (t + X::TP * q), N));
             }
         }
     }
-    // a_s[k1]: the Q aliases k1 + Lq k2 of the phased fold, kUP values of k1 per thread at a time
-    for (int k10 = threadIdx.x; k10 < Lq && (split || Q != 2); k10 += kUP * bd) {
-        double2 acc[kUP];
+    X::template forward<false>(v, buf + g * X::LEN, t, on, tw);
+    if (!on) return;
+    if constexpr (!ADJ) {
 #pragma unroll
-        for (int u = 0; u < kUP; ++u) acc[u] = make_double2(0.0, 0.0);
-        // every load of the kUP x Q terms (and, for a power of two, of the kUP twiddles) is
-        // issued before the first is used
-        double2 d[kMaxPieces][kUP], w1[kUP];
+        for (int q = 0; q < 16; ++q) store_pixel(out, st, a.npix, nstream, Q * X::out_index(t, q) + s, v[q]);
+    } else {
+        double2 *Pr = V + st.rowP, *Mr = V + st.rowM;
 #pragma unroll
-        for (int k2 = 0; k2 < kMaxPieces; ++k2)
-#pragma unroll
-            for (int u = 0; u < kUP; ++u) {
-                const int k1 = k10 + u * bd;
-                d[k2][u] = (k2 < Q && k1 < Lq) ? fold_one(Fp, Fm, k1 + Lq * k2, N, lmax, shifted) : make_double2(0.0, 0.0);
-            }
-#pragma unroll
-        for (int u = 0; u < kUP; ++u) {
-            const int k1 = k10 + u * bd;
-            w1[u] = (!split && k1 < Lq) ? tw_pi(tw, (long long)c * k1, N) : make_double2(1.0, 0.0);
-        }
-        // e^{i pi c (k1 + Lq k2) / N} = e^{i pi c k1 / N} e^{i pi c k2 / Q}: the k2 factor is an
-        // eighth root of unity (exactly +-1, +-i for Q = 2), the k1 factor is applied once
-#pragma unroll
-        for (int k2 = 0; k2 < kMaxPieces; ++k2) {
-            if (k2 >= Q) break;
-            const double2 w = root8((4 / Q) * c * k2);
-#pragma unroll
-            for (int u = 0; u < kUP; ++u) acc[u] = cadd(acc[u], k2 ? cmul(d[k2][u], w) : d[k2][u]);
-        }
-#pragma unroll
-        for (int u = 0; u < kUP; ++u) {
-            const int k1 = k10 + u * bd;
-            if (k1 >= Lq) continue;
-            // power of two: e^{i pi c k1 / N} from the table; kSplit4: e^{i pi c k1 / N} times the
-            // chirp w(k1) = e^{i pi k1^2 / Lq} = e^{i pi 4 k1^2 / N}, one exactly reduced argument
-            const double2 v = split ? cmul(acc[u], cis_pi((int)(((long long)c * k1 + 4LL * k1 * k1) % (2LL * N)), N, 0, 1))
-                                    : cmul(acc[u], w1[u]);
-            if (JHTB_IN(pidx(k1), kFftBufLen, 106)) buf[pidx(k1)] = v;
-        }
-    }
-    const int L = split ? rd.P : Lq;
-    for (int k = Lq + threadIdx.x; k < L; k += bd) buf[pidx(k)] = make_double2(0.0, 0.0);
-    __syncthreads();
-    if (split) {  // E[j] = w(j) sum_k (a[k] w(k)) conj(w(j - k)): FFT, chirp spectrum, inverse FFT
-        fft_stockham_sm(buf, L, -1.0, T);
-        for (int q0 = threadIdx.x; q0 < L; q0 += kUP * bd) {
-            double2 w[kUP];
-#pragma unroll
-            for (int u = 0; u < kUP; ++u) w[u] = q0 + u * bd < L ? bh_get(bh + rd.bh_off, L, q0 + u * bd, 1) : make_double2(0.0, 0.0);
-#pragma unroll
-            for (int u = 0; u < kUP; ++u)
-                if (q0 + u * bd < L) buf[pidx(q0 + u * bd)] = cmul(buf[pidx(q0 + u * bd)], w[u]);
-        }
-        __syncthreads();
-    }
-    fft_stockham_sm(buf, L, +1.0, T);
-    for (int j = threadIdx.x; j < Lq; j += bd) {
-        double2 v = buf[pidx(j)];
-        if (split) v = cmul(v, cis_pi((int)(((long long)j * j) % (2 * Lq)), Lq, 0, 1));
-        if (JHTB_IN(rd.start + (long long)Q * j + s, npix, 104)) {
-            outQ[(size_t)Q * j + s] = v.x;
-            if (SPIN) outU[(size_t)Q * j + s] = v.y;
+        for (int q = 0; q < 16; ++q) {
+            const int k = Q * X::out_index(t, q) + s;
+            const double2 w = conjd(sh ? cmul(v[q], belt_phase(a, k, N)) : v[q]);
+            scatter_orders(Pr, Mr, st.rowM != st.rowP, w, k, N, a.lmax, sh);
         }
     }
 }
 
-template <int SPIN>
-__global__ void __launch_bounds__(kFftThreads, kPieceMinBlocks) ring_adjoint_piece_kernel(const int *__restrict__ piece_list,
-                                                                             const RingDesc *__restrict__ rings, int lmax,
-                                                                             int M, int nrings, long long npix,
-                                                                             const double *__restrict__ maps_all,
-                                                                             double2 *__restrict__ V_all,
-                                                                             const double2 *__restrict__ tw,
-                                                                             const double2 *__restrict__ bh) {
-    extern __shared__ double2 buf[];
-    double2 *T = buf + kFftBufLen;  // twiddle table after the FFT buffer
-    sm_tw_init(T);
-    const int code = piece_list[blockIdx.x];
-    const int r = code >> 3, s = code & 7;
-    const RingDesc rd = rings[r];
-    const int N = rd.N, Q = ring_pieces(rd), Lq = N / Q;
-    const bool split = rd.mode == kSplit4;
-    const bool shifted = rd.phi0 != 0.0;
-    constexpr int nchan = SPIN ? 2 : 1;
-    const double *inQ = maps_all + (size_t)blockIdx.y * nchan * npix + rd.start;
-    const double *inU = inQ + npix;
-    double2 *Vp = V_all + ((size_t)blockIdx.y * nchan * nrings + r) * M;
-    double2 *Vm = SPIN ? Vp + (size_t)nrings * M : Vp;
-    const int bd = blockDim.x;
-    if (!split && Q == 2) {
-        // the belt's two-piece rings: 2 kUP values of j1 per thread and round (all loads first),
-        // twiddles from the shared table
-        constexpr int U = 2 * kUP;
-        const double sg = (s & 1) ? -1.0 : 1.0;  // e^{-2 pi i s j2 / 2} = (-1)^(s j2)
-        for (int j10 = threadIdx.x; j10 < Lq; j10 += U * bd) {
-            double2 a0[U], a1[U];
+// ---------------------------------------------------------------------------------
+// chirp: rings of N = 4 i points as four chirp-z transforms of length i
+// ---------------------------------------------------------------------------------
+// PPC pieces of 2^LOGP points of one ring per group of PPC * TP threads.  With
+// D[k1 + i k2] the (phased) input, piece s transforms
+//   a_s[k1] = in_s[k1] sum_{k2 < 4} i^{s k2} D[k1 + i k2],
+// in_s the table column that joins the piece twiddle, the ring phase and the chirp; the
+// result y[j] gets its last chirp factor from another column (kRingCols in the header).
+// Where a CTA holds all four pieces (i <= 512) the ring's points are staged in shared memory
+// on the way in and out, so that global accesses run in order; with two pieces on the way in
+// only; with one they are read from global memory (through L2) by every piece.
+template <int LOGP, int PPC, bool ADJ>
+__device__ __forceinline__ void chirp_unit(const RingArgs &a, const RingUnit &u, const double2 *F, double2 *V,
+                                           const double *in, double *out, double2 *buf) {
+    using X = Fft<LOGP>;
+    constexpr int GT = X::TP * PPC;  // threads of one ring
+    const int g = threadIdx.x / GT, tg = threadIdx.x % GT;
+    const int s = u.piece + tg / X::TP, t = tg % X::TP;
+    const bool on = g < u.n;
+    const int r = u.ring + (on ? g : 0);
+    const RingDesc rd = a.rings[r];
+    const Streams st = streams_of(a, r, rd);
+    const int N = rd.N, i = N >> 2, nstream = a.spin ? 2 : 1;
+    const bool sh = rd.shifted;
+    const double2 *ct = a.ctab + rd.ctab_off;
+    double2 *rb = buf + g * PPC * X::LEN;  // this ring's part of the buffer
+    const double2 *Pr = F + st.rowP, *Mr = F + st.rowM;
+    // e^{i pi k2 / 4}: the part of the ring phase that depends on the quarter
+    auto quarter = [&](double2 d, int k2) {
+        if (ADJ || !sh) return d;
+        return k2 == 0 ? d : cmul(d, root8(k2));
+    };
+    const int cs = class_stride(i);
+    if (PPC >= 2) {  // stage the ring's points, quarter after quarter
+        if (on) {
+            constexpr int U = 4;
+            if (!ADJ && N <= a.lmax) {
+#pragma unroll 1
+                for (int k = tg; k < N; k += GT)
+                    rb[k] = quarter(fold_sum(Pr, Mr, k, N, a.lmax, sh), (k >= i) + (k >= 2 * i) + (k >= 3 * i));
+            } else for (int k0 = tg; k0 < N; k0 += U * GT) {
+                double2 d[U];
+                if (ADJ) {
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int j = j10 + u * bd;
-                const bool ok = j < Lq && JHTB_IN(rd.start + j + Lq, npix, 103);
-                a0[u] = ok ? make_double2(inQ[j], SPIN ? inU[j] : 0.0) : make_double2(0.0, 0.0);
-                a1[u] = ok ? make_double2(inQ[j + Lq], SPIN ? inU[j + Lq] : 0.0) : make_double2(0.0, 0.0);
-            }
+                    for (int e = 0; e < U; ++e)
+                        d[e] = k0 + e * GT < N ? conjd(load_pixel(in, st, a.npix, nstream, k0 + e * GT)) : zero2();
+                } else {
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int j1 = j10 + u * bd;
-                if (j1 >= Lq) continue;
-                const double2 v = cmul(make_double2(fma(sg, a1[u].x, a0[u].x), fma(sg, a1[u].y, a0[u].y)),
-                                       sm_tw_pi(T, -2LL * s * j1, N));
-                if (JHTB_IN(pidx(j1), kFftBufLen, 106)) buf[pidx(j1)] = v;
-            }
-        }
-    }
-    // b_s[j1]: the Q pixels j1 + Lq j2 with e^{-2 pi i s j / N}
-    for (int j10 = threadIdx.x; j10 < Lq && (split || Q != 2); j10 += kUP * bd) {
-        double2 acc[kUP];
+                    for (int e = 0; e < U; ++e)
+                        d[e] = k0 + e * GT < N ? fold_one(Pr, Mr, k0 + e * GT, N, a.lmax, sh) : zero2();
+                }
 #pragma unroll
-        for (int u = 0; u < kUP; ++u) acc[u] = make_double2(0.0, 0.0);
-        double2 a[kMaxPieces][kUP], w1[kUP];  // every load issued before the first is used
-#pragma unroll
-        for (int j2 = 0; j2 < kMaxPieces; ++j2)
-#pragma unroll
-            for (int u = 0; u < kUP; ++u) {
-                const int j = j10 + u * bd + Lq * j2;
-                a[j2][u] = (j2 < Q && j10 + u * bd < Lq && JHTB_IN(rd.start + j, npix, 103)) ? make_double2(inQ[j], SPIN ? inU[j] : 0.0)
-                                                                                            : make_double2(0.0, 0.0);
-            }
-#pragma unroll
-        for (int u = 0; u < kUP; ++u) {
-            const int j1 = j10 + u * bd;
-            w1[u] = (!split && j1 < Lq) ? tw_pi(tw, -2LL * s * j1, N) : make_double2(1.0, 0.0);
-        }
-        // e^{-2 pi i s (j1 + Lq j2) / N} = e^{-2 pi i s j1 / N} e^{-2 pi i s j2 / Q}: the j2 factor
-        // is a fourth root of unity (exact), the j1 factor is applied once
-#pragma unroll
-        for (int j2 = 0; j2 < kMaxPieces; ++j2) {
-            if (j2 >= Q) break;
-            const double2 w = root8(-(8 / Q) * s * j2);
-#pragma unroll
-            for (int u = 0; u < kUP; ++u) acc[u] = cadd(acc[u], j2 ? cmul(a[j2][u], w) : a[j2][u]);
-        }
-#pragma unroll
-        for (int u = 0; u < kUP; ++u) {
-            const int j1 = j10 + u * bd;
-            if (j1 >= Lq) continue;
-            // power of two: e^{-2 pi i s j1 / N} from the table; kSplit4: times the chirp
-            // conj(w(j1)) = e^{-i pi 4 j1^2 / N}, one exactly reduced argument
-            const double2 v = split ? cmul(acc[u], cis_pi(-(int)(((long long)2 * s * j1 + 4LL * j1 * j1) % (2LL * N)), N, 0, 1))
-                                    : cmul(acc[u], w1[u]);
-            if (JHTB_IN(pidx(j1), kFftBufLen, 106)) buf[pidx(j1)] = v;
-        }
-    }
-    const int L = split ? rd.P : Lq;
-    for (int k = Lq + threadIdx.x; k < L; k += bd) buf[pidx(k)] = make_double2(0.0, 0.0);
-    __syncthreads();
-    fft_stockham_sm(buf, L, -1.0, T);
-    if (split) {  // W[k] = conj(w(k)) sum_j (b[j] conj(w(j))) w(k - j)
-        for (int q0 = threadIdx.x; q0 < L; q0 += kUP * bd) {
-            double2 w[kUP];
-#pragma unroll
-            for (int u = 0; u < kUP; ++u) w[u] = q0 + u * bd < L ? bh_get(bh + rd.bh_off, L, q0 + u * bd, -1) : make_double2(0.0, 0.0);
-#pragma unroll
-            for (int u = 0; u < kUP; ++u)
-                if (q0 + u * bd < L) buf[pidx(q0 + u * bd)] = cmul(buf[pidx(q0 + u * bd)], w[u]);
-        }
-        __syncthreads();
-        fft_stockham_sm(buf, L, +1.0, T);
-        for (int k = threadIdx.x; k < Lq; k += bd)
-            buf[pidx(k)] = cmul(buf[pidx(k)], cis_pi(-(int)(((long long)k * k) % (2 * Lq)), Lq, 0, 1));
-        __syncthreads();
-    }
-    // V rows: Vp[m] = W[m mod N] for m = s (mod Q), Vm[m] = conj(W[-m mod N]) for m = -s (mod Q),
-    // both times e^{-i m phi0} (gather_adjoint, restricted to this piece's residue class)
-    const int sm = (Q - s) % Q;
-    for (int m0 = threadIdx.x * Q; m0 <= lmax; m0 += kUP * bd * Q) {
-#pragma unroll
-        for (int u = 0; u < kUP; ++u) {
-            const int mp = m0 + u * bd * Q + s;  // Vp orders
-            if (mp <= lmax) {
-                const int kp = (mp % N - s) / Q;
-                double2 p = JHTB_IN(kp, Lq, 106) ? buf[pidx(kp)] : make_double2(0.0, 0.0);
-                if (shifted) p = cmul(p, split ? cis_pi(-(mp % (2 * N)), N, 0, 1) : tw_pi(tw, -(long long)mp, N));
-                if (JHTB_IN(mp, M, 105)) Vp[mp] = p;
-            }
-            if (SPIN) {
-                const int mm = m0 + u * bd * Q + sm;  // Vm orders
-                if (mm <= lmax) {
-                    const int k = (N - mm % N) % N;
-                    const int kq = (k - s) / Q;
-                    double2 q = JHTB_IN(kq, Lq, 106) ? conjd(buf[pidx(kq)]) : make_double2(0.0, 0.0);
-                    if (shifted) q = cmul(q, split ? cis_pi(-(mm % (2 * N)), N, 0, 1) : tw_pi(tw, -(long long)mm, N));
-                    if (JHTB_IN(mm, M, 105)) Vm[mm] = q;
+                for (int e = 0; e < U; ++e) {
+                    const int k = k0 + e * GT;
+                    if (k < N) rb[k] = quarter(d[e], (k >= i) + (k >= 2 * i) + (k >= 3 * i));
                 }
             }
         }
+        __syncthreads();
+    }
+    double2 v[16];
+    const double2 *win = ct + (ADJ ? (size_t)(kColAdjIn + s) : (size_t)((sh ? kColSynth : kColAdjIn) + s)) * i;
+    double2 *fb = rb + (tg / X::TP) * X::LEN;
+    if (on) {
+        const bool odd = s & 1;
+        const double sn = s & 2 ? -1.0 : 1.0;
+        // sum_{k2} i^{s k2} d[k2] = (d0 +- d2) + i^s (d1 +- d3)
+        auto combine = [&](const double2 (&d)[4]) {
+            const double2 e = odd ? csub(d[0], d[2]) : cadd(d[0], d[2]);
+            const double2 o = odd ? csub(d[1], d[3]) : cadd(d[1], d[3]);
+            return cadd(e, odd ? make_double2(-sn * o.y, sn * o.x) : make_double2(sn * o.x, sn * o.y));
+        };
+        if (PPC == 1 && !ADJ && N <= a.lmax) {  // aliased: through this thread's own buffer slots, one copy of the loop
+#pragma unroll 1
+            for (int q = 0; q < 8; ++q) {
+                const int k1 = t + X::TP * q;
+                if (k1 >= i) continue;
+                double2 d[4];
+#pragma unroll 1
+                for (int k2 = 0; k2 < 4; ++k2) {
+                    const double2 f = quarter(fold_sum(Pr, Mr, k1 + i * k2, N, a.lmax, sh), k2);
+                    if (k2 == 3) d[3] = f;
+                    else if (k2 == 2) d[2] = f;
+                    else if (k2 == 1) d[1] = f;
+                    else d[0] = f;
+                }
+                fb[X::template pos<0>(t, q)] = combine(d);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int k1 = t + X::TP * q;
+            if (k1 < i) {
+                double2 x;
+                if (PPC == 1 && !ADJ && N <= a.lmax) {
+                    x = fb[X::template pos<0>(t, q)];
+                } else {
+                    double2 d[4];
+#pragma unroll
+                    for (int k2 = 0; k2 < 4; ++k2) {
+                        const int k = k1 + i * k2;
+                        if (PPC >= 2) d[k2] = rb[k];
+                        else if (ADJ) d[k2] = conjd(load_pixel(in, st, a.npix, nstream, k));
+                        else d[k2] = quarter(fold_one(Pr, Mr, k, N, a.lmax, sh), k2);
+                    }
+                    x = combine(d);
+                }
+                v[q] = cmul(x, __ldg(&win[k1]));
+            } else {
+                v[q] = zero2();
+            }
+        }
+    }
+    if (PPC >= 2) __syncthreads();  // the staged points are read: the buffer is free
+    X::template forward<true>(v, fb, t, on, a.tw);
+    if (on) {
+        const double2 *B = a.bh + rd.bh_off;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = cmul(v[q], __ldg(&B[X::out_index(t, q)]));
+    }
+    X::backward(v, fb, t, on, a.tw);
+    // y[j] times the last chirp factor: pixel 4 j + s, or conj -> W'[4 j + s]
+    const double2 *wout = ct + (ADJ ? (size_t)(sh ? kColAdjOut + s : kColAdjIn) : (size_t)kColAdjIn) * i;
+    if (PPC == 4) {
+        __syncthreads();  // every thread has read its last points
+        if (on) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int j = t + X::TP * q;
+                if (j < i) {
+                    const double2 w = cmul(v[q], __ldg(&wout[j]));
+                    rb[s * cs + j] = ADJ ? conjd(w) : w;
+                }
+            }
+        }
+        __syncthreads();
+        if (!on) return;
+        if (!ADJ) {
+            for (int j = tg; j < N; j += GT) store_pixel(out, st, a.npix, nstream, j, rb[(j & 3) * cs + (j >> 2)]);
+        } else {
+            gather_orders(V + st.rowP, V + st.rowM, st.rowM != st.rowP, N, a.lmax, sh, tg, GT,
+                          [&](int k) { return rb[(k & 3) * cs + (k >> 2)]; });
+        }
+        return;
+    }
+    if (!on) return;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int j = t + X::TP * q;
+        if (j >= i) continue;
+        const double2 w = cmul(v[q], __ldg(&wout[j]));
+        if (!ADJ) store_pixel(out, st, a.npix, nstream, 4 * j + s, w);
+        else scatter_orders(V + st.rowP, V + st.rowM, st.rowM != st.rowP, conjd(w), 4 * j + s, N, a.lmax, sh);
     }
 }
 
-// One block per (Bluestein length, piece): Bh+[Q q + s] = (1/P) sum_n b[n] e^{-2 pi i (Qq+s) n / P}.
-__global__ void __launch_bounds__(kFftThreads) bluestein_setup_kernel(const int *__restrict__ lens,
-                                                                       const long long *__restrict__ offs,
-                                                                       const double2 *__restrict__ tw,
-                                                                       double2 *__restrict__ bh) {
-    extern __shared__ double2 buf[];
-    const int N = lens[blockIdx.x];
-    int P = 1;
-    while (P < 2 * N - 1) P <<= 1;
-    const int Q = P > kFftPiece ? P / kFftPiece : 1;
-    const int s = blockIdx.y;
-    if (s >= Q) return;
-    const int Pp = P / Q;
-    double2 *out = bh + offs[blockIdx.x];
-    for (int q = threadIdx.x; q < Pp; q += blockDim.x) {
-        double2 v = make_double2(0.0, 0.0);
-        for (int idx = q; idx < P; idx += Pp) {
-            // circular kernel: b[idx] = conj(w(n)) with n = idx (idx < N) or idx - P (idx > P - N)
-            long long n;
-            if (idx < N) n = idx;
-            else if (idx > P - N) n = (long long)P - idx;  // w(-n) = w(n)
-            else continue;
-            double2 b = conjd(chirp(n, N, 1.0));
-            if (s) b = cmul(b, root((long long)s * idx, P, -1.0));
-            v = cadd(v, b);
+// ---------------------------------------------------------------------------------
+// small: N <= kSmallRing points, one ring per CTA, a plain sum over k
+// ---------------------------------------------------------------------------------
+template <bool ADJ>
+__device__ __forceinline__ void small_unit(const RingArgs &a, const RingUnit &u, const double2 *F, double2 *V,
+                                           const double *in, double *out, double2 *buf) {
+    constexpr int NT = kRingThreads;
+    const int r = u.ring;
+    const RingDesc rd = a.rings[r];
+    const Streams st = streams_of(a, r, rd);
+    const int N = rd.N, n2 = 2 * N, nstream = a.spin ? 2 : 1;
+    const bool sh = rd.shifted;
+    double2 *root = buf, *D = buf + 2 * kSmallRing, *part = D + kSmallRing;  // part: NT slots
+    if ((int)threadIdx.x < n2) root[threadIdx.x] = cis_pi(threadIdx.x, N);
+    const int parts = NT / N;  // >= 2
+    const int k = threadIdx.x % N, p = threadIdx.x / N;
+    if (ADJ) {
+        if (p == 0) D[k] = load_pixel(in, st, a.npix, nstream, k);
+        __syncthreads();
+    } else {
+        // the aliases of each k split over the ring's parts, summed in a fixed order
+        if (p < parts) part[threadIdx.x] = fold_sum(F + st.rowP, F + st.rowM, k, N, a.lmax, sh, p, parts);
+        __syncthreads();
+        if (p == 0) {
+            double2 d = part[k];
+            for (int q = 1; q < parts; ++q) d = cadd(d, part[q * N + k]);
+            D[k] = d;
         }
-        buf[pidx(q)] = v;
+        __syncthreads();
+    }
+    // output k (pixel j or spectrum index): sum over e = p, p + parts, ... of D[e] times the root
+    // of index (2 k + sh) e mod 2 N (synthesis, phase e^{i pi e / N} of a shifted ring included) or
+    // -2 k e (adjoint)
+    if (p < parts) {
+        double2 acc = zero2();
+        const int step1 = ADJ ? (n2 - 2 * k) % n2 : (2 * k + (sh ? 1 : 0)) % n2;
+        int idx = (int)((long long)step1 * p % n2);
+        const int step = (int)((long long)step1 * parts % n2);
+        for (int e = p; e < N; e += parts) {
+            const double2 d = D[e], w = root[idx];
+            acc.x = fma(d.x, w.x, fma(-d.y, w.y, acc.x));
+            acc.y = fma(d.x, w.y, fma(d.y, w.x, acc.y));
+            idx += step;
+            if (idx >= n2) idx -= n2;
+        }
+        part[threadIdx.x] = acc;
     }
     __syncthreads();
-    fft_stockham(buf, Pp, -1.0, tw);
-    const double inv = 1.0 / (double)P;
-    for (int q = threadIdx.x; q < Pp; q += blockDim.x) {
-        const double2 v = buf[pidx(q)];
-        out[(long long)Q * q + s] = make_double2(v.x * inv, v.y * inv);
+    if (p == 0) {
+        double2 d = part[k];
+        for (int q = 1; q < parts; ++q) d = cadd(d, part[q * N + k]);
+        if (!ADJ) store_pixel(out, st, a.npix, nstream, k, d);
+        else D[k] = sh ? cmulc(d, root[k]) : d;  // W'[k]
+    }
+    if (!ADJ) return;
+    __syncthreads();
+    gather_orders(V + st.rowP, V + st.rowM, st.rowM != st.rowP, N, a.lmax, sh, threadIdx.x, NT, [&](int q) { return D[q]; });
+}
+
+template <bool ADJ>
+__device__ __forceinline__ void ring_unit(const RingArgs &a, const RingUnit &u, const double2 *F, double2 *V,
+                                          const double *in, double *out, double2 *buf) {
+    switch (u.cls) {
+        case kClsDirect + 8: direct_unit<8, ADJ>(a, u, F, V, in, out, buf); break;
+        case kClsDirect + 9: direct_unit<9, ADJ>(a, u, F, V, in, out, buf); break;
+        case kClsDirect + 10: direct_unit<10, ADJ>(a, u, F, V, in, out, buf); break;
+        case kClsDirect + 11: direct_unit<11, ADJ>(a, u, F, V, in, out, buf); break;
+        case kClsDirect + 12: direct_unit<12, ADJ>(a, u, F, V, in, out, buf); break;
+        case kClsChirp + 7: chirp_unit<7, 4, ADJ>(a, u, F, V, in, out, buf); break;
+        case kClsChirp + 8: chirp_unit<8, 4, ADJ>(a, u, F, V, in, out, buf); break;
+        case kClsChirp + 9: chirp_unit<9, 4, ADJ>(a, u, F, V, in, out, buf); break;
+        case kClsChirp + 10: chirp_unit<10, 4, ADJ>(a, u, F, V, in, out, buf); break;
+        case kClsChirp + 11: chirp_unit<11, 2, ADJ>(a, u, F, V, in, out, buf); break;
+        case kClsChirp + 12: chirp_unit<12, 1, ADJ>(a, u, F, V, in, out, buf); break;
+        default: small_unit<ADJ>(a, u, F, V, in, out, buf); break;
     }
 }
 
-int smem_bytes() { return kFftBufLen * (int)sizeof(double2); }
-int smem_bytes_piece() { return (kFftBufLen + kSmTwLen) * (int)sizeof(double2); }
+// One CTA per work unit and map, every class in one launch.  256 threads with up to 128
+// registers (16 complex points and their twiddles) and 74 KB of shared memory, two CTAs per SM.
+// Bound by instruction issue and L2 latency, not by HBM: the spectra and pixels of one spin-2
+// map at nside 1024 / lmax 2048 (0.47 GB) take 0.07 ms at 6.65 TB/s.  An earlier form (radix-16
+// passes of one generic length, a twiddle of two table entries per point, a sincospi per chirp
+// factor, every spin-0 ring by itself) issued 4000 instructions per thread for 16 points.
+// Measured, synthesis + adjoint, earlier -> this form: nside 1024 / lmax 2048, spin 2, one map
+// 0.62 + 0.58 -> 0.32 + 0.32 ms; nside 512 / lmax 1024, spin 0, 64 maps 9.42 + 9.48 -> 2.15 + 2.27 ms
+// (4.3x, of which 2x is the pairing); nside 2048 / lmax 4096, spin 2, 2.58 + 2.09 -> 1.39 + 1.20 ms.
+__global__ void __launch_bounds__(kRingThreads, 2) ring_synth_kernel(RingArgs a, const double2 *__restrict__ F,
+                                                                     double *__restrict__ maps, size_t fmap,
+                                                                     long long pmap) {
+    extern __shared__ double2 buf[];
+    const RingUnit u = a.units[blockIdx.x];
+    ring_unit<false>(a, u, F + blockIdx.y * fmap, nullptr, nullptr, maps + blockIdx.y * pmap, buf);
+}
+__global__ void __launch_bounds__(kRingThreads, 2) ring_adjoint_kernel(RingArgs a, const double *__restrict__ maps,
+                                                                       double2 *__restrict__ V, size_t fmap,
+                                                                       long long pmap) {
+    extern __shared__ double2 buf[];
+    const RingUnit u = a.units[blockIdx.x];
+    ring_unit<true>(a, u, V + blockIdx.y * fmap, V + blockIdx.y * fmap, maps + blockIdx.y * pmap, nullptr, buf);
+}
+// Chirp-z transforms of 8192 points (rings above 8192 points that are no power of two, nside >
+// 2048): 512 threads and 139 KB of shared memory.
+template <bool ADJ>
+__global__ void __launch_bounds__(512, 1) ring_long_kernel(RingArgs a, const double2 *__restrict__ F, double2 *__restrict__ V,
+                                                           const double *__restrict__ in, double *__restrict__ out,
+                                                           size_t fmap, long long pmap) {
+    extern __shared__ double2 buf[];
+    const RingUnit u = a.units[blockIdx.x];
+    chirp_unit<13, 1, ADJ>(a, u, ADJ ? nullptr : F + blockIdx.y * fmap, ADJ ? V + blockIdx.y * fmap : nullptr,
+                           ADJ ? in + blockIdx.y * pmap : nullptr, ADJ ? nullptr : out + blockIdx.y * pmap, buf);
+}
+
+// ---------------------------------------------------------------------------------
+// tables (plan creation)
+// ---------------------------------------------------------------------------------
+// The factor columns of one chirp length i (N = 4 i), every entry e^{i pi a / N}:
+//   kColAdjIn + s    a = 2 s k + 4 k^2             (s = 0: the chirp itself)
+//   kColSynth + s    a = (1 + 2 s) k + 4 k^2
+//   kColAdjOut + s   a = 4 k^2 + 4 k + s
+__global__ void ring_table_kernel(const int *__restrict__ lens, const long long *__restrict__ offs, double2 *__restrict__ tab) {
+    const int i = lens[blockIdx.x];
+    double2 *out = tab + offs[blockIdx.x];
+    const int s = blockIdx.y & 3, what = blockIdx.y >> 2;
+    for (int k = threadIdx.x; k < i; k += blockDim.x) {
+        const long long kk = 4LL * k * k;
+        const long long e = what == 0 ? 2LL * s * k + kk : what == 1 ? (1 + 2LL * s) * k + kk : kk + 4LL * k + s;
+        out[(size_t)blockIdx.y * i + k] = cis_pi(e, 4 * i);
+    }
+}
+static_assert(kColAdjIn == 0 && kColSynth == 4 && kColAdjOut == 8 && kRingCols == 12, "column order of ring_table_kernel");
+
+// e^{i pi a / N}, a < 2 N
+__global__ void belt_table_kernel(int N, double2 *__restrict__ tab) {
+    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a < 2 * N) tab[a] = cis_pi(a, N);
+}
+
+// Chirp spectrum of length i at P = 2^LOGP points: the transform of conj(w(n)) on |n| < i,
+// w(n) = e^{i pi n^2 / i}, divided by P.  One CTA per length of this P.
+template <int LOGP>
+__global__ void __launch_bounds__(Fft<LOGP>::TP < 32 ? 32 : Fft<LOGP>::TP) chirp_spectrum_kernel(
+    const int *__restrict__ lens, const long long *__restrict__ offs, const double2 *__restrict__ tw, double2 *__restrict__ bh) {
+    using X = Fft<LOGP>;
+    extern __shared__ double2 buf[];
+    const int i = lens[blockIdx.x], t = threadIdx.x;
+    const bool on = t < X::TP;
+    double2 v[16];
+    if (on) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const int p = t + X::TP * q;
+            const int n = p < i ? p : X::P - p;  // w(-n) = w(n)
+            v[q] = (p < i || n < i) ? conjd(cis_pi((long long)n * n, i)) : zero2();
+        }
+    }
+    X::template forward<false>(v, buf, t, on, tw);
+    if (!on) return;
+    double2 *out = bh + offs[blockIdx.x];
+    const double inv = 1.0 / (double)X::P;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) out[X::out_index(t, q)] = make_double2(v[q].x * inv, v[q].y * inv);
+}
 
 template <typename K>
-int ensure_smem(K kernel, int bytes = smem_bytes()) {
+int ensure_smem(K kernel, int bytes) {
     JHTB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     return JHTB_OK;
 }
 
-template <int SPIN>
-int launch_ring_synth_t(const Plan &p, const double2 *F, double *maps, int nb, cudaStream_t s) {
-    int rc;
-    if (p.nring_small > 0) {
-        if ((rc = ensure_smem(ring_synth_kernel<SPIN>))) return rc;
-        ring_synth_kernel<SPIN><<<dim3(p.nring_small, nb), kFftThreads, smem_bytes(), s>>>(
-            p.d_ring_small, p.d_rings, p.lmax, p.M, p.nrings, p.npix, F, maps, p.d_W, p.d_W2, p.d_tw, p.d_bh);
-        JHTB_CUDA_TRY(cudaGetLastError());
-    }
-    if (p.nring_piece > 0) {
-        if ((rc = ensure_smem(ring_synth_piece_kernel<SPIN>, smem_bytes_piece()))) return rc;
-        ring_synth_piece_kernel<SPIN><<<dim3(p.nring_piece, nb), kFftThreads, smem_bytes_piece(), s>>>(
-            p.d_ring_piece, p.d_rings, p.lmax, p.M, p.nrings, p.npix, F, maps, p.d_tw, p.d_bh);
-        JHTB_CUDA_TRY(cudaGetLastError());
-    }
-    return JHTB_OK;
+RingArgs make_args(const Plan &p) {
+    RingArgs a{};
+    a.rings = p.d_rings;
+    a.lmax = p.lmax;
+    a.M = p.M;
+    a.nrows = p.nrings;
+    a.spin = p.spin;
+    a.npix = p.npix;
+    a.tw = p.d_tw;
+    a.bh = p.d_bh;
+    a.ctab = p.d_ctab;
+    a.belt = p.d_belt;
+    a.belt_n = p.belt_n;
+    return a;
 }
 
-template <int SPIN>
-int launch_ring_adjoint_t(const Plan &p, const double *maps, double2 *V, double2 *W, int nb, cudaStream_t s) {
+// shared memory of the unit kernels: the largest layout of the classes (chirp 128-point pieces)
+template <int LOGP>
+constexpr int class_slots(int transforms) { return transforms * Fft<LOGP>::LEN; }
+constexpr int kRingSlots = std::max({class_slots<12>(1), class_slots<11>(2), class_slots<10>(4), class_slots<9>(8),
+                                     class_slots<8>(16), class_slots<7>(32), 3 * kSmallRing + kRingThreads});
+constexpr int kRingSmem = kRingSlots * (int)sizeof(double2);
+constexpr int kLongSmem = Fft<13>::LEN * (int)sizeof(double2);
+
+template <int LOGP>
+int launch_spectrum(const int *lens, const long long *offs, int n, const double2 *tw, double2 *bh, cudaStream_t s) {
+    using X = Fft<LOGP>;
+    if (n <= 0) return JHTB_OK;
+    const int smem = X::LEN * (int)sizeof(double2);
     int rc;
-    if (p.nring_small > 0) {
-        if ((rc = ensure_smem(ring_adjoint_kernel<SPIN>))) return rc;
-        ring_adjoint_kernel<SPIN><<<dim3(p.nring_small, nb), kFftThreads, smem_bytes(), s>>>(
-            p.d_ring_small, p.d_rings, p.lmax, p.M, p.nrings, p.npix, maps, V, p.d_W2, W, p.d_tw, p.d_bh);
-        JHTB_CUDA_TRY(cudaGetLastError());
-    }
-    if (p.nring_piece > 0) {
-        if ((rc = ensure_smem(ring_adjoint_piece_kernel<SPIN>, smem_bytes_piece()))) return rc;
-        ring_adjoint_piece_kernel<SPIN><<<dim3(p.nring_piece, nb), kFftThreads, smem_bytes_piece(), s>>>(
-            p.d_ring_piece, p.d_rings, p.lmax, p.M, p.nrings, p.npix, maps, V, p.d_tw, p.d_bh);
-        JHTB_CUDA_TRY(cudaGetLastError());
-    }
+    if ((rc = ensure_smem(chirp_spectrum_kernel<LOGP>, smem))) return rc;
+    chirp_spectrum_kernel<LOGP><<<n, X::TP < 32 ? 32 : X::TP, smem, s>>>(lens, offs, tw, bh);
+    JHTB_CUDA_TRY(cudaGetLastError());
     return JHTB_OK;
 }
 
@@ -1099,21 +851,70 @@ JHTB_DEBUG_ACCESSOR(ringfft)
 
 int launch_ring_synth(const Plan &p, const double2 *F, double *maps, int nb, cudaStream_t s) {
     if (nb <= 0) return JHTB_OK;
-    return p.spin ? launch_ring_synth_t<2>(p, F, maps, nb, s) : launch_ring_synth_t<0>(p, F, maps, nb, s);
-}
-
-int launch_ring_adjoint(const Plan &p, const double *maps, double2 *V, double2 *W, int nb, cudaStream_t s) {
-    if (nb <= 0) return JHTB_OK;
-    return p.spin ? launch_ring_adjoint_t<2>(p, maps, V, W, nb, s) : launch_ring_adjoint_t<0>(p, maps, V, W, nb, s);
-}
-
-int launch_bluestein_setup(const Plan &p, const int *lengths, const long long *offs, int nlen, cudaStream_t s) {
-    if (nlen <= 0) return JHTB_OK;
     int rc;
-    if ((rc = ensure_smem(bluestein_setup_kernel))) return rc;
-    dim3 grid(nlen, 8);
-    bluestein_setup_kernel<<<grid, kFftThreads, smem_bytes(), s>>>(lengths, offs, p.d_tw, p.d_bh);
+    RingArgs a = make_args(p);
+    const size_t fmap = (size_t)p.ncomp * p.nrings * p.M;
+    const long long pmap = (long long)p.ncomp * p.npix;
+    if (p.nunit_long > 0) {
+        if ((rc = ensure_smem(ring_long_kernel<false>, kLongSmem))) return rc;
+        a.units = p.d_ring_units + p.nunit;
+        ring_long_kernel<false><<<dim3(p.nunit_long, nb), 512, kLongSmem, s>>>(a, F, nullptr, nullptr, maps, fmap, pmap);
+        JHTB_CUDA_TRY(cudaGetLastError());
+    }
+    if (p.nunit > 0) {
+        if ((rc = ensure_smem(ring_synth_kernel, kRingSmem))) return rc;
+        a.units = p.d_ring_units;
+        ring_synth_kernel<<<dim3(p.nunit, nb), kRingThreads, kRingSmem, s>>>(a, F, maps, fmap, pmap);
+        JHTB_CUDA_TRY(cudaGetLastError());
+    }
+    return JHTB_OK;
+}
+
+int launch_ring_adjoint(const Plan &p, const double *maps, double2 *V, int nb, cudaStream_t s) {
+    if (nb <= 0) return JHTB_OK;
+    int rc;
+    RingArgs a = make_args(p);
+    const size_t fmap = (size_t)p.ncomp * p.nrings * p.M;
+    const long long pmap = (long long)p.ncomp * p.npix;
+    if (p.nunit_long > 0) {
+        if ((rc = ensure_smem(ring_long_kernel<true>, kLongSmem))) return rc;
+        a.units = p.d_ring_units + p.nunit;
+        ring_long_kernel<true><<<dim3(p.nunit_long, nb), 512, kLongSmem, s>>>(a, nullptr, V, maps, nullptr, fmap, pmap);
+        JHTB_CUDA_TRY(cudaGetLastError());
+    }
+    if (p.nunit > 0) {
+        if ((rc = ensure_smem(ring_adjoint_kernel, kRingSmem))) return rc;
+        a.units = p.d_ring_units;
+        ring_adjoint_kernel<<<dim3(p.nunit, nb), kRingThreads, kRingSmem, s>>>(a, maps, V, fmap, pmap);
+        JHTB_CUDA_TRY(cudaGetLastError());
+    }
+    return JHTB_OK;
+}
+
+int launch_ring_tables(const Plan &p, const int *lens, const long long *ctab_offs, const long long *bh_offs,
+                       const int (&count)[14], cudaStream_t s) {
+    if (p.belt_n > 0) {
+        belt_table_kernel<<<(2 * p.belt_n + 255) / 256, 256, 0, s>>>(p.belt_n, p.d_belt);
+        JHTB_CUDA_TRY(cudaGetLastError());
+    }
+    int n = 0;
+    for (int c : count) n += c;
+    if (n <= 0) return JHTB_OK;
+    ring_table_kernel<<<dim3(n, kRingCols), 128, 0, s>>>(lens, ctab_offs, p.d_ctab);
     JHTB_CUDA_TRY(cudaGetLastError());
+    // the lengths are sorted by their P: count[log2 P] of each
+    int rc, o = 0;
+#define JHTB_SPECTRUM(L)                                                                                   \
+    if ((rc = launch_spectrum<L>(lens + o, bh_offs + o, count[L], p.d_tw, p.d_bh, s))) return rc; \
+    o += count[L];
+    JHTB_SPECTRUM(7)
+    JHTB_SPECTRUM(8)
+    JHTB_SPECTRUM(9)
+    JHTB_SPECTRUM(10)
+    JHTB_SPECTRUM(11)
+    JHTB_SPECTRUM(12)
+    JHTB_SPECTRUM(13)
+#undef JHTB_SPECTRUM
     return JHTB_OK;
 }
 

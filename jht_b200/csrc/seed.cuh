@@ -37,4 +37,20 @@ __device__ __forceinline__ double seed_log2(const SeedParam &sp, int h, double l
     return v;
 }
 
+// Spin-0 ring pairs of the azimuthal stage: north and south coefficients to P = n + i s and
+// M = n - i s, and back.  At m = 0 only the real parts belong to a real field; a ring without
+// a mirror (the equator) keeps its own coefficient.
+__device__ __forceinline__ void spin0_pair(double2 &n, double2 &s, bool m0, bool mirror) {
+    if (m0) n.y = s.y = 0.0;
+    if (!mirror) return;
+    const double2 a = n, b = s;
+    n = make_double2(a.x - b.y, a.y + b.x);
+    s = make_double2(a.x + b.y, a.y - b.x);
+}
+__device__ __forceinline__ void spin0_unpair(double2 &p, double2 &m) {
+    const double2 a = p, b = m;
+    p = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y + b.y));
+    m = make_double2(0.5 * (a.y - b.y), 0.5 * (b.x - a.x));
+}
+
 }  // namespace jhtb

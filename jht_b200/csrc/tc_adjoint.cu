@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // (order, ring chunk), in the exact shared-memory layout the MMA reads
 // ---------------------------------------------------------------------------------
 template <int SPIN>
-__global__ void __launch_bounds__(256) adj_prep_kernel(int lmax, int T, int nrings, int M, const SeedParam *__restrict__ seed,
+__global__ void __launch_bounds__(256) adj_prep_kernel(int lmax, int T, int nrings, int M, int paired, const SeedParam *__restrict__ seed,
                                                        const double2 *__restrict__ F, int nb, int nchunk,
                                                        unsigned char *__restrict__ Bt) {
     __shared__ __align__(16) unsigned char tile[kBStage];
@@ -601,8 +601,9 @@ __global__ void __launch_bounds__(256) adj_prep_kernel(int lmax, int T, int nrin
                 col[3] = ssign * vs.y;
             } else {
                 const double2 *Fb = F + (size_t)b * fmap;
-                const double2 vn = Fb[(size_t)t * M + m];
-                const double2 vs = south ? Fb[(size_t)rs * M + m] : make_double2(0.0, 0.0);
+                double2 vn = Fb[(size_t)t * M + m];
+                double2 vs = south ? Fb[(size_t)rs * M + m] : make_double2(0.0, 0.0);
+                if (paired && south) spin0_unpair(vn, vs);
                 col[0] = vn.x;
                 col[1] = vn.y;
                 col[2] = vs.x;
@@ -700,7 +701,7 @@ int launch_tca_block_states(const Plan &p, cudaStream_t s) {
 }
 
 template <int SPIN>
-static int launch_tca_t(const Plan &p, const double2 *F, double2 *alm, int nb, cudaStream_t s) {
+static int launch_tca_t(const Plan &p, const double2 *F, double2 *alm, int nb, bool paired, cudaStream_t s) {
     auto k = tc_adjoint_kernel<SPIN>;
     const int smem = (int)sizeof(AdjSmem<SPIN>) + 1024;
     int dev = 0, nsm = 148;
@@ -730,7 +731,7 @@ static int launch_tca_t(const Plan &p, const double2 *F, double2 *alm, int nb, c
     for (int b0 = 0; b0 < nb; b0 += kTcaMaps) {
         const int cnt = std::min(kTcaMaps, nb - b0);
         const long long nblk = (long long)p.M * p.tca_nchunk;
-        adj_prep_kernel<SPIN><<<(unsigned)nblk, 256, 0, s>>>(p.lmax, p.T, p.nrings, p.M, p.d_seed, F + b0 * fmap, cnt,
+        adj_prep_kernel<SPIN><<<(unsigned)nblk, 256, 0, s>>>(p.lmax, p.T, p.nrings, p.M, paired, p.d_seed, F + b0 * fmap, cnt,
                                                               p.tca_nchunk, p.d_tca_B);
         JHTB_CUDA_TRY(cudaGetLastError());
         k<<<nsm, kThreads, smem, s>>>(q, alm + b0 * amap, cnt);
@@ -739,9 +740,9 @@ static int launch_tca_t(const Plan &p, const double2 *F, double2 *alm, int nb, c
     return JHTB_OK;
 }
 
-int launch_tc_adjoint(const Plan &p, const double2 *F, double2 *alm, int nb, cudaStream_t s) {
+int launch_tc_adjoint(const Plan &p, const double2 *F, double2 *alm, int nb, bool paired, cudaStream_t s) {
     if (nb <= 0) return JHTB_OK;
-    return p.spin ? launch_tca_t<2>(p, F, alm, nb, s) : launch_tca_t<0>(p, F, alm, nb, s);
+    return p.spin ? launch_tca_t<2>(p, F, alm, nb, paired, s) : launch_tca_t<0>(p, F, alm, nb, paired, s);
 }
 
 }  // namespace jhtb

@@ -37,6 +37,7 @@
 #include <algorithm>
 
 #include "jhtb_internal.cuh"
+#include "seed.cuh"
 #include "tc_common.cuh"
 
 namespace jhtb {
@@ -51,6 +52,7 @@ constexpr int kTcK = 16;         // l steps per chunk = MMA K (BF16)
 
 struct TcParams {
     int lmax, T, nrings, M, nside;
+    int paired;  // spin 0: rows written as P = north + i south, M = north - i south
     long long K;
     const double *x;
     const SeedParam *seed;
@@ -211,8 +213,10 @@ __device__ __forceinline__ void tc_store_F(const TcParams &p, double2 *__restric
         if (t < p.T - 1) Fs[rs * p.M + m] = make_double2(ssign * v[2], ssign * v[3]);
     } else {
         double2 *F = F_all + (size_t)b * p.nrings * p.M;
-        F[(size_t)t * p.M + m] = make_double2(v[0], v[1]);
-        if (t < p.T - 1) F[rs * p.M + m] = make_double2(v[2], v[3]);
+        double2 n = make_double2(v[0], v[1]), s = make_double2(v[2], v[3]);
+        if (p.paired) spin0_pair(n, s, m == 0, t < p.T - 1);
+        F[(size_t)t * p.M + m] = n;
+        if (t < p.T - 1) F[rs * p.M + m] = s;
     }
 }
 
@@ -584,7 +588,7 @@ static int launch_tc_synth_t(const Plan &p, const TcParams &q, const double2 *al
     return JHTB_OK;
 }
 
-int launch_tc_synth(const Plan &p, const double2 *alm, double2 *F, int nb, cudaStream_t s) {
+int launch_tc_synth(const Plan &p, const double2 *alm, double2 *F, int nb, bool paired, cudaStream_t s) {
     if (nb <= 0) return JHTB_OK;
     TcParams q;
     q.lmax = p.lmax;
@@ -592,6 +596,7 @@ int launch_tc_synth(const Plan &p, const double2 *alm, double2 *F, int nb, cudaS
     q.nrings = p.nrings;
     q.M = p.M;
     q.nside = p.nside;
+    q.paired = paired;
     q.K = p.K;
     q.x = p.d_x;
     q.seed = p.d_seed;
