@@ -26,9 +26,9 @@
 // lmax 4096).  At plan creation start_state_kernel runs that part once per warp
 // tile and stores, at the first l where any ring of the tile is representable
 // (rounded down to an even offset from lmin), every ring's (mu_{l-1}, mu_{l-2}, sc).
-// The transforms then start there; rings still scaled run the rescale-check
-// variant until the whole warp is representable, after which the loop is
-// branch-free.
+// The transforms then start there; while a warp still holds scaled rings it runs a variant
+// that counts their values as zero (a select per value, issued beside the FP64 math) and
+// rescales them once per 8 steps; after that the loop is branch-free.
 //
 // Parity.  Step i = l - lmin alternates between accumulator slots A (i even) and
 // B (i odd); N/S outputs are A +- B, realising jht's total / signed sums.
@@ -48,6 +48,12 @@ constexpr int kStage = 32;  // steps staged per warp per round (one per lane)
 #define JHTB_ADJ_SUB 8
 #endif
 constexpr int kSub = JHTB_ADJ_SUB;  // adjoint steps per warp reduction
+// Steps between rescale checks of rings in the underflow range.  A step multiplies a value by
+// less than 2^8 (|alpha| + |gamma| stays below sqrt(2 m + 3) + 4, m < 16384), so a group
+// grows it by less than 2^64 of the 2^623 above the threshold, and what a late check drops is
+// below 2^-336.
+constexpr int kGroup = 8;
+static_assert(kSub <= kGroup, "the adjoint checks once per reduction group");
 // resident CTAs per SM the adjoint kernels are compiled for (their register budget)
 #ifndef JHTB_ADJ0_MINB
 #define JHTB_ADJ0_MINB 4
@@ -239,40 +245,62 @@ struct Stage2 {
     double2 cp[kStage], cm[kStage];
 };
 
-template <int R, bool SLOW>
+template <int R, bool MASK>
 __device__ __forceinline__ void synth0_step(double al, double2 c, const double (&x)[R], double (&u1)[R],
-                                            double (&u2)[R], int (&sc)[R], double (&ar)[R], double (&ai)[R]) {
+                                            double (&u2)[R], const bool (&live)[R], double (&ar)[R], double (&ai)[R]) {
 #pragma unroll
     for (int k = 0; k < R; ++k) {
         double u = fma(al * x[k], u1[k], -u2[k]);
-        double prev = u1[k];
-        if (SLOW) rescale(u, prev, sc[k]);
-        u2[k] = prev;
+        u2[k] = u1[k];
         u1[k] = u;
-        if (SLOW && sc[k] != 0) u = 0.0;
+        if (MASK && !live[k]) u = 0.0;
         ar[k] = fma(c.x, u, ar[k]);
         ai[k] = fma(c.y, u, ai[k]);
     }
+}
+
+// Up to kGroup steps with rings in the underflow range: their values count as zero and are
+// rescaled once, after the group (see kGroup).
+template <int R>
+__device__ __forceinline__ void synth0_group(int q0, int cnt, const Stage0 &sb, const double (&x)[R], double (&u1)[R],
+                                             double (&u2)[R], int (&sc)[R], double (&Ar)[R], double (&Ai)[R],
+                                             double (&Br)[R], double (&Bi)[R]) {
+    bool live[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) live[k] = sc[k] == 0;
+#pragma unroll
+    for (int q = 0; q < kGroup; q += 2) {
+        if (q0 + q < cnt) synth0_step<R, true>(sb.al[q0 + q], sb.c[q0 + q], x, u1, u2, live, Ar, Ai);
+        if (q0 + q + 1 < cnt) synth0_step<R, true>(sb.al[q0 + q + 1], sb.c[q0 + q + 1], x, u1, u2, live, Br, Bi);
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) rescale(u1[k], u2[k], sc[k]);
 }
 
 template <int R, bool SLOW>
 __device__ __forceinline__ void synth0_chunk(int cnt, const Stage0 &sb, const double (&x)[R], double (&u1)[R],
                                              double (&u2)[R], int (&sc)[R], double (&Ar)[R], double (&Ai)[R],
                                              double (&Br)[R], double (&Bi)[R]) {
+    if (SLOW) {
+#pragma unroll 1
+        for (int q0 = 0; q0 < cnt; q0 += kGroup) synth0_group<R>(q0, cnt, sb, x, u1, u2, sc, Ar, Ai, Br, Bi);
+        return;
+    }
+    const bool live[R] = {};
     if (cnt == kStage) {
 #pragma unroll
         for (int q = 0; q < kStage; q += 2) {
-            synth0_step<R, SLOW>(sb.al[q], sb.c[q], x, u1, u2, sc, Ar, Ai);
-            synth0_step<R, SLOW>(sb.al[q + 1], sb.c[q + 1], x, u1, u2, sc, Br, Bi);
+            synth0_step<R, false>(sb.al[q], sb.c[q], x, u1, u2, live, Ar, Ai);
+            synth0_step<R, false>(sb.al[q + 1], sb.c[q + 1], x, u1, u2, live, Br, Bi);
         }
         return;
     }
     int q = 0;
     for (; q + 1 < cnt; q += 2) {
-        synth0_step<R, SLOW>(sb.al[q], sb.c[q], x, u1, u2, sc, Ar, Ai);
-        synth0_step<R, SLOW>(sb.al[q + 1], sb.c[q + 1], x, u1, u2, sc, Br, Bi);
+        synth0_step<R, false>(sb.al[q], sb.c[q], x, u1, u2, live, Ar, Ai);
+        synth0_step<R, false>(sb.al[q + 1], sb.c[q + 1], x, u1, u2, live, Br, Bi);
     }
-    if (q < cnt) synth0_step<R, SLOW>(sb.al[q], sb.c[q], x, u1, u2, sc, Ar, Ai);
+    if (q < cnt) synth0_step<R, false>(sb.al[q], sb.c[q], x, u1, u2, live, Ar, Ai);
 }
 
 template <int R>
@@ -345,29 +373,22 @@ struct Acc2 {
     double ppr, ppi, pmr, pmi, mmr, mmi, mpr, mpi;
 };
 
-template <int R, bool SLOW, int SGN>
+template <int R, bool MASK, int SGN>
 __device__ __forceinline__ void synth2_step(double al, double ga, double2 cp, double2 cm, const double (&x)[R],
-                                            double (&p1)[R], double (&p2)[R], int (&sp)[R], double (&m1)[R],
-                                            double (&m2)[R], int (&sm)[R], Acc2 (&acc)[R]) {
+                                            double (&p1)[R], double (&p2)[R], const bool (&lp)[R], double (&m1)[R],
+                                            double (&m2)[R], const bool (&lm)[R], Acc2 (&acc)[R]) {
 #pragma unroll
     for (int k = 0; k < R; ++k) {
         const double tp = fma(al, x[k], ga);
         const double tm = fma(al, x[k], -ga);
         double up = fma(tp, p1[k], -p2[k]);
         double um = fma(tm, m1[k], -m2[k]);
-        double pp = p1[k], pm = m1[k];
-        if (SLOW) {
-            rescale(up, pp, sp[k]);
-            rescale(um, pm, sm[k]);
-        }
-        p2[k] = pp;
+        p2[k] = p1[k];
         p1[k] = up;
-        m2[k] = pm;
+        m2[k] = m1[k];
         m1[k] = um;
-        if (SLOW) {
-            if (sp[k] != 0) up = 0.0;
-            if (sm[k] != 0) um = 0.0;
-        }
+        if (MASK && !lp[k]) up = 0.0;
+        if (MASK && !lm[k]) um = 0.0;
         Acc2 &a = acc[k];
         a.ppr = fma(cp.x, up, a.ppr);
         a.ppi = fma(cp.y, up, a.ppi);
@@ -380,24 +401,53 @@ __device__ __forceinline__ void synth2_step(double al, double ga, double2 cp, do
     }
 }
 
+template <int R>
+__device__ __forceinline__ void synth2_group(int q0, int cnt, const Stage2 &sb, const double (&x)[R], double (&p1)[R],
+                                             double (&p2)[R], int (&sp)[R], double (&m1)[R], double (&m2)[R],
+                                             int (&sm)[R], Acc2 (&acc)[R]) {
+    bool lp[R], lm[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        lp[k] = sp[k] == 0;
+        lm[k] = sm[k] == 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kGroup; q += 2) {
+        const int a = q0 + q, b = a + 1;
+        if (a < cnt) synth2_step<R, true, 1>(sb.ag[a].x, sb.ag[a].y, sb.cp[a], sb.cm[a], x, p1, p2, lp, m1, m2, lm, acc);
+        if (b < cnt) synth2_step<R, true, -1>(sb.ag[b].x, sb.ag[b].y, sb.cp[b], sb.cm[b], x, p1, p2, lp, m1, m2, lm, acc);
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        rescale(p1[k], p2[k], sp[k]);
+        rescale(m1[k], m2[k], sm[k]);
+    }
+}
+
 template <int R, bool SLOW>
 __device__ __forceinline__ void synth2_chunk(int cnt, const Stage2 &sb, const double (&x)[R], double (&p1)[R],
                                              double (&p2)[R], int (&sp)[R], double (&m1)[R], double (&m2)[R],
                                              int (&sm)[R], Acc2 (&acc)[R]) {
+    if (SLOW) {
+#pragma unroll 1
+        for (int q0 = 0; q0 < cnt; q0 += kGroup) synth2_group<R>(q0, cnt, sb, x, p1, p2, sp, m1, m2, sm, acc);
+        return;
+    }
+    const bool live[R] = {};
     if (cnt == kStage) {  // whole chunk: fully unrolled so the shared-memory loads pipeline
 #pragma unroll
         for (int q = 0; q < kStage; q += 2) {
-            synth2_step<R, SLOW, 1>(sb.ag[q].x, sb.ag[q].y, sb.cp[q], sb.cm[q], x, p1, p2, sp, m1, m2, sm, acc);
-            synth2_step<R, SLOW, -1>(sb.ag[q + 1].x, sb.ag[q + 1].y, sb.cp[q + 1], sb.cm[q + 1], x, p1, p2, sp, m1, m2, sm, acc);
+            synth2_step<R, false, 1>(sb.ag[q].x, sb.ag[q].y, sb.cp[q], sb.cm[q], x, p1, p2, live, m1, m2, live, acc);
+            synth2_step<R, false, -1>(sb.ag[q + 1].x, sb.ag[q + 1].y, sb.cp[q + 1], sb.cm[q + 1], x, p1, p2, live, m1, m2, live, acc);
         }
         return;
     }
     int q = 0;
     for (; q + 1 < cnt; q += 2) {
-        synth2_step<R, SLOW, 1>(sb.ag[q].x, sb.ag[q].y, sb.cp[q], sb.cm[q], x, p1, p2, sp, m1, m2, sm, acc);
-        synth2_step<R, SLOW, -1>(sb.ag[q + 1].x, sb.ag[q + 1].y, sb.cp[q + 1], sb.cm[q + 1], x, p1, p2, sp, m1, m2, sm, acc);
+        synth2_step<R, false, 1>(sb.ag[q].x, sb.ag[q].y, sb.cp[q], sb.cm[q], x, p1, p2, live, m1, m2, live, acc);
+        synth2_step<R, false, -1>(sb.ag[q + 1].x, sb.ag[q + 1].y, sb.cp[q + 1], sb.cm[q + 1], x, p1, p2, live, m1, m2, live, acc);
     }
-    if (q < cnt) synth2_step<R, SLOW, 1>(sb.ag[q].x, sb.ag[q].y, sb.cp[q], sb.cm[q], x, p1, p2, sp, m1, m2, sm, acc);
+    if (q < cnt) synth2_step<R, false, 1>(sb.ag[q].x, sb.ag[q].y, sb.cp[q], sb.cm[q], x, p1, p2, live, m1, m2, live, acc);
 }
 
 template <int R>
@@ -520,18 +570,16 @@ struct AStage {
 };
 
 // ---------------- spin 0 ----------------
-template <int R, bool SLOW>
+template <int R, bool MASK>
 __device__ __forceinline__ double2 adj0_step(double al, const double (&x)[R], double (&u1)[R], double (&u2)[R],
-                                             int (&sc)[R], const double2 (&U)[R]) {
+                                             const bool (&live)[R], const double2 (&U)[R]) {
     double2 part = make_double2(0.0, 0.0);
 #pragma unroll
     for (int k = 0; k < R; ++k) {
         double u = fma(al * x[k], u1[k], -u2[k]);
-        double prev = u1[k];
-        if (SLOW) rescale(u, prev, sc[k]);
-        u2[k] = prev;
+        u2[k] = u1[k];
         u1[k] = u;
-        if (SLOW && sc[k] != 0) u = 0.0;
+        if (MASK && !live[k]) u = 0.0;
         part.x = fma(u, U[k].x, part.x);
         part.y = fma(u, U[k].y, part.y);
     }
@@ -605,23 +653,27 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj0MinBlocks) adj0_kern
                     double2 prev = make_double2(0.0, 0.0);
                     if (acc && wr && JHTB_IN(b0 + i0 + qw, p.K, 204)) prev = part[b0 + i0 + qw];
                     const bool f = __all_sync(kFull, fast);
+                    bool live[R] = {};
                     if (f && q0 + kSub <= cnt) {  // one straight sequence of steps (see adj2_kernel)
 #pragma unroll
                         for (int q = 0; q < kSub; q += 2) {
-                            rb.v[q][lane] = adj0_step<R, false>(sb.ag[q0 + q].x, x, u1, u2, sc, UA);
-                            rb.v[q + 1][lane] = adj0_step<R, false>(sb.ag[q0 + q + 1].x, x, u1, u2, sc, UB);
+                            rb.v[q][lane] = adj0_step<R, false>(sb.ag[q0 + q].x, x, u1, u2, live, UA);
+                            rb.v[q + 1][lane] = adj0_step<R, false>(sb.ag[q0 + q + 1].x, x, u1, u2, live, UB);
                         }
                     } else {
 #pragma unroll
+                        for (int r = 0; r < R; ++r) live[r] = sc[r] == 0;
+#pragma unroll
                         for (int q = 0; q < kSub; q += 2) {
-                            if (q0 + q < cnt) rb.v[q][lane] = adj0_step<R, true>(sb.ag[q0 + q].x, x, u1, u2, sc, UA);
-                            if (q0 + q + 1 < cnt) rb.v[q + 1][lane] = adj0_step<R, true>(sb.ag[q0 + q + 1].x, x, u1, u2, sc, UB);
+                            if (q0 + q < cnt) rb.v[q][lane] = adj0_step<R, true>(sb.ag[q0 + q].x, x, u1, u2, live, UA);
+                            if (q0 + q + 1 < cnt) rb.v[q + 1][lane] = adj0_step<R, true>(sb.ag[q0 + q + 1].x, x, u1, u2, live, UB);
                         }
-                    }
-                    if (!f) {
                         fast = true;
 #pragma unroll
-                        for (int r = 0; r < R; ++r) fast &= sc[r] == 0;
+                        for (int r = 0; r < R; ++r) {
+                            rescale(u1[r], u2[r], sc[r]);
+                            fast &= sc[r] == 0;
+                        }
                     }
                     __syncwarp();
                     const double2 tot = red_sum<kSub>(rb, lane);
@@ -642,10 +694,10 @@ struct In2 {
     double2 vpn, spA, vmn, smA;  // north data and the (-1)^(m+lmin)-signed south data
 };
 
-template <int R, bool SLOW, int SGN>
+template <int R, bool MASK, int SGN>
 __device__ __forceinline__ void adj2_step(double al, double ga, const double (&x)[R], double (&p1)[R],
-                                          double (&p2)[R], int (&sp)[R], double (&m1)[R], double (&m2)[R],
-                                          int (&sm)[R], const In2 (&in)[R], double2 &op, double2 &om) {
+                                          double (&p2)[R], const bool (&lp)[R], double (&m1)[R], double (&m2)[R],
+                                          const bool (&lm)[R], const In2 (&in)[R], double2 &op, double2 &om) {
     op = make_double2(0.0, 0.0);
     om = make_double2(0.0, 0.0);
 #pragma unroll
@@ -654,19 +706,12 @@ __device__ __forceinline__ void adj2_step(double al, double ga, const double (&x
         const double tm = fma(al, x[k], -ga);
         double up = fma(tp, p1[k], -p2[k]);
         double um = fma(tm, m1[k], -m2[k]);
-        double qp = p1[k], qm = m1[k];
-        if (SLOW) {
-            rescale(up, qp, sp[k]);
-            rescale(um, qm, sm[k]);
-        }
-        p2[k] = qp;
+        p2[k] = p1[k];
         p1[k] = up;
-        m2[k] = qm;
+        m2[k] = m1[k];
         m1[k] = um;
-        if (SLOW) {
-            if (sp[k] != 0) up = 0.0;
-            if (sm[k] != 0) um = 0.0;
-        }
+        if (MASK && !lp[k]) up = 0.0;
+        if (MASK && !lm[k]) um = 0.0;
         const In2 &d = in[k];
         // p2 += lp Vpn + (-1)^l lm Sp ;  m2 += lm Vmn + (-1)^l lp Sm   (_recursion.py:565-566)
         op.x = fma(up, d.vpn.x, op.x);
@@ -757,6 +802,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj2MinBlocks) adj2_kern
                     double2 prev = make_double2(0.0, 0.0);
                     if (acc && wr && JHTB_IN(b0 + i0 + qw, p.K, 204)) prev = dstw[b0 + i0 + qw];
                     const bool f = __all_sync(kFull, fast);
+                    bool lp[R] = {}, lm[R] = {};
                     // The variant is chosen once per group, not per step: a whole group of
                     // representable rings runs one straight sequence of steps (choosing per
                     // step made the two variants' register assignments meet after every step).
@@ -764,33 +810,40 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj2MinBlocks) adj2_kern
 #pragma unroll
                         for (int q = 0; q < kSub; q += 2) {
                             double2 op, om;
-                            adj2_step<R, false, 1>(sb.ag[q0 + q].x, sb.ag[q0 + q].y, x, p1, p2, sp, m1, m2, sm, in, op, om);
+                            adj2_step<R, false, 1>(sb.ag[q0 + q].x, sb.ag[q0 + q].y, x, p1, p2, lp, m1, m2, lm, in, op, om);
                             rb.v[q][lane] = op;
                             rb.v[kSub + q][lane] = om;
-                            adj2_step<R, false, -1>(sb.ag[q0 + q + 1].x, sb.ag[q0 + q + 1].y, x, p1, p2, sp, m1, m2, sm, in, op, om);
+                            adj2_step<R, false, -1>(sb.ag[q0 + q + 1].x, sb.ag[q0 + q + 1].y, x, p1, p2, lp, m1, m2, lm, in, op, om);
                             rb.v[q + 1][lane] = op;
                             rb.v[kSub + q + 1][lane] = om;
                         }
                     } else {
 #pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            lp[r] = sp[r] == 0;
+                            lm[r] = sm[r] == 0;
+                        }
+#pragma unroll
                         for (int q = 0; q < kSub; q += 2) {
                             double2 op, om;
                             if (q0 + q < cnt) {
-                                adj2_step<R, true, 1>(sb.ag[q0 + q].x, sb.ag[q0 + q].y, x, p1, p2, sp, m1, m2, sm, in, op, om);
+                                adj2_step<R, true, 1>(sb.ag[q0 + q].x, sb.ag[q0 + q].y, x, p1, p2, lp, m1, m2, lm, in, op, om);
                                 rb.v[q][lane] = op;
                                 rb.v[kSub + q][lane] = om;
                             }
                             if (q0 + q + 1 < cnt) {
-                                adj2_step<R, true, -1>(sb.ag[q0 + q + 1].x, sb.ag[q0 + q + 1].y, x, p1, p2, sp, m1, m2, sm, in, op, om);
+                                adj2_step<R, true, -1>(sb.ag[q0 + q + 1].x, sb.ag[q0 + q + 1].y, x, p1, p2, lp, m1, m2, lm, in, op, om);
                                 rb.v[q + 1][lane] = op;
                                 rb.v[kSub + q + 1][lane] = om;
                             }
                         }
-                    }
-                    if (!f) {
                         fast = true;
 #pragma unroll
-                        for (int r = 0; r < R; ++r) fast &= (sp[r] == 0) && (sm[r] == 0);
+                        for (int r = 0; r < R; ++r) {
+                            rescale(p1[r], p2[r], sp[r]);
+                            rescale(m1[r], m2[r], sm[r]);
+                            fast &= (sp[r] == 0) && (sm[r] == 0);
+                        }
                     }
                     __syncwarp();
                     const double2 tot = red_sum<NV>(rb, lane);
