@@ -149,6 +149,10 @@ struct Plan {
     int *d_adj_order;    // [M * nsuper]
     int *d_adj_tiles;    // [M * nsuper][tps]
     unsigned *d_counter; // work-queue counter
+    // batched FP64 kernels (legendre_batch.cu): (order, 128-ring tile) and (order, ring range)
+    // items by falling cost; ring ranges per order
+    int *d_b_synth_order, *d_b_adj_order;
+    int nb_synth, b_nsuper;
     double2 *d_part;     // [chunk][nsuper][ncomp][K] adjoint partial sums
 
     // tensor-core path (precision BF16X3): 128-ring (spin 2) or 256-ring (spin 0) tiles;
@@ -230,6 +234,14 @@ enum Stage : int { kStageLegSynth = 0, kStageRingSynth = 1, kStageRingAdj = 2, k
 // azimuthal stage transforms; otherwise as the two rings' own coefficients
 int launch_legendre_synth(const Plan &p, const double2 *alm, double2 *F, int nb, bool paired, cudaStream_t s);
 int launch_legendre_adjoint(const Plan &p, const double2 *F, double2 *alm, int nb, bool paired, cudaStream_t s);
+// How a batch is served: `wide` maps in groups of 8 (spin 0) or 4 (spin 2) on the matrix unit,
+// `narrow` maps as one half-width group, `single` ones by the one-map kernels.
+struct BatchSplit {
+    int wide, narrow, single;
+};
+BatchSplit batch_split(const Plan &p, int nb);
+int launch_batch_synth(const Plan &p, const double2 *alm, double2 *F, const BatchSplit &sp, bool paired, cudaStream_t s);
+int launch_batch_adjoint(const Plan &p, const double2 *V, double2 *part, const BatchSplit &sp, bool paired, cudaStream_t s);
 int launch_ring_synth(const Plan &p, const double2 *F, double *maps, int nb, cudaStream_t s);
 int launch_ring_adjoint(const Plan &p, const double *maps, double2 *F, int nb, cudaStream_t s);
 int launch_start_states(const Plan &p, cudaStream_t s);
@@ -293,6 +305,7 @@ __device__ __forceinline__ bool debug_in_range(long long i, long long n, int sit
 #define JHTB_DEBUG_ACCESSOR(name)
 #endif
 int debug_record_legendre(DebugRecord *out, bool reset);
+int debug_record_legendre_batch(DebugRecord *out, bool reset);
 int debug_record_ringfft(DebugRecord *out, bool reset);
 int debug_record_tc_synth(DebugRecord *out, bool reset);
 int debug_record_tc_adjoint(DebugRecord *out, bool reset);

@@ -961,24 +961,49 @@ int launch_start_states_r(const Plan &p, int R, int ntiles, int *lw, double2 *st
     return JHTB_OK;
 }
 
+// Several maps share one recursion on the matrix unit (legendre_batch.cu, with the rule); a
+// left-over single map, and batches below one wave of items, run here.
 int launch_legendre_synth(const Plan &p, const double2 *alm, double2 *F, int nb, bool paired, cudaStream_t s) {
     if (nb <= 0) return JHTB_OK;
+    const BatchSplit sp = batch_split(p, nb);
+    int rc = launch_batch_synth(p, alm, F, sp, paired, s);
+    if (rc || sp.single == 0) return rc;
+    alm += (size_t)(nb - sp.single) * p.ncomp * p.K;
+    F += (size_t)(nb - sp.single) * p.ncomp * p.nrings * p.M;
     JHTB_CUDA_TRY(cudaMemsetAsync(p.d_counter, 0, sizeof(unsigned), s));
     LegParams q = make_params(p);
     q.paired = paired;
     if (p.spin == 0) {
         auto k = synth0_kernel<kR0>;
-        k<<<leg_grid(p, k), kWarpsPerBlock * 32, 0, s>>>(q, alm, F, nb);
+        k<<<leg_grid(p, k), kWarpsPerBlock * 32, 0, s>>>(q, alm, F, sp.single);
     } else {
         auto k = synth2_kernel<kR2>;
-        k<<<leg_grid(p, k), kWarpsPerBlock * 32, 0, s>>>(q, alm, F, nb);
+        k<<<leg_grid(p, k), kWarpsPerBlock * 32, 0, s>>>(q, alm, F, sp.single);
     }
+    JHTB_CUDA_TRY(cudaGetLastError());
+    return JHTB_OK;
+}
+
+static int launch_adj_reduce(const Plan &p, int nsuper, const double2 *part, double2 *alm, int nb, cudaStream_t s) {
+    if (nb <= 0) return JHTB_OK;
+    const long long total = (long long)nb * p.K;
+    const int grid = (int)std::min<long long>((total + 255) / 256, 148LL * 32);
+    if (p.spin == 0) adj_reduce_kernel<0><<<grid, 256, 0, s>>>(p.lmax, p.K, nsuper, p.d_seed, p.d_cnorm, part, alm, nb);
+    else adj_reduce_kernel<2><<<grid, 256, 0, s>>>(p.lmax, p.K, nsuper, p.d_seed, p.d_cnorm, part, alm, nb);
     JHTB_CUDA_TRY(cudaGetLastError());
     return JHTB_OK;
 }
 
 int launch_legendre_adjoint(const Plan &p, const double2 *F, double2 *alm, int nb, bool paired, cudaStream_t s) {
     if (nb <= 0) return JHTB_OK;
+    const BatchSplit sp = batch_split(p, nb);
+    const int nmat = nb - sp.single;
+    int rc = launch_batch_adjoint(p, F, p.d_part, sp, paired, s);
+    if (!rc) rc = launch_adj_reduce(p, p.b_nsuper, p.d_part, alm, nmat, s);
+    if (rc || sp.single == 0) return rc;
+    F += (size_t)nmat * p.ncomp * p.nrings * p.M;
+    alm += (size_t)nmat * p.ncomp * p.K;
+    double2 *part = p.d_part + (size_t)nmat * p.nsuper * p.ncomp * p.K;  // nsuper >= b_nsuper
     JHTB_CUDA_TRY(cudaMemsetAsync(p.d_counter, 0, sizeof(unsigned), s));
     LegParams q = make_params(p);
     q.paired = paired;
@@ -988,18 +1013,13 @@ int launch_legendre_adjoint(const Plan &p, const double2 *F, double2 *alm, int n
     q.stsc = p.d_a_stsc;
     if (p.spin == 0) {
         auto k = adj0_kernel<kRA0>;
-        k<<<leg_grid(p, k), kWarpsPerBlock * 32, 0, s>>>(q, F, p.d_part, nb);
+        k<<<leg_grid(p, k), kWarpsPerBlock * 32, 0, s>>>(q, F, part, sp.single);
     } else {
         auto k = adj2_kernel<kRA2>;
-        k<<<leg_grid(p, k), kWarpsPerBlock * 32, 0, s>>>(q, F, p.d_part, nb);
+        k<<<leg_grid(p, k), kWarpsPerBlock * 32, 0, s>>>(q, F, part, sp.single);
     }
     JHTB_CUDA_TRY(cudaGetLastError());
-    const long long total = (long long)nb * p.K;
-    const int grid = (int)std::min<long long>((total + 255) / 256, 148LL * 32);
-    if (p.spin == 0) adj_reduce_kernel<0><<<grid, 256, 0, s>>>(p.lmax, p.K, p.nsuper, p.d_seed, p.d_cnorm, p.d_part, alm, nb);
-    else adj_reduce_kernel<2><<<grid, 256, 0, s>>>(p.lmax, p.K, p.nsuper, p.d_seed, p.d_cnorm, p.d_part, alm, nb);
-    JHTB_CUDA_TRY(cudaGetLastError());
-    return JHTB_OK;
+    return launch_adj_reduce(p, p.nsuper, part, alm, sp.single, s);
 }
 
 }  // namespace jhtb

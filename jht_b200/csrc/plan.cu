@@ -84,7 +84,8 @@ void free_plan(Plan *p) {
     void *ptrs[] = {p->d_x,     p->d_logsin, p->d_logch, p->d_logsh,   p->d_rings, p->d_tw,
                     p->d_bh,    p->d_seed,   p->d_alpha, p->d_gamma,   p->d_cnorm, p->d_F,
                     p->d_ctab,  p->d_belt,   p->d_scratch, p->d_lw, p->d_st, p->d_stsc, p->d_synth_order,
-                    p->d_adj_order, p->d_adj_tiles, p->d_counter, p->d_part, p->d_err, p->d_ring_units};
+                    p->d_adj_order, p->d_adj_tiles, p->d_counter, p->d_part, p->d_err, p->d_ring_units,
+                    p->d_b_synth_order, p->d_b_adj_order};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (p->a_owns_tables) {
@@ -166,6 +167,33 @@ int build_orders(Plan *p) {
         std::stable_sort(ao.begin(), ao.end(), [&](int a, int b) { return acost[a] > acost[b]; });
         if ((rc = refresh(&p->d_adj_order, ao))) return rc;
         if ((rc = refresh(&p->d_adj_tiles, at))) return rc;
+    }
+    // batched FP64 kernels: (order, 128-ring tile) items, and (order, range of 256-ring blocks)
+    if (p->precision == JHTB_PREC_FP64) {
+        const int tw = 32 * (p->spin ? kRA2 : kRA0), nt = p->a_ntiles;
+        const std::vector<int> &lw = p->h_a_lw;
+        auto cost = [&](long long it) { return std::max(0, L + 1 - lw[it]); };
+        std::vector<int> so;
+        for (long long i = 0; i < (long long)M * nt; ++i) {
+            const int tile = (int)(i % nt);
+            if (tile * tw >= t0 && tile * tw < t1) so.push_back((int)i);
+        }
+        std::stable_sort(so.begin(), so.end(), [&](int a, int b) { return cost(a) > cost(b); });
+        p->nb_synth = (int)so.size();
+        if ((rc = refresh(&p->d_b_synth_order, so))) return rc;
+        const int lo = t0 / kRingGranule, hi = (t1 + kRingGranule - 1) / kRingGranule, per = kRingGranule / tw;
+        const int nblk = (hi - lo + p->b_nsuper - 1) / p->b_nsuper;
+        std::vector<int> ao(M * p->b_nsuper);
+        std::vector<long long> acost(ao.size(), 0);
+        for (int m = 0; m < M; ++m)
+            for (int s = 0; s < p->b_nsuper; ++s) {
+                const int it = m * p->b_nsuper + s;
+                ao[it] = it;
+                for (int t = (lo + s * nblk) * per; t < std::min(std::min(lo + (s + 1) * nblk, hi) * per, nt); ++t)
+                    acost[it] += cost((long long)m * nt + t);
+            }
+        std::stable_sort(ao.begin(), ao.end(), [&](int a, int b) { return acost[a] > acost[b]; });
+        if ((rc = refresh(&p->d_b_adj_order, ao))) return rc;
     }
     // tensor-core kernel: tiles of 128 (spin 2) or 256 (spin 0) rings
     if (p->precision == JHTB_PREC_BF16X3) {
@@ -425,6 +453,7 @@ int build_plan(Plan *p, const jhtb_host_tables *ht) {
         p->a_ntiles = (T + 32 * RA - 1) / (32 * RA);
         p->nsuper = std::min(4, p->a_ntiles);
         p->tps = (p->a_ntiles + p->nsuper - 1) / p->nsuper;
+        p->b_nsuper = std::min(4, (T + kRingGranule - 1) / kRingGranule);
         if (RA == R) {
             p->a_owns_tables = false;
             p->d_a_lw = p->d_lw;
@@ -921,7 +950,7 @@ int jhtb_debug_bounds(int64_t *count, int *site, int64_t *index, int64_t *extent
     *index = *extent = 0;
 #ifdef JHTB_DEBUG
     JHTB_CUDA_TRY(cudaDeviceSynchronize());
-    int (*const readers[])(DebugRecord *, bool) = {debug_record_legendre, debug_record_ringfft, debug_record_tc_synth,
+    int (*const readers[])(DebugRecord *, bool) = {debug_record_legendre, debug_record_legendre_batch, debug_record_ringfft, debug_record_tc_synth,
                                                    debug_record_tc_adjoint, debug_record_vecops};
     for (auto rd : readers) {
         DebugRecord r{};
