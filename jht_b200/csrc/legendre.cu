@@ -53,6 +53,10 @@ constexpr int kSub = JHTB_ADJ_SUB;  // adjoint steps per warp reduction
 // grows it by less than 2^64 of the 2^623 above the threshold, and what a late check drops is
 // below 2^-336.
 constexpr int kGroup = 8;
+// Groups per unrolled iteration of the plain synthesis loops.  Spin 0 (32 instructions a step)
+// fits the instruction cache better rolled (nside 512 / lmax 1024: 169 us against 173 unrolled by
+// four, nside 1024: 1.09 against 1.13 ms); spin 2 gains a little from four (nside 2048: 24.3 against 24.5 ms).
+constexpr int kGroupUnroll0 = 1, kGroupUnroll2 = 4;
 static_assert(kSub <= kGroup, "the adjoint checks once per reduction group");
 // resident CTAs per SM the adjoint kernels are compiled for (their register budget)
 #ifndef JHTB_ADJ0_MINB
@@ -259,52 +263,28 @@ __device__ __forceinline__ void synth0_step(double al, double2 c, const double (
     }
 }
 
-// Up to kGroup steps with rings in the underflow range: their values count as zero and are
-// rescaled once, after the group (see kGroup).
-template <int R>
-__device__ __forceinline__ void synth0_group(int q0, int cnt, const Stage0 &sb, const double (&x)[R], double (&u1)[R],
+// kGroup steps from staged slot q0.  SLOW: with rings in the underflow range, whose values count
+// as zero and which are rescaled once, after the group (see kGroup).
+template <int R, bool SLOW>
+__device__ __forceinline__ void synth0_group(int q0, const Stage0 &sb, const double (&x)[R], double (&u1)[R],
                                              double (&u2)[R], int (&sc)[R], double (&Ar)[R], double (&Ai)[R],
                                              double (&Br)[R], double (&Bi)[R]) {
     bool live[R];
 #pragma unroll
-    for (int k = 0; k < R; ++k) live[k] = sc[k] == 0;
+    for (int k = 0; k < R; ++k) live[k] = !SLOW || sc[k] == 0;
 #pragma unroll
-    for (int q = 0; q < kGroup; q += 2) {
-        if (q0 + q < cnt) synth0_step<R, true>(sb.al[q0 + q], sb.c[q0 + q], x, u1, u2, live, Ar, Ai);
-        if (q0 + q + 1 < cnt) synth0_step<R, true>(sb.al[q0 + q + 1], sb.c[q0 + q + 1], x, u1, u2, live, Br, Bi);
+    for (int q = q0; q < q0 + kGroup; q += 2) {
+        synth0_step<R, SLOW>(sb.al[q], sb.c[q], x, u1, u2, live, Ar, Ai);
+        synth0_step<R, SLOW>(sb.al[q + 1], sb.c[q + 1], x, u1, u2, live, Br, Bi);
     }
-#pragma unroll
-    for (int k = 0; k < R; ++k) rescale(u1[k], u2[k], sc[k]);
-}
-
-template <int R, bool SLOW>
-__device__ __forceinline__ void synth0_chunk(int cnt, const Stage0 &sb, const double (&x)[R], double (&u1)[R],
-                                             double (&u2)[R], int (&sc)[R], double (&Ar)[R], double (&Ai)[R],
-                                             double (&Br)[R], double (&Bi)[R]) {
     if (SLOW) {
-#pragma unroll 1
-        for (int q0 = 0; q0 < cnt; q0 += kGroup) synth0_group<R>(q0, cnt, sb, x, u1, u2, sc, Ar, Ai, Br, Bi);
-        return;
-    }
-    const bool live[R] = {};
-    if (cnt == kStage) {
 #pragma unroll
-        for (int q = 0; q < kStage; q += 2) {
-            synth0_step<R, false>(sb.al[q], sb.c[q], x, u1, u2, live, Ar, Ai);
-            synth0_step<R, false>(sb.al[q + 1], sb.c[q + 1], x, u1, u2, live, Br, Bi);
-        }
-        return;
+        for (int k = 0; k < R; ++k) rescale(u1[k], u2[k], sc[k]);
     }
-    int q = 0;
-    for (; q + 1 < cnt; q += 2) {
-        synth0_step<R, false>(sb.al[q], sb.c[q], x, u1, u2, live, Ar, Ai);
-        synth0_step<R, false>(sb.al[q + 1], sb.c[q + 1], x, u1, u2, live, Br, Bi);
-    }
-    if (q < cnt) synth0_step<R, false>(sb.al[q], sb.c[q], x, u1, u2, live, Ar, Ai);
 }
 
 template <int R>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) synth0_kernel(LegParams p, const double2 *__restrict__ alm_all,
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) synth0_kernel(LegParams p, const double2 *__restrict__ alm_all,
                                                                      double2 *__restrict__ F_all, int nb) {
     __shared__ Stage0 stage[kWarpsPerBlock];
     const int lane = threadIdx.x & 31;
@@ -334,20 +314,33 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) synth0_kernel(LegParams p
             fast &= sc[r] == 0;
             Ar[r] = Ai[r] = Br[r] = Bi[r] = 0.0;
         }
-        for (int i0 = i_start; i0 < nst; i0 += kStage) {
-            const int cnt = min(kStage, nst - i0);
-            if (lane < cnt && JHTB_IN(b0 + i0 + lane, p.K, 201)) {
-                const long long idx = b0 + i0 + lane;
-                const double c = p.cnorm[idx];
-                const double2 a = alm[idx];
-                sb.al[lane] = p.alpha[idx];
-                sb.c[lane] = make_double2(a.x * c, a.y * c);
+        // a round's coefficients, fetched one round ahead; past lmax they are zero, so every
+        // group runs whole (the values of a zero alpha stay bounded and are added with c = 0)
+        double fal, fc;
+        double2 fa;
+        auto fetch = [&](int i0) {
+            const long long idx = b0 + i0 + lane;
+            fal = fc = 0.0;
+            fa = make_double2(0.0, 0.0);
+            if (i0 + lane < nst && JHTB_IN(idx, p.K, 201)) {
+                fal = p.alpha[idx];
+                fc = p.cnorm[idx];
+                fa = alm[idx];
             }
+        };
+        fetch(i_start);
+        for (int i0 = i_start; i0 < nst; i0 += kStage) {
+            sb.al[lane] = fal;
+            sb.c[lane] = make_double2(fa.x * fc, fa.y * fc);
             __syncwarp();
+            if (i0 + kStage < nst) fetch(i0 + kStage);
+            const int cnt = min(kStage, nst - i0);
             if (__all_sync(kFull, fast)) {
-                synth0_chunk<R, false>(cnt, sb, x, u1, u2, sc, Ar, Ai, Br, Bi);
+#pragma unroll kGroupUnroll0
+                for (int q0 = 0; q0 < cnt; q0 += kGroup) synth0_group<R, false>(q0, sb, x, u1, u2, sc, Ar, Ai, Br, Bi);
             } else {
-                synth0_chunk<R, true>(cnt, sb, x, u1, u2, sc, Ar, Ai, Br, Bi);
+#pragma unroll 1
+                for (int q0 = 0; q0 < cnt; q0 += kGroup) synth0_group<R, true>(q0, sb, x, u1, u2, sc, Ar, Ai, Br, Bi);
                 fast = true;
 #pragma unroll
                 for (int r = 0; r < R; ++r) fast &= sc[r] == 0;
@@ -401,57 +394,32 @@ __device__ __forceinline__ void synth2_step(double al, double ga, double2 cp, do
     }
 }
 
-template <int R>
-__device__ __forceinline__ void synth2_group(int q0, int cnt, const Stage2 &sb, const double (&x)[R], double (&p1)[R],
+template <int R, bool SLOW>
+__device__ __forceinline__ void synth2_group(int q0, const Stage2 &sb, const double (&x)[R], double (&p1)[R],
                                              double (&p2)[R], int (&sp)[R], double (&m1)[R], double (&m2)[R],
                                              int (&sm)[R], Acc2 (&acc)[R]) {
     bool lp[R], lm[R];
 #pragma unroll
     for (int k = 0; k < R; ++k) {
-        lp[k] = sp[k] == 0;
-        lm[k] = sm[k] == 0;
+        lp[k] = !SLOW || sp[k] == 0;
+        lm[k] = !SLOW || sm[k] == 0;
     }
 #pragma unroll
-    for (int q = 0; q < kGroup; q += 2) {
-        const int a = q0 + q, b = a + 1;
-        if (a < cnt) synth2_step<R, true, 1>(sb.ag[a].x, sb.ag[a].y, sb.cp[a], sb.cm[a], x, p1, p2, lp, m1, m2, lm, acc);
-        if (b < cnt) synth2_step<R, true, -1>(sb.ag[b].x, sb.ag[b].y, sb.cp[b], sb.cm[b], x, p1, p2, lp, m1, m2, lm, acc);
+    for (int q = q0; q < q0 + kGroup; q += 2) {
+        synth2_step<R, SLOW, 1>(sb.ag[q].x, sb.ag[q].y, sb.cp[q], sb.cm[q], x, p1, p2, lp, m1, m2, lm, acc);
+        synth2_step<R, SLOW, -1>(sb.ag[q + 1].x, sb.ag[q + 1].y, sb.cp[q + 1], sb.cm[q + 1], x, p1, p2, lp, m1, m2, lm, acc);
     }
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-        rescale(p1[k], p2[k], sp[k]);
-        rescale(m1[k], m2[k], sm[k]);
-    }
-}
-
-template <int R, bool SLOW>
-__device__ __forceinline__ void synth2_chunk(int cnt, const Stage2 &sb, const double (&x)[R], double (&p1)[R],
-                                             double (&p2)[R], int (&sp)[R], double (&m1)[R], double (&m2)[R],
-                                             int (&sm)[R], Acc2 (&acc)[R]) {
     if (SLOW) {
-#pragma unroll 1
-        for (int q0 = 0; q0 < cnt; q0 += kGroup) synth2_group<R>(q0, cnt, sb, x, p1, p2, sp, m1, m2, sm, acc);
-        return;
-    }
-    const bool live[R] = {};
-    if (cnt == kStage) {  // whole chunk: fully unrolled so the shared-memory loads pipeline
 #pragma unroll
-        for (int q = 0; q < kStage; q += 2) {
-            synth2_step<R, false, 1>(sb.ag[q].x, sb.ag[q].y, sb.cp[q], sb.cm[q], x, p1, p2, live, m1, m2, live, acc);
-            synth2_step<R, false, -1>(sb.ag[q + 1].x, sb.ag[q + 1].y, sb.cp[q + 1], sb.cm[q + 1], x, p1, p2, live, m1, m2, live, acc);
+        for (int k = 0; k < R; ++k) {
+            rescale(p1[k], p2[k], sp[k]);
+            rescale(m1[k], m2[k], sm[k]);
         }
-        return;
     }
-    int q = 0;
-    for (; q + 1 < cnt; q += 2) {
-        synth2_step<R, false, 1>(sb.ag[q].x, sb.ag[q].y, sb.cp[q], sb.cm[q], x, p1, p2, live, m1, m2, live, acc);
-        synth2_step<R, false, -1>(sb.ag[q + 1].x, sb.ag[q + 1].y, sb.cp[q + 1], sb.cm[q + 1], x, p1, p2, live, m1, m2, live, acc);
-    }
-    if (q < cnt) synth2_step<R, false, 1>(sb.ag[q].x, sb.ag[q].y, sb.cp[q], sb.cm[q], x, p1, p2, live, m1, m2, live, acc);
 }
 
 template <int R>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) synth2_kernel(LegParams p, const double2 *__restrict__ alm_all,
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) synth2_kernel(LegParams p, const double2 *__restrict__ alm_all,
                                                                      double2 *__restrict__ F_all, int nb) {
     __shared__ Stage2 stage[kWarpsPerBlock];
     const int lane = threadIdx.x & 31;
@@ -487,22 +455,34 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) synth2_kernel(LegParams p
             fast &= (sp[r] == 0) && (sm[r] == 0);
             acc[r] = Acc2{0, 0, 0, 0, 0, 0, 0, 0};
         }
-        for (int i0 = i_start; i0 < nst; i0 += kStage) {
-            const int cnt = min(kStage, nst - i0);
-            if (lane < cnt && JHTB_IN(b0 + i0 + lane, p.K, 201)) {
-                const long long idx = b0 + i0 + lane;
-                const double c = p.cnorm[idx];
-                const double2 e = aE[idx], bb = aB[idx];
-                sb.ag[lane] = make_double2(p.alpha[idx], p.gamma[idx]);
-                // cp = -(aE + i aB) c, cm = -(aE - i aB) c   (healpix.py:316-318)
-                sb.cp[lane] = make_double2(-(e.x - bb.y) * c, -(e.y + bb.x) * c);
-                sb.cm[lane] = make_double2(-(e.x + bb.y) * c, -(e.y - bb.x) * c);
+        double2 fe, fb, fag;  // the round's coefficients, one round ahead (see synth0_kernel)
+        double fc;
+        auto fetch = [&](int i0) {
+            const long long idx = b0 + i0 + lane;
+            fc = 0.0;
+            fe = fb = fag = make_double2(0.0, 0.0);
+            if (i0 + lane < nst && JHTB_IN(idx, p.K, 201)) {
+                fc = p.cnorm[idx];
+                fe = aE[idx];
+                fb = aB[idx];
+                fag = make_double2(p.alpha[idx], p.gamma[idx]);
             }
+        };
+        fetch(i_start);
+        for (int i0 = i_start; i0 < nst; i0 += kStage) {
+            sb.ag[lane] = fag;
+            // cp = -(aE + i aB) c, cm = -(aE - i aB) c   (healpix.py:316-318)
+            sb.cp[lane] = make_double2(-(fe.x - fb.y) * fc, -(fe.y + fb.x) * fc);
+            sb.cm[lane] = make_double2(-(fe.x + fb.y) * fc, -(fe.y - fb.x) * fc);
             __syncwarp();
+            if (i0 + kStage < nst) fetch(i0 + kStage);
+            const int cnt = min(kStage, nst - i0);
             if (__all_sync(kFull, fast)) {
-                synth2_chunk<R, false>(cnt, sb, x, p1, p2, sp, m1, m2, sm, acc);
+#pragma unroll kGroupUnroll2
+                for (int q0 = 0; q0 < cnt; q0 += kGroup) synth2_group<R, false>(q0, sb, x, p1, p2, sp, m1, m2, sm, acc);
             } else {
-                synth2_chunk<R, true>(cnt, sb, x, p1, p2, sp, m1, m2, sm, acc);
+#pragma unroll 1
+                for (int q0 = 0; q0 < cnt; q0 += kGroup) synth2_group<R, true>(q0, sb, x, p1, p2, sp, m1, m2, sm, acc);
                 fast = true;
 #pragma unroll
                 for (int r = 0; r < R; ++r) fast &= (sp[r] == 0) && (sm[r] == 0);
@@ -641,10 +621,14 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj0MinBlocks) adj0_kern
                 UB[r] = make_double2(vn.x - vs.x, vn.y - vs.y);
                 fast &= sc[r] == 0;
             }
+            double fal;  // the round's coefficient, one round ahead
+            auto fetch = [&](int i0) { fal = i0 + lane < nst ? p.alpha[b0 + i0 + lane] : 0.0; };
+            fetch(i_start);
             for (int i0 = i_start; i0 < nst; i0 += kStage) {
                 const int cnt = min(kStage, nst - i0);
-                if (lane < cnt) sb.ag[lane].x = p.alpha[b0 + i0 + lane];
+                sb.ag[lane].x = fal;  // zero past lmax: every group runs whole
                 __syncwarp();
+                if (i0 + kStage < nst) fetch(i0 + kStage);
                 for (int q0 = 0; q0 < cnt; q0 += kSub) {
                     // the writer lane's output slot is known up front: issue its load of
                     // the running row sum now so the L2 round trip overlaps the steps
@@ -654,7 +638,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj0MinBlocks) adj0_kern
                     if (acc && wr && JHTB_IN(b0 + i0 + qw, p.K, 204)) prev = part[b0 + i0 + qw];
                     const bool f = __all_sync(kFull, fast);
                     bool live[R] = {};
-                    if (f && q0 + kSub <= cnt) {  // one straight sequence of steps (see adj2_kernel)
+                    if (f) {  // one straight sequence of steps (see adj2_kernel)
 #pragma unroll
                         for (int q = 0; q < kSub; q += 2) {
                             rb.v[q][lane] = adj0_step<R, false>(sb.ag[q0 + q].x, x, u1, u2, live, UA);
@@ -665,8 +649,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj0MinBlocks) adj0_kern
                         for (int r = 0; r < R; ++r) live[r] = sc[r] == 0;
 #pragma unroll
                         for (int q = 0; q < kSub; q += 2) {
-                            if (q0 + q < cnt) rb.v[q][lane] = adj0_step<R, true>(sb.ag[q0 + q].x, x, u1, u2, live, UA);
-                            if (q0 + q + 1 < cnt) rb.v[q + 1][lane] = adj0_step<R, true>(sb.ag[q0 + q + 1].x, x, u1, u2, live, UB);
+                            rb.v[q][lane] = adj0_step<R, true>(sb.ag[q0 + q].x, x, u1, u2, live, UA);
+                            rb.v[q + 1][lane] = adj0_step<R, true>(sb.ag[q0 + q + 1].x, x, u1, u2, live, UB);
                         }
                         fast = true;
 #pragma unroll
@@ -792,7 +776,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj2MinBlocks) adj2_kern
             }
             for (int i0 = i_start; i0 < nst; i0 += kStage) {
                 const int cnt = min(kStage, nst - i0);
-                if (lane < cnt) sb.ag[lane] = make_double2(p.alpha[b0 + i0 + lane], p.gamma[b0 + i0 + lane]);
+                // zero past lmax: every group runs whole
+                sb.ag[lane] = lane < cnt ? make_double2(p.alpha[b0 + i0 + lane], p.gamma[b0 + i0 + lane]) : make_double2(0.0, 0.0);
                 __syncwarp();
                 for (int q0 = 0; q0 < cnt; q0 += kSub) {
                     const int e = lane / LPE;  // entry of this lane's sum: 0..kSub-1 p2, kSub.. m2
@@ -806,7 +791,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj2MinBlocks) adj2_kern
                     // The variant is chosen once per group, not per step: a whole group of
                     // representable rings runs one straight sequence of steps (choosing per
                     // step made the two variants' register assignments meet after every step).
-                    if (f && q0 + kSub <= cnt) {
+                    if (f) {
 #pragma unroll
                         for (int q = 0; q < kSub; q += 2) {
                             double2 op, om;
@@ -826,16 +811,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj2MinBlocks) adj2_kern
 #pragma unroll
                         for (int q = 0; q < kSub; q += 2) {
                             double2 op, om;
-                            if (q0 + q < cnt) {
-                                adj2_step<R, true, 1>(sb.ag[q0 + q].x, sb.ag[q0 + q].y, x, p1, p2, lp, m1, m2, lm, in, op, om);
-                                rb.v[q][lane] = op;
-                                rb.v[kSub + q][lane] = om;
-                            }
-                            if (q0 + q + 1 < cnt) {
-                                adj2_step<R, true, -1>(sb.ag[q0 + q + 1].x, sb.ag[q0 + q + 1].y, x, p1, p2, lp, m1, m2, lm, in, op, om);
-                                rb.v[q + 1][lane] = op;
-                                rb.v[kSub + q + 1][lane] = om;
-                            }
+                            adj2_step<R, true, 1>(sb.ag[q0 + q].x, sb.ag[q0 + q].y, x, p1, p2, lp, m1, m2, lm, in, op, om);
+                            rb.v[q][lane] = op;
+                            rb.v[kSub + q][lane] = om;
+                            adj2_step<R, true, -1>(sb.ag[q0 + q + 1].x, sb.ag[q0 + q + 1].y, x, p1, p2, lp, m1, m2, lm, in, op, om);
+                            rb.v[q + 1][lane] = op;
+                            rb.v[kSub + q + 1][lane] = om;
                         }
                         fast = true;
 #pragma unroll
