@@ -54,6 +54,10 @@ constexpr int kR2 = JHTB_R2;  // spin 2
 #endif
 constexpr int kRA0 = JHTB_RA0;  // adjoint, spin 0
 constexpr int kRA2 = JHTB_RA2;  // adjoint, spin 2
+// Up to this many (order, tile) items the one-map kernels run in smaller units (legendre.cu):
+// the synthesis with one ring per lane, the adjoint with its degrees split over four warps.
+constexpr long long kSmallSynthItems = 2 * 148 * 16;  // two waves of 16 warps per SM
+constexpr long long kSmallAdjItems = 16384;
 #ifndef JHTB_TC_MAPS
 #define JHTB_TC_MAPS 16
 #endif
@@ -146,6 +150,10 @@ struct Plan {
     double2 *d_a_st;
     int *d_a_stsc;
     bool a_owns_tables;
+    // small problems (kSmallAdjItems): the states at the starts of the later degree segments, per
+    // adjoint tile [M * a_ntiles][3][nrec][kRA][32]
+    double2 *d_sg_st;
+    int *d_sg_sc;
     int *d_adj_order;    // [M * nsuper]
     int *d_adj_tiles;    // [M * nsuper][tps]
     unsigned *d_counter; // work-queue counter
@@ -245,6 +253,7 @@ int launch_batch_adjoint(const Plan &p, const double2 *V, double2 *part, const B
 int launch_ring_synth(const Plan &p, const double2 *F, double *maps, int nb, cudaStream_t s);
 int launch_ring_adjoint(const Plan &p, const double *maps, double2 *F, int nb, cudaStream_t s);
 int launch_start_states(const Plan &p, cudaStream_t s);
+int launch_seg_states(const Plan &p, cudaStream_t s);
 int launch_start_states_r(const Plan &p, int R, int ntiles, int *lw, double2 *st, int *stsc, cudaStream_t s);
 int launch_tc_synth(const Plan &p, const double2 *alm, double2 *F, int nb, bool paired, cudaStream_t s);
 int launch_tc_adjoint(const Plan &p, const double2 *F, double2 *alm, int nb, bool paired, cudaStream_t s);

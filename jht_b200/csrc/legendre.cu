@@ -83,6 +83,8 @@ struct LegParams {
     const int *lw;            // [M * ntiles] start l per (m, tile)
     const double2 *st;        // [M * ntiles][nrec][R][32] start (u1, u2)
     const int *stsc;          // [M * ntiles][nrec][R][32] start scale
+    const double2 *sgst;      // [M * ntiles][kSegs - 1][nrec][R][32] states at the later segments' first degrees
+    const int *sgsc;
     const int *synth_order;   // [M * ntiles]
     const int *adj_order;     // [M * nsuper]
     const int *adj_tiles;     // [M * nsuper][tps] tile ids, ascending start l, -1 padded
@@ -126,6 +128,22 @@ __device__ __forceinline__ void rescale(double &u, double &prev, int &sc) {
         prev *= kScaleDown;
         sc += 1;
     }
+}
+
+// Small problems last as long as their longest order takes one warp, not as the
+// work of all of them: nside 128 / lmax 256, spin 2, kept 13% of the warps active and a third of the
+// SMs busy on average.  The synthesis then gives each warp one ring per lane instead of 2 or 4 (the
+// same sums in the same order), and the adjoint splits an item's degrees over the four warps of
+// a CTA: warp seg takes [seg SL, (seg + 1) SL) from lmin, SL a multiple of kGroup, from stored states.
+// Neither needs the item queue (or its counter's memset).  The lines: small_synth, small_adj.
+constexpr int kSegs = kWarpsPerBlock;
+__device__ __forceinline__ int seg_len(int nst) { return ((nst + kSegs - 1) / kSegs + kGroup - 1) & ~(kGroup - 1); }
+// The part [i0, i1) of segment seg that a tile starting at i_start has (i0 == i1: none).
+__device__ __forceinline__ void seg_range(int nst, int seg, int i_start, int &i0, int &i1) {
+    const int sl = seg_len(nst), b = min(nst, seg * sl);
+    i0 = max(b, i_start);
+    i1 = max(i0, min(nst, b + sl));
+    if (b + sl <= i_start || b >= nst) i0 = i1 = b;
 }
 
 __device__ __forceinline__ int next_item(unsigned *counter) {
@@ -222,18 +240,90 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) start_state_kernel(LegPar
         }
 }
 
-// Load the start state of ring slot r for recursion h; invalid rings read (0, 0, 0).
-template <int R>
+// Load the start states of R ring slots from r0 on (tables of RT slots per tile) for recursion h;
+// invalid rings read (0, 0, 0).
+template <int R, int RT = R>
 __device__ __forceinline__ void load_start(const LegParams &p, int item, int h, int nrec, int lane, double (&u1)[R],
-                                           double (&u2)[R], int (&sc)[R]) {
-    const double2 *st = p.st + (size_t)item * nrec * R * 32;
-    const int *stsc = p.stsc + (size_t)item * nrec * R * 32;
+                                           double (&u2)[R], int (&sc)[R], int r0 = 0) {
+    const double2 *st = p.st + (size_t)item * nrec * RT * 32;
+    const int *stsc = p.stsc + (size_t)item * nrec * RT * 32;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        const double2 s = st[(h * R + r) * 32 + lane];
+        const double2 s = st[(h * RT + r0 + r) * 32 + lane];
         u1[r] = s.x;
         u2[r] = s.y;
-        sc[r] = stsc[(h * R + r) * 32 + lane];
+        sc[r] = stsc[(h * RT + r0 + r) * 32 + lane];
+    }
+}
+// The state at degree offset i0 of segment seg: the tile's start state where the segment holds
+// its start, else the stored state of the segment's first degree.
+template <int R>
+__device__ __forceinline__ void load_seg(const LegParams &p, int item, int h, int nrec, int lane, int seg, bool at_start,
+                                         double (&u1)[R], double (&u2)[R], int (&sc)[R]) {
+    if (at_start) {
+        load_start<R>(p, item, h, nrec, lane, u1, u2, sc);
+        return;
+    }
+    const size_t o = ((size_t)item * (kSegs - 1) + seg - 1) * nrec * R * 32;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const double2 s = p.sgst[o + (h * R + r) * 32 + lane];
+        u1[r] = s.x;
+        u2[r] = s.y;
+        sc[r] = p.sgsc[o + (h * R + r) * 32 + lane];
+    }
+}
+
+// Plan creation: run every tile's recursion on from its start and keep the state at each later
+// segment's first degree.
+template <int SPIN, int R>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32) seg_state_kernel(LegParams p, int nitems) {
+    constexpr int NREC = SPIN ? 2 : 1;
+    const int lane = threadIdx.x & 31;
+    const int item = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+    if (item >= nitems) return;
+    const int m = item / p.ntiles, tile = item % p.ntiles;
+    const SeedParam sd = p.seed[m];
+    const long long b0 = alm_index(sd.lmin, m, p.lmax);
+    const int nst = p.lmax - sd.lmin + 1, i_start = p.lw[item] - sd.lmin;
+    if (nst <= 0) return;
+    const int sl = seg_len(nst);
+    double x[R], u1[NREC][R], u2[NREC][R];
+    int sc[NREC][R];
+#pragma unroll
+    for (int h = 0; h < NREC; ++h) load_start<R>(p, item, h, NREC, lane, u1[h], u2[h], sc[h]);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int t = tile * 32 * R + r * 32 + lane;
+        x[r] = t < p.T ? p.x[t] : 0.0;
+    }
+    double2 *st = const_cast<double2 *>(p.sgst) + (size_t)item * (kSegs - 1) * NREC * R * 32;
+    int *stsc = const_cast<int *>(p.sgsc) + (size_t)item * (kSegs - 1) * NREC * R * 32;
+    for (int i = i_start; i < min(nst, (kSegs - 1) * sl + 1); ++i) {
+        if (i > i_start && i % sl == 0) {
+            const int s = i / sl - 1;
+#pragma unroll
+            for (int h = 0; h < NREC; ++h)
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int o = ((s * NREC + h) * R + r) * 32 + lane;
+                    st[o] = make_double2(u1[h][r], u2[h][r]);
+                    stsc[o] = sc[h][r];
+                }
+        }
+        const double al = p.alpha[b0 + i];
+        const double ga = SPIN ? p.gamma[b0 + i] : 0.0;
+#pragma unroll
+        for (int h = 0; h < NREC; ++h)
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const double tt = SPIN ? fma(al, x[r], h ? -ga : ga) : al * x[r];
+                double u = fma(tt, u1[h][r], -u2[h][r]);
+                double prev = u1[h][r];
+                rescale(u, prev, sc[h][r]);
+                u2[h][r] = prev;
+                u1[h][r] = u;
+            }
     }
 }
 
@@ -283,19 +373,21 @@ __device__ __forceinline__ void synth0_group(int q0, const Stage0 &sb, const dou
     }
 }
 
-template <int R>
+template <int R, int RT>  // R rings per lane, RT in the start tables; R < RT: one work unit per warp, no queue
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) synth0_kernel(LegParams p, const double2 *__restrict__ alm_all,
                                                                      double2 *__restrict__ F_all, int nb) {
     __shared__ Stage0 stage[kWarpsPerBlock];
-    const int lane = threadIdx.x & 31;
-    Stage0 &sb = stage[threadIdx.x >> 5];
-    const int nitems = p.nsynth;
+    constexpr bool NARROW = R < RT;
+    constexpr int SUB = RT / R;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Stage0 &sb = stage[warp];
+    const int nitems = p.nsynth * SUB;
     const int L = p.lmax;
     for (;;) {
-        const int it = next_item(p.counter);
+        const int it = NARROW ? (int)blockIdx.x * kWarpsPerBlock + warp : next_item(p.counter);
         if (it >= nitems * nb) break;
         const int b = it / nitems;
-        const int item = p.synth_order[it - b * nitems];
+        const int item = p.synth_order[(it - b * nitems) / SUB], r0 = (it - b * nitems) % SUB * R;
         const int m = item / p.ntiles, tile = item % p.ntiles;
         const double2 *alm = alm_all + (size_t)b * p.K;
         double2 *F = F_all + (size_t)b * p.nrings * p.M;
@@ -305,11 +397,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) synth0_kernel(LegParam
         const int i_start = p.lw[item] - sd.lmin;
         double x[R], u1[R], u2[R], Ar[R], Ai[R], Br[R], Bi[R];
         int sc[R];
-        load_start<R>(p, item, 0, 1, lane, u1, u2, sc);
+        load_start<R, RT>(p, item, 0, 1, lane, u1, u2, sc, r0);
         bool fast = true;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const int t = tile * 32 * R + r * 32 + lane;
+            const int t = tile * 32 * RT + (r0 + r) * 32 + lane;
             x[r] = t < p.T ? p.x[t] : 0.0;
             fast &= sc[r] == 0;
             Ar[r] = Ai[r] = Br[r] = Bi[r] = 0.0;
@@ -350,7 +442,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) synth0_kernel(LegParam
         // F_north = A + B; F_south = (-1)^m (E - O) = A - B   (healpix.py:250-253)
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const int t = tile * 32 * R + r * 32 + lane;
+            const int t = tile * 32 * RT + (r0 + r) * 32 + lane;
             if (t < p.T && JHTB_IN((long long)(p.nrings - 1 - t) * p.M + m, (long long)p.nrings * p.M, 202)) {
                 double2 n = make_double2(Ar[r] + Br[r], Ai[r] + Bi[r]);
                 double2 sth = make_double2(Ar[r] - Br[r], Ai[r] - Bi[r]);
@@ -359,6 +451,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) synth0_kernel(LegParam
                 if (t < p.T - 1) F[(size_t)(p.nrings - 1 - t) * p.M + m] = sth;
             }
         }
+        if (NARROW) return;
     }
 }
 
@@ -418,19 +511,21 @@ __device__ __forceinline__ void synth2_group(int q0, const Stage2 &sb, const dou
     }
 }
 
-template <int R>
+template <int R, int RT>  // R rings per lane, RT in the start tables; R < RT: one work unit per warp, no queue
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) synth2_kernel(LegParams p, const double2 *__restrict__ alm_all,
                                                                      double2 *__restrict__ F_all, int nb) {
     __shared__ Stage2 stage[kWarpsPerBlock];
-    const int lane = threadIdx.x & 31;
-    Stage2 &sb = stage[threadIdx.x >> 5];
-    const int nitems = p.nsynth;
+    constexpr bool NARROW = R < RT;
+    constexpr int SUB = RT / R;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Stage2 &sb = stage[warp];
+    const int nitems = p.nsynth * SUB;
     const int L = p.lmax;
     for (;;) {
-        const int it = next_item(p.counter);
+        const int it = NARROW ? (int)blockIdx.x * kWarpsPerBlock + warp : next_item(p.counter);
         if (it >= nitems * nb) break;
         const int b = it / nitems;
-        const int item = p.synth_order[it - b * nitems];
+        const int item = p.synth_order[(it - b * nitems) / SUB], r0 = (it - b * nitems) % SUB * R;
         const int m = item / p.ntiles, tile = item % p.ntiles;
         const double2 *aE = alm_all + (size_t)b * 2 * p.K;
         const double2 *aB = aE + p.K;
@@ -445,12 +540,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) synth2_kernel(LegParam
         double x[R], p1[R], p2[R], m1[R], m2[R];
         int sp[R], sm[R];
         Acc2 acc[R];
-        load_start<R>(p, item, 0, 2, lane, p1, p2, sp);
-        load_start<R>(p, item, 1, 2, lane, m1, m2, sm);
+        load_start<R, RT>(p, item, 0, 2, lane, p1, p2, sp, r0);
+        load_start<R, RT>(p, item, 1, 2, lane, m1, m2, sm, r0);
         bool fast = true;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const int t = tile * 32 * R + r * 32 + lane;
+            const int t = tile * 32 * RT + (r0 + r) * 32 + lane;
             x[r] = t < p.T ? p.x[t] : 0.0;
             fast &= (sp[r] == 0) && (sm[r] == 0);
             acc[r] = Acc2{0, 0, 0, 0, 0, 0, 0, 0};
@@ -491,7 +586,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) synth2_kernel(LegParam
         }
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const int t = tile * 32 * R + r * 32 + lane;
+            const int t = tile * 32 * RT + (r0 + r) * 32 + lane;
             if (t < p.T && JHTB_IN((long long)(p.nrings - 1 - t) * p.M + m, (long long)p.nrings * p.M, 202)) {
                 const Acc2 &a = acc[r];
                 Fp[(size_t)t * p.M + m] = make_double2(a.ppr, a.ppi);
@@ -503,6 +598,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) synth2_kernel(LegParam
                 }
             }
         }
+        if (NARROW) return;
     }
 }
 
@@ -566,7 +662,7 @@ __device__ __forceinline__ double2 adj0_step(double al, const double (&x)[R], do
     return part;
 }
 
-template <int R>
+template <int R, bool SEG>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj0MinBlocks) adj0_kernel(LegParams p, const double2 *__restrict__ V_all,
                                                                    double2 *__restrict__ part_all, int nb) {
     __shared__ AStage stage[kWarpsPerBlock];
@@ -578,7 +674,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj0MinBlocks) adj0_kern
     const int nsup = p.M * p.nsuper;
     const int L = p.lmax;
     for (;;) {
-        const int it = next_item(p.counter);
+        const int it = SEG ? (int)blockIdx.x : next_item(p.counter);
         if (it >= nsup * nb) break;
         const int b = it / nsup;
         const int sitem = p.adj_order[it - b * nsup];
@@ -588,20 +684,23 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj0MinBlocks) adj0_kern
         const SeedParam sd = p.seed[m];
         const long long b0 = alm_index(sd.lmin, m, L);
         const int nst = L - sd.lmin + 1;
+        int row0 = 0, row1 = nst;  // this warp's part of the row
+        if (SEG) seg_range(nst, threadIdx.x >> 5, 0, row0, row1);
         bool any = false;  // a live tile has already written the row
         for (int j = 0; j < p.tps; ++j) {
             const int tile = p.adj_tiles[(size_t)sitem * p.tps + j];
             if (tile < 0) break;
             const int item = m * p.ntiles + tile;
-            const int i_start = p.lw[item] - sd.lmin;
-            if (i_start >= nst) break;  // ascending order: the rest are dead too
+            const int tile_start = p.lw[item] - sd.lmin;
+            if (tile_start >= row1 || row0 >= row1) break;  // ascending order: the rest are dead too
+            const int i_start = max(row0, tile_start);
             const bool acc = any;       // later tiles add onto the row (their range is inside)
             if (!any)                   // first live tile: zero the prefix no tile reaches
-                for (int i = lane; i < i_start; i += 32) part[b0 + i] = make_double2(0.0, 0.0);
+                for (int i = row0 + lane; i < i_start; i += 32) part[b0 + i] = make_double2(0.0, 0.0);
             double x[R], u1[R], u2[R];
             int sc[R];
             double2 UA[R], UB[R];
-            load_start<R>(p, item, 0, 1, lane, u1, u2, sc);
+            load_seg<R>(p, item, 0, 1, lane, threadIdx.x >> 5, !SEG || i_start == tile_start, u1, u2, sc);
             bool fast = true;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
@@ -622,13 +721,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj0MinBlocks) adj0_kern
                 fast &= sc[r] == 0;
             }
             double fal;  // the round's coefficient, one round ahead
-            auto fetch = [&](int i0) { fal = i0 + lane < nst ? p.alpha[b0 + i0 + lane] : 0.0; };
+            auto fetch = [&](int i0) { fal = i0 + lane < row1 ? p.alpha[b0 + i0 + lane] : 0.0; };
             fetch(i_start);
-            for (int i0 = i_start; i0 < nst; i0 += kStage) {
-                const int cnt = min(kStage, nst - i0);
+            for (int i0 = i_start; i0 < row1; i0 += kStage) {
+                const int cnt = min(kStage, row1 - i0);
                 sb.ag[lane].x = fal;  // zero past lmax: every group runs whole
                 __syncwarp();
-                if (i0 + kStage < nst) fetch(i0 + kStage);
+                if (i0 + kStage < row1) fetch(i0 + kStage);
                 for (int q0 = 0; q0 < cnt; q0 += kSub) {
                     // the writer lane's output slot is known up front: issue its load of
                     // the running row sum now so the L2 round trip overlaps the steps
@@ -669,7 +768,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj0MinBlocks) adj0_kern
             any = true;
         }
         if (!any)  // no live tile: the whole row is zero
-            for (int i = lane; i < nst; i += 32) part[b0 + i] = make_double2(0.0, 0.0);
+            for (int i = row0 + lane; i < row1; i += 32) part[b0 + i] = make_double2(0.0, 0.0);
+        if (SEG) return;
     }
 }
 
@@ -709,7 +809,7 @@ __device__ __forceinline__ void adj2_step(double al, double ga, const double (&x
     }
 }
 
-template <int R>
+template <int R, bool SEG>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj2MinBlocks) adj2_kernel(LegParams p, const double2 *__restrict__ V_all,
                                                                    double2 *__restrict__ part_all, int nb) {
     constexpr int NV = 2 * kSub;
@@ -722,7 +822,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj2MinBlocks) adj2_kern
     const int nsup = p.M * p.nsuper;
     const int L = p.lmax;
     for (;;) {
-        const int it = next_item(p.counter);
+        const int it = SEG ? (int)blockIdx.x : next_item(p.counter);
         if (it >= nsup * nb) break;
         const int b = it / nsup;
         const int sitem = p.adj_order[it - b * nsup];
@@ -735,24 +835,27 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj2MinBlocks) adj2_kern
         const long long b0 = alm_index(sd.lmin, m, L);
         const int nst = L - sd.lmin + 1;
         const double ssign = ((m + sd.lmin) & 1) ? -1.0 : 1.0;
+        int row0 = 0, row1 = nst;
+        if (SEG) seg_range(nst, threadIdx.x >> 5, 0, row0, row1);
         bool any = false;
         for (int j = 0; j < p.tps; ++j) {
             const int tile = p.adj_tiles[(size_t)sitem * p.tps + j];
             if (tile < 0) break;
             const int item = m * p.ntiles + tile;
-            const int i_start = p.lw[item] - sd.lmin;
-            if (i_start >= nst) break;
+            const int tile_start = p.lw[item] - sd.lmin;
+            if (tile_start >= row1 || row0 >= row1) break;
+            const int i_start = max(row0, tile_start);
             const bool acc = any;
             if (!any)
-                for (int i = lane; i < i_start; i += 32) {
+                for (int i = row0 + lane; i < i_start; i += 32) {
                     partP[b0 + i] = make_double2(0.0, 0.0);
                     partM[b0 + i] = make_double2(0.0, 0.0);
                 }
             double x[R], p1[R], p2[R], m1[R], m2[R];
             int sp[R], sm[R];
             In2 in[R];
-            load_start<R>(p, item, 0, 2, lane, p1, p2, sp);
-            load_start<R>(p, item, 1, 2, lane, m1, m2, sm);
+            load_seg<R>(p, item, 0, 2, lane, threadIdx.x >> 5, !SEG || i_start == tile_start, p1, p2, sp);
+            load_seg<R>(p, item, 1, 2, lane, threadIdx.x >> 5, !SEG || i_start == tile_start, m1, m2, sm);
             bool fast = true;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
@@ -774,8 +877,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj2MinBlocks) adj2_kern
                 in[r] = d;
                 fast &= (sp[r] == 0) && (sm[r] == 0);
             }
-            for (int i0 = i_start; i0 < nst; i0 += kStage) {
-                const int cnt = min(kStage, nst - i0);
+            for (int i0 = i_start; i0 < row1; i0 += kStage) {
+                const int cnt = min(kStage, row1 - i0);
                 // zero past lmax: every group runs whole
                 sb.ag[lane] = lane < cnt ? make_double2(p.alpha[b0 + i0 + lane], p.gamma[b0 + i0 + lane]) : make_double2(0.0, 0.0);
                 __syncwarp();
@@ -836,10 +939,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kAdj2MinBlocks) adj2_kern
             any = true;
         }
         if (!any)
-            for (int i = lane; i < nst; i += 32) {
+            for (int i = row0 + lane; i < row1; i += 32) {
                 partP[b0 + i] = make_double2(0.0, 0.0);
                 partM[b0 + i] = make_double2(0.0, 0.0);
             }
+        if (SEG) return;
     }
 }
 
@@ -942,6 +1046,31 @@ int launch_start_states_r(const Plan &p, int R, int ntiles, int *lw, double2 *st
     return JHTB_OK;
 }
 
+int launch_seg_states(const Plan &p, cudaStream_t s) {
+    if (!p.d_sg_st) return JHTB_OK;
+    LegParams q = make_params(p);
+    q.ntiles = p.a_ntiles;
+    q.lw = p.d_a_lw;
+    q.st = p.d_a_st;
+    q.stsc = p.d_a_stsc;
+    q.sgst = p.d_sg_st;
+    q.sgsc = p.d_sg_sc;
+    const int n = p.M * p.a_ntiles, w = kWarpsPerBlock;
+    if (p.spin == 0) seg_state_kernel<0, kRA0><<<(n + w - 1) / w, w * 32, 0, s>>>(q, n);
+    else seg_state_kernel<2, kRA2><<<(n + w - 1) / w, w * 32, 0, s>>>(q, n);
+    JHTB_CUDA_TRY(cudaGetLastError());
+    return JHTB_OK;
+}
+
+// The lines between the plain and the small-problem forms, by items of one launch.  One map,
+// Legendre stage in a graph, plain -> small, us: synthesis nside 128 / lmax 256 spin 2 41 -> 16
+// (1028 items), nside 256 / lmax 512 spin 0 53 -> 30 (2052), spin 2 86 -> 73 (4104), but nside 400 /
+// lmax 800 spin 0 103 -> 113 (5607).  Adjoint nside 128 spin 2 78 -> 22 (514), nside 300 / lmax 641
+// spin 2 356 -> 179 (3210), nside 512 / lmax 1024 spin 0 288 -> 256 and spin 2 657 -> 615 (8200), but
+// nside 1024 / lmax 2048 spin 2 4073 -> 4179 (32784).
+static bool small_synth(const Plan &p, int nb) { return (long long)nb * p.M * p.ntiles <= kSmallSynthItems; }
+static bool small_adj(const Plan &p, int nb) { return p.d_sg_st && (long long)nb * p.M * p.a_ntiles <= kSmallAdjItems; }
+
 // Several maps share one recursion on the matrix unit (legendre_batch.cu, with the rule); a
 // left-over single map, and batches below one wave of items, run here.
 int launch_legendre_synth(const Plan &p, const double2 *alm, double2 *F, int nb, bool paired, cudaStream_t s) {
@@ -951,14 +1080,22 @@ int launch_legendre_synth(const Plan &p, const double2 *alm, double2 *F, int nb,
     if (rc || sp.single == 0) return rc;
     alm += (size_t)(nb - sp.single) * p.ncomp * p.K;
     F += (size_t)(nb - sp.single) * p.ncomp * p.nrings * p.M;
-    JHTB_CUDA_TRY(cudaMemsetAsync(p.d_counter, 0, sizeof(unsigned), s));
     LegParams q = make_params(p);
     q.paired = paired;
+    if (small_synth(p, sp.single)) {
+        const long long units = (long long)p.nsynth * (p.spin ? kR2 : kR0) * sp.single;
+        const unsigned grid = (unsigned)((units + kWarpsPerBlock - 1) / kWarpsPerBlock);
+        if (p.spin == 0) synth0_kernel<1, kR0><<<grid, kWarpsPerBlock * 32, 0, s>>>(q, alm, F, sp.single);
+        else synth2_kernel<1, kR2><<<grid, kWarpsPerBlock * 32, 0, s>>>(q, alm, F, sp.single);
+        JHTB_CUDA_TRY(cudaGetLastError());
+        return JHTB_OK;
+    }
+    JHTB_CUDA_TRY(cudaMemsetAsync(p.d_counter, 0, sizeof(unsigned), s));
     if (p.spin == 0) {
-        auto k = synth0_kernel<kR0>;
+        auto k = synth0_kernel<kR0, kR0>;
         k<<<leg_grid(p, k), kWarpsPerBlock * 32, 0, s>>>(q, alm, F, sp.single);
     } else {
-        auto k = synth2_kernel<kR2>;
+        auto k = synth2_kernel<kR2, kR2>;
         k<<<leg_grid(p, k), kWarpsPerBlock * 32, 0, s>>>(q, alm, F, sp.single);
     }
     JHTB_CUDA_TRY(cudaGetLastError());
@@ -985,18 +1122,27 @@ int launch_legendre_adjoint(const Plan &p, const double2 *F, double2 *alm, int n
     F += (size_t)nmat * p.ncomp * p.nrings * p.M;
     alm += (size_t)nmat * p.ncomp * p.K;
     double2 *part = p.d_part + (size_t)nmat * p.nsuper * p.ncomp * p.K;  // nsuper >= b_nsuper
-    JHTB_CUDA_TRY(cudaMemsetAsync(p.d_counter, 0, sizeof(unsigned), s));
     LegParams q = make_params(p);
     q.paired = paired;
     q.ntiles = p.a_ntiles;
     q.lw = p.d_a_lw;
     q.st = p.d_a_st;
     q.stsc = p.d_a_stsc;
+    if (small_adj(p, sp.single)) {
+        q.sgst = p.d_sg_st;
+        q.sgsc = p.d_sg_sc;
+        const int grid = p.M * p.nsuper * sp.single;
+        if (p.spin == 0) adj0_kernel<kRA0, true><<<grid, kWarpsPerBlock * 32, 0, s>>>(q, F, part, sp.single);
+        else adj2_kernel<kRA2, true><<<grid, kWarpsPerBlock * 32, 0, s>>>(q, F, part, sp.single);
+        JHTB_CUDA_TRY(cudaGetLastError());
+        return launch_adj_reduce(p, p.nsuper, part, alm, sp.single, s);
+    }
+    JHTB_CUDA_TRY(cudaMemsetAsync(p.d_counter, 0, sizeof(unsigned), s));
     if (p.spin == 0) {
-        auto k = adj0_kernel<kRA0>;
+        auto k = adj0_kernel<kRA0, false>;
         k<<<leg_grid(p, k), kWarpsPerBlock * 32, 0, s>>>(q, F, part, sp.single);
     } else {
-        auto k = adj2_kernel<kRA2>;
+        auto k = adj2_kernel<kRA2, false>;
         k<<<leg_grid(p, k), kWarpsPerBlock * 32, 0, s>>>(q, F, part, sp.single);
     }
     JHTB_CUDA_TRY(cudaGetLastError());

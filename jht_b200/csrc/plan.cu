@@ -85,7 +85,7 @@ void free_plan(Plan *p) {
                     p->d_bh,    p->d_seed,   p->d_alpha, p->d_gamma,   p->d_cnorm, p->d_F,
                     p->d_ctab,  p->d_belt,   p->d_scratch, p->d_lw, p->d_st, p->d_stsc, p->d_synth_order,
                     p->d_adj_order, p->d_adj_tiles, p->d_counter, p->d_part, p->d_err, p->d_ring_units,
-                    p->d_b_synth_order, p->d_b_adj_order};
+                    p->d_b_synth_order, p->d_b_adj_order, p->d_sg_st, p->d_sg_sc};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (p->a_owns_tables) {
@@ -473,6 +473,16 @@ int build_plan(Plan *p, const jhtb_host_tables *ht) {
             p->h_a_lw.resize(nitems);
             JHTB_CUDA_TRY(cudaMemcpy(p->h_a_lw.data(), p->d_a_lw, sizeof(int) * nitems, cudaMemcpyDeviceToHost));
         }
+    }
+
+    // ---- degree segments of small problems (adjoint) -----------------------------------------
+    if (p->precision == JHTB_PREC_FP64 && (long long)M * p->a_ntiles <= kSmallAdjItems) {
+        const size_t nel = (size_t)M * p->a_ntiles * 3 * (spin ? 2 : 1) * (spin ? kRA2 : kRA0) * 32;
+        JHTB_CUDA_TRY(cudaMalloc((void **)&p->d_sg_st, sizeof(double2) * nel));
+        JHTB_CUDA_TRY(cudaMalloc((void **)&p->d_sg_sc, sizeof(int) * nel));
+        bytes += (sizeof(double2) + sizeof(int)) * nel;
+        if ((rc = launch_seg_states(*p, 0))) return rc;
+        JHTB_CUDA_TRY(cudaDeviceSynchronize());
     }
 
     // ---- tensor-core path: 128-ring tiles ---------------------------------------------------
