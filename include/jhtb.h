@@ -190,6 +190,16 @@ int jhtb_nufft_spread_tiles(const void *vals, const double *theta, const double 
                             const int64_t *seg_tile, int tiles_m, int nk, int nm, int W, double beta,
                             void *grid, void *stream);
 
+/* ---- coefficient layouts (masked.py:117-175, healpix.py:58-74) ----
+ * One launch each for what jht writes as gathers and concatenations.  alm: device
+ * complex128 [batch][ncomp][K]; x: device float64 [batch][ncomp * (n0 + 2 np)], per channel
+ * the a_l0 (l >= spin), then sqrt2 Re and sqrt2 Im of the m > 0 modes in packed order. */
+int jhtb_real_to_alm(int lmax, int spin, int batch, const double *x, void *alm, void *stream);
+int jhtb_alm_to_real(int lmax, int spin, int batch, const void *alm, double *x, void *stream);
+/* In place: S^T g -> the gradient of <g, S a> in the complex a (dL/dRe + i dL/dIm): twice the
+ * value at m > 0; at m = 0 the value (spin 0) or (Re E + i Re B, Re B - i Re E) (spin 2). */
+int jhtb_synthesis_cotangent(int lmax, int spin, int batch, void *alm, void *stream);
+
 /* ---- sharding over devices (no counterpart in jht, which runs on one device) ----
  * A plan can be restricted to the ring pairs of half-grid rings [t0, t1) (the
  * northern rings t0..t1-1, the equator included when t1 = 2 nside, and their

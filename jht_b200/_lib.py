@@ -57,6 +57,9 @@ EXPORTS = (
     "jhtb_nufft_spread_tiles",
     "jhtb_debug_bounds",
     "jhtb_fft_c2c",
+    "jhtb_real_to_alm",
+    "jhtb_alm_to_real",
+    "jhtb_synthesis_cotangent",
 )
 
 
@@ -125,6 +128,9 @@ def load_library(path: str | os.PathLike | None = None):
                                               vp, vp]),
             "jhtb_debug_bounds": (i32, [ctypes.POINTER(i64), ctypes.POINTER(i32), ctypes.POINTER(i64),
                                         ctypes.POINTER(i64)]),
+            "jhtb_real_to_alm": (i32, [i32, i32, i32, dp, vp, vp]),
+            "jhtb_alm_to_real": (i32, [i32, i32, i32, vp, dp, vp]),
+            "jhtb_synthesis_cotangent": (i32, [i32, i32, i32, vp, vp]),
             "jhtb_fft_c2c": (i32, [vp, vp, i32, i64, i64, i64, i64, i64, i64, i64, i64, i32, ctypes.c_double, i64,
                                    vp, vp]),
         }

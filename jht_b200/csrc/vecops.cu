@@ -7,6 +7,8 @@
 // All are HBM-bound streaming kernels: grid-stride loops, 8-byte coalesced accesses.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "jhtb_internal.cuh"
 
 namespace jhtb {
@@ -130,6 +132,119 @@ int jhtb_dot(const jhtb_plan *plan, int64_t n, const double *x, const double *y,
     if (nb < 1) nb = 1;
     dot_partial_kernel<<<nb, kVecThreads, 0, s>>>(n, x, y, p.d_scratch);
     dot_final_kernel<<<1, kVecThreads, 0, s>>>(nb, p.d_scratch, result);
+    JHTB_CUDA_TRY(cudaGetLastError());
+    return JHTB_OK;
+}
+
+}  // extern "C"
+
+// ---------------------------------------------------------------------------------------
+// coefficient layouts: one launch where the callers would otherwise chain about eight gather,
+// scatter, scale and concatenate kernels per conversion (at nside 256 / lmax 512, four maps, those
+// took as long as the Legendre stage).  HBM-bound; the m > 0 modes follow the lmax + 1 ones of
+// m = 0 in the packed order, and for spin 2 the first of them, (1, 1), is not a degree of freedom.
+// ---------------------------------------------------------------------------------------
+namespace jhtb {
+namespace {
+constexpr double kSqrt2 = 1.41421356237309504880;
+struct DofLayout {
+    int n0;           // a_l0 with l >= spin
+    long long np;     // modes with m > 0
+    long long off;    // packed index of the first of them
+};
+DofLayout dof_layout(int lmax, int spin, long long K) {
+    DofLayout d;
+    d.n0 = lmax + 1 > spin ? lmax + 1 - spin : 0;
+    d.off = std::min<long long>(K, lmax + 1 + (spin ? 1 : 0));
+    d.np = K - d.off;
+    return d;
+}
+__global__ void real_to_alm_kernel(long long K, int lmax, int spin, DofLayout d, const double *__restrict__ x,
+                                   double2 *__restrict__ alm, long long total) {
+    const long long nx = d.n0 + 2 * d.np;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+        const long long c = i / K, k = i - c * K;
+        const double *v = x + c * nx;
+        double2 a = make_double2(0.0, 0.0);
+        if (k <= lmax) {
+            if (k >= spin) a.x = v[k - spin];
+        } else if (k >= d.off) {
+            a = make_double2(v[d.n0 + k - d.off] / kSqrt2, v[d.n0 + d.np + k - d.off] / kSqrt2);
+        }
+        alm[i] = a;
+    }
+}
+__global__ void alm_to_real_kernel(long long K, int lmax, int spin, DofLayout d, const double2 *__restrict__ alm,
+                                   double *__restrict__ x, long long total) {
+    const long long nx = d.n0 + 2 * d.np;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+        const long long c = i / K, k = i - c * K;
+        const double2 a = alm[i];
+        double *v = x + c * nx;
+        if (k <= lmax) {
+            if (k >= spin) v[k - spin] = a.x;
+        } else if (k >= d.off) {
+            v[d.n0 + k - d.off] = kSqrt2 * a.x;
+            v[d.n0 + d.np + k - d.off] = kSqrt2 * a.y;
+        }
+    }
+}
+template <int SPIN>
+__global__ void synthesis_cotangent_kernel(long long K, int lmax, double2 *__restrict__ alm, long long total) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+        const long long b = i / K, k = i - b * K;
+        double2 *p = alm + b * (SPIN ? 2 : 1) * K + k;
+        const double2 e = p[0];
+        if (SPIN) {
+            const double2 g = p[K];
+            p[0] = k <= lmax ? make_double2(e.x, g.x) : make_double2(2.0 * e.x, 2.0 * e.y);
+            p[K] = k <= lmax ? make_double2(g.x, -e.x) : make_double2(2.0 * g.x, 2.0 * g.y);
+        } else if (k > lmax) {
+            p[0] = make_double2(2.0 * e.x, 2.0 * e.y);
+        }
+    }
+}
+
+int check_layout(const char *who, int lmax, int spin, int batch, const void *a, const void *b) {
+    const std::string w(who);
+    if (spin != 0 && spin != 2) return fail(JHTB_ERR_UNSUPPORTED, w + ": spin must be 0 or 2");
+    if (lmax < 0 || lmax > 16383) return fail(JHTB_ERR_INVALID, w + ": lmax must be in [0, 16383]");
+    if (batch < 0) return fail(JHTB_ERR_INVALID, w + ": negative batch");
+    if (!a || !b) return fail(JHTB_ERR_INVALID, w + ": NULL argument");
+    return JHTB_OK;
+}
+}  // namespace
+}  // namespace jhtb
+
+extern "C" {
+
+int jhtb_real_to_alm(int lmax, int spin, int batch, const double *x, void *alm, void *stream) {
+    const int rc = check_layout("jhtb_real_to_alm", lmax, spin, batch, x, alm);
+    if (rc || batch == 0) return rc;
+    const long long K = (long long)(lmax + 1) * (lmax + 2) / 2, total = K * batch * (spin ? 2 : 1);
+    real_to_alm_kernel<<<grid_for(total), kVecThreads, 0, (cudaStream_t)stream>>>(K, lmax, spin, dof_layout(lmax, spin, K), x,
+                                                                                  (double2 *)alm, total);
+    JHTB_CUDA_TRY(cudaGetLastError());
+    return JHTB_OK;
+}
+
+int jhtb_alm_to_real(int lmax, int spin, int batch, const void *alm, double *x, void *stream) {
+    const int rc = check_layout("jhtb_alm_to_real", lmax, spin, batch, alm, x);
+    if (rc || batch == 0) return rc;
+    const long long K = (long long)(lmax + 1) * (lmax + 2) / 2, total = K * batch * (spin ? 2 : 1);
+    alm_to_real_kernel<<<grid_for(total), kVecThreads, 0, (cudaStream_t)stream>>>(K, lmax, spin, dof_layout(lmax, spin, K),
+                                                                                  (const double2 *)alm, x, total);
+    JHTB_CUDA_TRY(cudaGetLastError());
+    return JHTB_OK;
+}
+
+int jhtb_synthesis_cotangent(int lmax, int spin, int batch, void *alm, void *stream) {
+    const int rc = check_layout("jhtb_synthesis_cotangent", lmax, spin, batch, alm, alm);
+    if (rc || batch == 0) return rc;
+    const long long K = (long long)(lmax + 1) * (lmax + 2) / 2, total = K * batch;
+    cudaStream_t s = (cudaStream_t)stream;
+    if (spin) synthesis_cotangent_kernel<2><<<grid_for(total), kVecThreads, 0, s>>>(K, lmax, (double2 *)alm, total);
+    else synthesis_cotangent_kernel<0><<<grid_for(total), kVecThreads, 0, s>>>(K, lmax, (double2 *)alm, total);
     JHTB_CUDA_TRY(cudaGetLastError());
     return JHTB_OK;
 }

@@ -218,7 +218,12 @@ class _Synthesis(torch.autograd.Function):
     def backward(ctx, g):
         nside, lmax, spin, precision = ctx.geom
         b = _Adjoint.apply(g.contiguous(), nside, lmax, spin, precision)
-        return _synthesis_cotangent(b, lmax, spin), None, None, None, None
+        if torch.is_grad_enabled():  # create_graph: every operation stays differentiable
+            return _synthesis_cotangent(b, lmax, spin), None, None, None, None
+        if b.numel():  # the same values written over the fresh S^T g in one launch
+            _lib.check(_lib.load_library().jhtb_synthesis_cotangent(lmax, spin, b.shape[0], b.data_ptr(), _lib.stream_ptr()),
+                       "jhtb_synthesis_cotangent")
+        return b, None, None, None, None
 
 
 class _Adjoint(torch.autograd.Function):

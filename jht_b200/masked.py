@@ -15,6 +15,7 @@ from functools import lru_cache
 
 import numpy as np
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib
 from ._analysis import _pix_w_device, analysis
@@ -94,8 +95,22 @@ def pseudo_alm(maps, mask, nside: int, lmax: int, spin: int = 0, niter: int = 3,
     return analysis((msk if spin == 0 else msk[None, :]) * m, nside, lmax, spin, niter, use_weights)
 
 
+def _one_launch(t: torch.Tensor, dtype: torch.dtype, shape: tuple) -> bool:
+    """Whether the library's layout kernels apply: a plain, non-empty tensor of this dtype and shape
+    (behind the batch axis) on the current device, with no gradient or tangent to record."""
+    return (t.is_cuda and t.numel() > 0 and t.dtype == dtype and tuple(t.shape[1:]) == shape and t.device.index == torch.cuda.current_device()
+            and not (torch.is_grad_enabled() and t.requires_grad) and forward_ad._current_level < 0)
+
+
 def _real_batch(a: torch.Tensor, lmax: int, spin: int) -> torch.Tensor:
     """(B, ncomp, K) complex -> (B, n_dof) real."""
+    if _one_launch(a, torch.complex128, (1 if spin == 0 else 2, alm_size(lmax))):
+        a = a.contiguous()
+        x = torch.empty((a.shape[0], n_dof(lmax, spin)), dtype=torch.float64, device=a.device)
+        if x.numel():
+            _lib.check(_lib.load_library().jhtb_alm_to_real(lmax, spin, a.shape[0], a.data_ptr(), x.data_ptr(),
+                                                            _lib.stream_ptr()), "jhtb_alm_to_real")
+        return x
     k0, kp = _dof_index(lmax, spin, _dev_index(a))
     parts = []
     for c in range(a.shape[1]):
@@ -106,6 +121,13 @@ def _real_batch(a: torch.Tensor, lmax: int, spin: int) -> torch.Tensor:
 
 def _alm_batch(x: torch.Tensor, lmax: int, spin: int) -> torch.Tensor:
     """(B, n_dof) real -> (B, ncomp, K) complex."""
+    if _one_launch(x, torch.float64, (n_dof(lmax, spin),)):
+        x = x.contiguous()
+        a = torch.empty((x.shape[0], 1 if spin == 0 else 2, alm_size(lmax)), dtype=torch.complex128, device=x.device)
+        if a.numel():
+            _lib.check(_lib.load_library().jhtb_real_to_alm(lmax, spin, x.shape[0], x.data_ptr(), a.data_ptr(),
+                                                            _lib.stream_ptr()), "jhtb_real_to_alm")
+        return a
     k0, kp = _dof_index(lmax, spin, _dev_index(x))
     n0, npos = k0.numel(), kp.numel()
     ncomp = 1 if spin == 0 else 2
