@@ -135,72 +135,123 @@ __global__ void __launch_bounds__(kNuThreads) spread_kernel(const double2 *__res
 }
 
 // Tiled spread: the points arrive grouped by kTile x kTile-cell tiles of the grid (segments
-// of one tile, at most kSegPoints points each).  A CTA adds its segment's windows into a
-// shared-memory copy of the tile plus its W-cell halo, then adds that block to the grid once
-// per cell, so the global atomics fall from 2 W^2 per point to 2 (kTile + W)^2 per segment.
-// A point whose window leaves the block (a coordinate outside the tile its key named) is
-// added straight to the grid.
+// of one tile, at most kSegPoints points each).  A CTA sums its segment's windows over the tile and
+// its W-cell halo on chip and adds that block to the grid once per cell, so the global atomics
+// fall from 2 W^2 per point to 2 (kTile + W)^2 per segment.
+//
+// The sum over a segment's points is a matrix product, G[k][m] = sum_j wk_j[k] (v_j wm_j[m]), with
+// each point's two windows as zero-padded rows of the 48 x 48-cell block (cells as re, im column
+// pairs), so it runs on the FP64 matrix unit: 9 of the block's 6 x 12 products of 8 x 8 per warp,
+// four points per step, accumulators in registers.  That is ten times the additions of the windows
+// alone, but needs no atomics; adding the windows into shared memory took 392 shared FP64 atomics per
+// point (compare-and-swap loops).  A point whose window leaves the block (a coordinate outside the tile its
+// key named) is added straight to the grid.
 constexpr int kTile = 32;
-constexpr int kSpreadThreads = 128;
+constexpr int kSpreadThreads = 256;
+constexpr int kSpreadPts = 32;                    // points staged per round
+constexpr int kBlkCells = 48;                     // block edge, >= kTile + 16
+constexpr int kSA = kBlkCells + 4, kSB = 2 * kBlkCells + 4;  // strides = 4 mod 16: conflict-free fragment loads
+
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
+
+// Weight a of the window of one coordinate (the value window() gives at index a).
+template <int W>
+__device__ __forceinline__ double window_at(double u, double f, int a, double beta) {
+    const double t = u - (f + a);
+    const double z = t * (2.0 / W);
+    const double z2 = z * z;
+    return z2 < 1.0 ? exp(beta * (sqrt(1.0 - z2) - 1.0)) : 0.0;
+}
 
 template <int W>
-__global__ void __launch_bounds__(kSpreadThreads) spread_tiles_kernel(
+__global__ void __launch_bounds__(kSpreadThreads, 3) spread_tiles_kernel(
     const double2 *__restrict__ vals, const double *__restrict__ theta, const double *__restrict__ phi,
     long long npts, const long long *__restrict__ seg_start, const int *__restrict__ seg_count,
     const long long *__restrict__ seg_tile, int tiles_m, int nk, int nm, double beta, double2 *__restrict__ grid) {
     constexpr int B = kTile + W;  // block edge: the tile and its halo
-    __shared__ double acc[B * B * 2];
-    for (int i = threadIdx.x; i < B * B * 2; i += blockDim.x) acc[i] = 0.0;
-    __syncthreads();
+    static_assert(B <= kBlkCells, "block of 6 x 12 products");
+    __shared__ __align__(16) double sa[kSpreadPts][kSA];  // wk of each point, row = grid row of the block
+    __shared__ __align__(16) double sb[kSpreadPts][kSB];  // v wm, column pair = grid column of the block
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int lr = lane >> 2, lk = lane & 3;
+    const int rb0 = (warp & 1) * 3, cb0 = (warp >> 1) * 3;  // this warp's 3 x 3 products
     const long long seg = blockIdx.x;
     const long long tile = seg_tile[seg];
     const long long k_org = (tile / tiles_m) * kTile - W / 2, m_org = (tile % tiles_m) * kTile - W / 2;
     const long long p0 = seg_start[seg];
     const int cnt = seg_count[seg];
-    for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
-        const long long j = p0 + q;
-        if (j < 0 || j >= npts) continue;
-        long long k0, m0;
-        double wk[W], wm[W], unused[W];
-        window<W, false>(theta[j], nk, beta, k0, wk, unused);
-        window<W, false>(phi[j], nm, beta, m0, wm, unused);
-        const double2 v = vals[j];
-        const long long lk = k0 - k_org, lm = m0 - m_org;
-        if (lk >= 0 && lk + W <= B && lm >= 0 && lm + W <= B) {
-#pragma unroll 1
-            for (int a = 0; a < W; ++a) {
-                double *row = acc + 2 * ((lk + a) * B + lm);
-                const double vx = wk[a] * v.x, vy = wk[a] * v.y;
+    double acc[3][3][2];
 #pragma unroll
-                for (int b = 0; b < W; ++b) {
-                    atomicAdd(row + 2 * b, wm[b] * vx);
-                    atomicAdd(row + 2 * b + 1, wm[b] * vy);
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[r][c][0] = acc[r][c][1] = 0.0;
+    const int pt = threadIdx.x >> 3, sub = threadIdx.x & 7;  // eight threads stage a point
+    for (int q0 = 0; q0 < cnt; q0 += kSpreadPts) {
+        __syncthreads();  // the round before is read
+        for (int i = threadIdx.x; i < kSpreadPts * (kSA + kSB) / 2; i += kSpreadThreads) {
+            double2 *z = i < kSpreadPts * kSA / 2 ? reinterpret_cast<double2 *>(&sa[0][0]) + i
+                                                  : reinterpret_cast<double2 *>(&sb[0][0]) + (i - kSpreadPts * kSA / 2);
+            *z = make_double2(0.0, 0.0);
+        }
+        __syncthreads();
+        const long long j = p0 + q0 + pt;
+        if (q0 + pt < cnt && j >= 0 && j < npts) {
+            const double uk = theta[j] * (double)nk / kTwoPi, um = phi[j] * (double)nm / kTwoPi;
+            const double fk = ceil(uk - 0.5 * W), fm = ceil(um - 0.5 * W);
+            const long long k0 = (fk > -4.0e18 && fk < 4.0e18) ? (long long)fk : 0;
+            const long long m0 = (fm > -4.0e18 && fm < 4.0e18) ? (long long)fm : 0;
+            const double2 v = vals[j];
+            const long long bk = k0 - k_org, bm = m0 - m_org;
+            // an infinite value would reach the block's other cells as 0 x inf
+            if (bk >= 0 && bk + W <= B && bm >= 0 && bm + W <= B && isfinite(v.x) && isfinite(v.y)) {
+                for (int a = sub; a < W; a += 8) {
+                    sa[pt][bk + a] = window_at<W>(uk, fk, a, beta);
+                    const double wm = window_at<W>(um, fm, a, beta);
+                    *reinterpret_cast<double2 *>(&sb[pt][2 * (bm + a)]) = make_double2(wm * v.x, wm * v.y);
                 }
-            }
-        } else {
-            int mi[W];
-#pragma unroll
-            for (int b = 0; b < W; ++b) mi[b] = wrap(m0 + b, nm);
-#pragma unroll 1
-            for (int a = 0; a < W; ++a) {
-                double *row = reinterpret_cast<double *>(grid + (size_t)wrap(k0 + a, nk) * nm);
-                const double vx = wk[a] * v.x, vy = wk[a] * v.y;
-#pragma unroll
-                for (int b = 0; b < W; ++b) {
-                    atomicAdd(row + 2 * mi[b], wm[b] * vx);
-                    atomicAdd(row + 2 * mi[b] + 1, wm[b] * vy);
+            } else {
+                for (int a = sub; a < W; a += 8) {
+                    double *row = reinterpret_cast<double *>(grid + (size_t)wrap(k0 + a, nk) * nm);
+                    const double wk = window_at<W>(uk, fk, a, beta);
+                    for (int b = 0; b < W; ++b) {
+                        const double wm = window_at<W>(um, fm, b, beta);
+                        const int mi = wrap(m0 + b, nm);
+                        atomicAdd(row + 2 * mi, wm * (wk * v.x));
+                        atomicAdd(row + 2 * mi + 1, wm * (wk * v.y));
+                    }
                 }
             }
         }
+        __syncthreads();
+#pragma unroll 2
+        for (int ks = 0; ks < kSpreadPts / 4; ++ks) {
+            double af[3], bf[3];
+#pragma unroll
+            for (int r = 0; r < 3; ++r) af[r] = sa[4 * ks + lk][8 * (rb0 + r) + lr];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) bf[c] = sb[4 * ks + lk][8 * (cb0 + c) + lr];
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) dmma(acc[r][c], af[r], bf[c]);
+        }
     }
-    __syncthreads();
-    for (int c = threadIdx.x; c < B * B; c += blockDim.x) {
-        const double x = acc[2 * c], y = acc[2 * c + 1];
-        if (x == 0.0 && y == 0.0) continue;
-        const int a = c / B, b = c - a * B;
-        double *cell = reinterpret_cast<double *>(grid + (size_t)wrap(k_org + a, nk) * nm + wrap(m_org + b, nm));
-        atomicAdd(cell, x);
-        atomicAdd(cell + 1, y);
+    // this lane holds row 8 (rb0 + r) + lr, cell 4 (cb0 + c) + lk
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const int a = 8 * (rb0 + r) + lr;
+        if (a >= B) continue;
+        double *row = reinterpret_cast<double *>(grid + (size_t)wrap(k_org + a, nk) * nm);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int b = 4 * (cb0 + c) + lk;
+            if (b >= B || (acc[r][c][0] == 0.0 && acc[r][c][1] == 0.0)) continue;
+            double *cell = row + 2 * wrap(m_org + b, nm);
+            atomicAdd(cell, acc[r][c][0]);
+            atomicAdd(cell + 1, acc[r][c][1]);
+        }
     }
 }
 
