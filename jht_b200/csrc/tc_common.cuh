@@ -190,10 +190,7 @@ __device__ __forceinline__ uint32_t cvt_bf16x2(float hi, float lo) {
 // consecutive pair is split with paired conversions: h = bf16(x), m = bf16(x - h),
 // l = x - h - m (exact: at most 8 significant bits remain), packed pk[part][pair] with the
 // even value in the low half.
-__device__ __forceinline__ void split3_pack8(const double (&v)[8], uint32_t (&pk)[3][4]) {
-    float f[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = (float)v[i];
+__device__ __forceinline__ void split3_packf8(const float *f, uint32_t (&pk)[3][4]) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const float x0 = f[2 * q], x1 = f[2 * q + 1];
@@ -205,6 +202,12 @@ __device__ __forceinline__ void split3_pack8(const double (&v)[8], uint32_t (&pk
         pk[1][q] = m;
         pk[2][q] = __byte_perm(__float_as_uint(r20), __float_as_uint(r21), 0x7632);
     }
+}
+__device__ __forceinline__ void split3_pack8(const double (&v)[8], uint32_t (&pk)[3][4]) {
+    float f[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = (float)v[i];
+    split3_packf8(f, pk);
 }
 
 

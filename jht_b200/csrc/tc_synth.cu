@@ -16,12 +16,14 @@
 // working at one time read the same orders' chunks from L2.
 //
 // The CTA is warp-specialised and its roles meet only at mbarriers:
-//   producer warps (one thread per A row = tensor-memory lane and recursion chain) run
-//     the FP64 recursion (same normalised form and start states as the FP64 kernels),
-//     round mu to FP32, split it into three BF16 parts and store their rows of the A
-//     operands straight into tensor memory (tcgen05.st), so the six split products never
-//     re-read A through shared memory; every 256 degrees they fold the FP32 block sums
-//     into FP64 accumulators in shared memory and at the item's end write the spectra;
+//   recursion warps (one thread per A row = tensor-memory lane and recursion chain) run
+//     the FP64 recursion (same normalised form and start states as the FP64 kernels) and
+//     hand mu, rounded to FP32, on through shared memory;
+//   split warps (the same rows) split it into three BF16 parts and store their rows of the A
+//     operands into tensor memory (tcgen05.st), so the six split products never re-read A
+//     through shared memory;
+//   fold warps (the same rows) fold the FP32 block sums into FP64 accumulators in shared
+//     memory every 256 degrees and at the item's end write the spectra;
 //   one loader warp: a bulk copy per chunk of the prepared tiles and coefficients;
 //   one MMA warp issues the six split products hh, hm, mh, hl, lh, mm per GEMM
 //     (kind::f16, A from tensor memory, B from shared memory, FP32 accumulators in
@@ -31,6 +33,13 @@
 // products (relative size <= 2^-8) accumulate over the whole item.  Every wait is
 // bounded; on timeout the kernel records an error, every role leaves its loop, and
 // tensor memory is released after the last MMA has drained.
+//
+// Bound by latencies between the roles: per 16-degree chunk of a 128-ring tile the products take
+// 384 cycles and the CTA about 2500, of which a recursion warp waits 640 and computes the rest (the
+// chunk's dependent FMAs, conversions and stores alone take 520 with eight warps), and a barrier
+// test costs 130 to 200 cycles even when it passes.  With one set of eight warps doing all three of
+// recursion, split and fold (two warps per scheduler) a chunk took 2800; nside 1024 / lmax 2048, spin
+// 2, 16 maps: 18.6 -> 16.4 ms, nside 512 / lmax 1024, spin 0, 64 maps: 5.77 -> 4.99 ms.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -76,15 +85,18 @@ struct TcCfg {
     static constexpr int NBT = SPIN ? 2 : 1;        // B tiles per chunk (spin 0: both GEMMs share one)
     static constexpr int N = 4 * BM;                // columns per GEMM
     static constexpr int CH = BM >= 16 ? 1 : 2;     // recursion chains (GEMMs) per producer thread
-    static constexpr int NPW = 4 * NG / CH;         // producer warps: one thread per A row (TMEM lane) and chain
-    static constexpr int LOAD_WARP = NPW;
-    static constexpr int MMA_WARP = NPW + 1;
-    static constexpr int NTHREADS = (NPW + 2) * 32;
+    static constexpr int NPW = 4 * NG / CH;         // recursion warps, as many split warps and as many fold
+                                                    // warps: one thread per A row (TMEM lane) and chain
+    static constexpr int LOAD_WARP = 3 * NPW;
+    static constexpr int MMA_WARP = 3 * NPW + 1;
+    static constexpr int NTHREADS = (3 * NPW + 2) * 32;
+    static constexpr int NSX = 2;                   // stages of the FP32 values between them
     static constexpr int NSA = JHTB_TC_NSA;         // A stages (in tensor memory)
-    static constexpr int NSB = 6;                   // B stages (with the chunk's coefficients): deep enough to cover the bulk copies' latency
+    static constexpr int NSB = SPIN && BM >= 16 ? 5 : 6;  // B stages (with the chunk's coefficients): deep enough to cover
+                                                          // the bulk copies' latency
     static constexpr int BTILE = N * kTcK * 2;
     static constexpr int BBYTES = NBT * 3 * BTILE + kTcK * 16;  // tiles, then 16 (alpha, gamma) pairs
-    static constexpr int BSTRIDE = (BBYTES + 1023) / 1024 * 1024;
+    static constexpr int BSTRIDE = (BBYTES + 127) / 128 * 128;
     static constexpr int ACOLS = kTcK / 2;          // tensor-memory columns of one A row (16 BF16)
     // tensor memory: hh block sums [buffer][GEMM], correction sums [GEMM], then the A stages
     static constexpr int COL_CORR = 2 * NG * N;
@@ -101,6 +113,8 @@ struct TcSmem {
     using C = TcCfg<SPIN, BM>;
     alignas(1024) unsigned char B[C::NSB][C::BSTRIDE];
     double acc[C::NG][C::N][kTcRows];  // FP64 sums [GEMM][column][row]: a warp touches 32 consecutive words
+    float4 x[C::NSX][C::NPW][C::CH * 4][32];  // a chunk's values per recursion warp: 4 degrees per lane and slot
+    alignas(8) uint64_t fullX[C::NSX][C::NPW], emptyX[C::NSX][C::NPW];
     alignas(8) uint64_t fullA[C::NSA], emptyA[C::NSA], fullB[C::NSB], emptyB[C::NSB];
     uint64_t accFull[2], accEmpty[2], corrEmpty, fin;
     uint32_t taddr;
@@ -127,6 +141,12 @@ __device__ __forceinline__ TcItem tc_item_of(const TcParams &p, int item) {
     return q;
 }
 
+// GEMM j's ring of an item tile (spin 0: two 128-ring halves).
+template <int SPIN>
+__device__ __forceinline__ int tc_ring(int tile, int j, int row) {
+    return SPIN ? tile * kTcRows + row : tile * 2 * kTcRows + j * kTcRows + row;
+}
+
 // Whether any role has recorded a failure; one verdict per warp (see mbar_wait_warp).
 __device__ __forceinline__ bool tc_failed(const int *f) {
     return __any_sync(0xffffffffu, *(volatile const int *)f != 0);
@@ -148,23 +168,19 @@ __device__ __forceinline__ double tc_step(double t, double &u1, double &u2, int 
     return (SLOW && sc != 0) ? 0.0 : u;
 }
 
-// 16 steps of this thread's CH recursion chains (GEMMs j0 .. j0 + CH - 1), split into
-// BF16 parts and stored as its row (= its tensor-memory lane) of those GEMMs' three A
-// operands: tA[c] is the lane-offset tensor-memory address of chain c's split-0 operand,
-// the splits following at ACOLS columns apart.  Spin 2: GEMM 0 is the +2 recursion
-// (+gamma), GEMM 1 the -2 one (-gamma), same ring; spin 0: the GEMMs are rings row and
-// 128 + row of the item tile (gamma = 0).  Past the end of the column the
-// coefficients are zero, which keeps the state bounded (u_k = -u_{k-2}) while the B
+// 16 steps of this thread's CH recursion chains (GEMMs j0 .. j0 + CH - 1), rounded to FP32.
+// Spin 2: GEMM 0 is the +2 recursion (+gamma), GEMM 1 the -2 one (-gamma), same ring; spin 0:
+// the GEMMs are rings row and 128 + row of the item tile (gamma = 0).  Past the end of the
+// column the coefficients are zero, which keeps the state bounded (u_k = -u_{k-2}) while the B
 // rows there are zero; rows past the last ring start from a zero state and stay zero.
 // In the item's first chunk (FIRST) the `skip` steps before the start state are zero and
 // leave the state untouched.  Each half-chunk first loads its eight coefficient pairs
 // and forms the multipliers t = alpha x +- gamma, so only one FMA per step stays on the
 // dependency chain.
 template <bool SLOW, bool FIRST, int CH>
-__device__ __forceinline__ void tc_chunk(const double2 *coef, const double (&x)[CH], double (&u1)[CH],
-                                         double (&u2)[CH], int (&sc)[CH], const uint32_t (&tA)[CH], int skip,
-                                         unsigned long long gflip) {
-    constexpr uint32_t AC = kTcK / 2;
+__device__ __forceinline__ void tc_values(const double2 *coef, const double (&x)[CH], double (&u1)[CH],
+                                          double (&u2)[CH], int (&sc)[CH], int skip, unsigned long long gflip,
+                                          float4 (*out)[32], int lane) {
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         double t[CH][8];
@@ -179,21 +195,18 @@ __device__ __forceinline__ void tc_chunk(const double2 *coef, const double (&x)[
                 t[c][k] = fma(a.x, x[c], g);
             }
         }
-        uint32_t pk[CH][3][4];
-        double v[CH][8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const bool dead = FIRST && half * 8 + q < skip;
 #pragma unroll
-            for (int c = 0; c < CH; ++c) v[c][q] = dead ? 0.0 : tc_step<SLOW>(t[c][q], u1[c], u2[c], sc[c]);
+            for (int c = 0; c < CH; ++c) t[c][q] = dead ? 0.0 : tc_step<SLOW>(t[c][q], u1[c], u2[c], sc[c]);
         }
-#pragma unroll
-        for (int c = 0; c < CH; ++c) split3_pack8(v[c], pk[c]);
 #pragma unroll
         for (int c = 0; c < CH; ++c)
 #pragma unroll
-            for (int sp = 0; sp < 3; ++sp)
-                tmem_st4(tA[c] + sp * AC + half * 4, pk[c][sp][0], pk[c][sp][1], pk[c][sp][2], pk[c][sp][3]);
+            for (int k = 0; k < 2; ++k)
+                out[c * 4 + half * 2 + k][lane] = make_float4((float)t[c][4 * k], (float)t[c][4 * k + 1], (float)t[c][4 * k + 2],
+                                                              (float)t[c][4 * k + 3]);
     }
 }
 
@@ -233,15 +246,13 @@ __device__ __forceinline__ void fold32(double *accj, uint32_t ta, int col, int r
 }
 
 // ---------------------------------------------------------------------------------
-// producer warps: recursion -> A tiles; block folds and the item's output
+// recursion warps: FP64 recursion -> the chunk's FP32 values in shared memory
 // ---------------------------------------------------------------------------------
 template <int SPIN, int BM>
-__device__ void tc_producer(const TcParams &p, TcSmem<SPIN, BM> &sm, double2 *__restrict__ F_all, int nb,
-                            uint32_t tbase, int warp, int lane) {
+__device__ void tc_recursion(const TcParams &p, TcSmem<SPIN, BM> &sm, int warp, int lane) {
     using C = TcCfg<SPIN, BM>;
-    constexpr int N = C::N;
     constexpr int CH = C::CH;
-    const int row = (warp & 3) * 32 + lane;  // A row = TMEM lane (warp w reaches lanes 32 (w % 4) ..)
+    const int row = (warp & 3) * 32 + lane;  // A row
     const int j0 = (warp >> 2) * CH;         // this thread's first GEMM
     // sign bits of gamma for the thread's chains: chain c (GEMM j0 + c) is the -gamma
     // recursion when j0 + c is odd; bit 63 - c of gflip (spin 0 has gamma = 0)
@@ -249,109 +260,154 @@ __device__ void tc_producer(const TcParams &p, TcSmem<SPIN, BM> &sm, double2 *__
 #pragma unroll
     for (int c = 0; c < CH; ++c)
         if ((j0 + c) & 1) gflip |= 1ull << (63 - c);
-    const uint32_t tl = tbase + ((uint32_t)((warp & 3) * 32) << 16);
-    const int nitems = p.norder;
-    unsigned gc = 0, bk = 0;
+    unsigned gc = 0;
     bool ok = true;
-    // GEMM j's ring (spin 0: two 128-ring halves of the item tile) and start-state slot
-    auto ring_of = [&](int tile, int j) { return SPIN ? tile * kTcRows + row : tile * 2 * kTcRows + j * kTcRows + row; };
-    auto st_of = [&](int id, int j) { return ((size_t)id * 2 + j) * kTcRows + row; };
-    for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
+    for (int it = blockIdx.x; it < p.norder && ok; it += gridDim.x) {
         if (tc_failed(&sm.fail)) break;
         const int id = __ldg(&p.order[it]);
         const TcItem q = tc_item_of(p, id);
-        int tr[CH];
         double x[CH], u1[CH], u2[CH];
         int sc[CH];
         bool fast = true;
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
-            tr[c] = ring_of(q.tile, j0 + c);
-            const double2 st = p.st[st_of(id, j0 + c)];
-            x[c] = tr[c] < p.T ? __ldg(&p.x[tr[c]]) : 0.0;
+            const int t = tc_ring<SPIN>(q.tile, j0 + c, row);
+            const size_t slot = ((size_t)id * 2 + j0 + c) * kTcRows + row;
+            const double2 st = p.st[slot];
+            x[c] = t < p.T ? __ldg(&p.x[t]) : 0.0;
             u1[c] = st.x;
             u2[c] = st.y;
-            sc[c] = tr[c] < p.T ? p.stsc[st_of(id, j0 + c)] : 0;
+            sc[c] = t < p.T ? p.stsc[slot] : 0;
             fast &= sc[c] == 0;
         }
         for (int c = 0; c < q.nck; ++c, ++gc) {
-            const int sA = gc % C::NSA, sB = gc % C::NSB;
+            const int sB = gc % C::NSB, sX = gc % C::NSX;
             if (!mbar_wait_warp(&sm.fullB[sB], (gc / C::NSB) & 1u, p.wait_ns)) { ok = false; break; }
-            if (gc >= (unsigned)C::NSA && !mbar_wait_warp(&sm.emptyA[sA], ((gc / C::NSA) - 1u) & 1u, p.wait_ns)) { ok = false; break; }
-            tc_fence_after();  // the stage's previous MMAs are complete before it is overwritten
-            uint32_t tA[CH];
-#pragma unroll
-            for (int e = 0; e < CH; ++e) tA[e] = tl + (uint32_t)(C::COL_A + (sA * C::NG + j0 + e) * 3 * C::ACOLS);
             const double2 *coef = reinterpret_cast<const double2 *>(sm.B[sB] + C::NBT * 3 * C::BTILE);
+            if (gc >= (unsigned)C::NSX && !mbar_wait_warp(&sm.emptyX[sX][warp], ((gc / C::NSX) - 1u) & 1u, p.wait_ns)) { ok = false; break; }
             const bool f = __all_sync(0xffffffffu, fast);
+            float4 (*out)[32] = sm.x[sX][warp];
             if (c == 0)  // the first chunk: steps before the start state are dead
-                tc_chunk<true, true, CH>(coef, x, u1, u2, sc, tA, q.skip, gflip);
+                tc_values<true, true, CH>(coef, x, u1, u2, sc, q.skip, gflip, out, lane);
             else if (f)
-                tc_chunk<false, false, CH>(coef, x, u1, u2, sc, tA, 0, gflip);
+                tc_values<false, false, CH>(coef, x, u1, u2, sc, 0, gflip, out, lane);
             else
-                tc_chunk<true, false, CH>(coef, x, u1, u2, sc, tA, 0, gflip);
+                tc_values<true, false, CH>(coef, x, u1, u2, sc, 0, gflip, out, lane);
             if (!f || c == 0) {
                 fast = true;
 #pragma unroll
                 for (int e = 0; e < CH; ++e) fast &= sc[e] == 0;
+            }
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&sm.fullX[sX][warp]);
+                mbar_arrive(&sm.emptyB[sB]);
+            }
+        }
+    }
+    if (!ok) tc_fail(&sm.fail, p.err);
+}
+
+// ---------------------------------------------------------------------------------
+// split warps: FP32 values -> A operands in tensor memory
+// ---------------------------------------------------------------------------------
+template <int SPIN, int BM>
+__device__ void tc_split(const TcParams &p, TcSmem<SPIN, BM> &sm, uint32_t tbase, int warp, int lane) {
+    using C = TcCfg<SPIN, BM>;
+    constexpr int CH = C::CH;
+    constexpr uint32_t AC = kTcK / 2;
+    const int j0 = (warp >> 2) * CH;
+    const uint32_t tl = tbase + ((uint32_t)((warp & 3) * 32) << 16);  // warp w reaches lanes 32 (w % 4) ..
+    unsigned gc = 0;
+    bool ok = true;
+    for (int it = blockIdx.x; it < p.norder && ok; it += gridDim.x) {
+        if (tc_failed(&sm.fail)) break;
+        const TcItem q = tc_item_of(p, __ldg(&p.order[it]));
+        for (int c = 0; c < q.nck; ++c, ++gc) {
+            const int sA = gc % C::NSA, sX = gc % C::NSX;
+            if (!mbar_wait_warp(&sm.fullX[sX][warp], (gc / C::NSX) & 1u, p.wait_ns)) { ok = false; break; }
+            if (gc >= (unsigned)C::NSA && !mbar_wait_warp(&sm.emptyA[sA], ((gc / C::NSA) - 1u) & 1u, p.wait_ns)) { ok = false; break; }
+            tc_fence_after();  // the stage's previous MMAs are complete before it is overwritten
+#pragma unroll
+            for (int e = 0; e < CH; ++e) {
+                const uint32_t tA = tl + (uint32_t)(C::COL_A + (sA * C::NG + j0 + e) * 3 * C::ACOLS);
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const float4 a = sm.x[sX][warp][e * 4 + half * 2][lane], b = sm.x[sX][warp][e * 4 + half * 2 + 1][lane];
+                    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                    uint32_t pk[3][4];
+                    split3_packf8(v, pk);
+#pragma unroll
+                    for (int sp = 0; sp < 3; ++sp) tmem_st4(tA + sp * AC + half * 4, pk[sp][0], pk[sp][1], pk[sp][2], pk[sp][3]);
+                }
             }
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(&sm.fullA[sA]);
-                mbar_arrive(&sm.emptyB[sB]);
-            }
-            const bool last = c == q.nck - 1;
-            if ((c % p.flush) == p.flush - 1 || last) {
-                const unsigned kb = bk & 1u;
-                if (!mbar_wait_warp(&sm.accFull[kb], (bk >> 1) & 1u, p.wait_ns)) { ok = false; break; }
-                tc_fence_after();
-                const bool first_block = c < p.flush;
-#pragma unroll 1
-                for (int e = 0; e < CH; ++e) {
-                    const int j = j0 + e;
-                    double *accj = &sm.acc[j][0][0];
-                    const uint32_t th = tl + (uint32_t)((kb * C::NG + j) * N);
-#pragma unroll 1
-                    for (int col = 0; col < N; col += 32) fold32(accj, th + col, col, row, first_block);
-                    if (last) {
-                        const uint32_t tcorr = tl + (uint32_t)(C::COL_CORR + j * N);
-#pragma unroll 1
-                        for (int col = 0; col < N; col += 32) fold32(accj, tcorr + col, col, row, false);
-                    }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&sm.accEmpty[kb]);
-                    if (last) mbar_arrive(&sm.corrEmpty);
-                }
-                ++bk;
-                if (last) {
-                    // the item's spectra for every map of the group
-#pragma unroll 1
-                    for (int e = 0; e < CH; ++e) {
-                        const int j = j0 + e, t = tr[e];
-                        if (t >= p.T) continue;
-                        for (int bm = 0; bm < nb; ++bm) {
-                            double v[4];
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) v[u] = sm.acc[j][4 * bm + u][row];
-                            tc_store_F<SPIN>(p, F_all, bm, SPIN ? j : 0, t, q.m, q.lmin, v);
-                        }
-                    }
-                }
+                mbar_arrive(&sm.emptyX[sX][warp]);
             }
         }
-        if (ok && q.nck == 0) {
-            // no representable term in this tile: the rows are exactly zero
-            const double z[4] = {0.0, 0.0, 0.0, 0.0};
+    }
+    if (!ok) tc_fail(&sm.fail, p.err);
+}
+
+// ---------------------------------------------------------------------------------
+// fold warps: FP32 block sums -> FP64 sums, and the item's output
+// ---------------------------------------------------------------------------------
+template <int SPIN, int BM>
+__device__ void tc_fold(const TcParams &p, TcSmem<SPIN, BM> &sm, double2 *__restrict__ F_all, int nb, uint32_t tbase,
+                        int warp, int lane) {
+    using C = TcCfg<SPIN, BM>;
+    constexpr int N = C::N;
+    constexpr int CH = C::CH;
+    const int row = (warp & 3) * 32 + lane;  // A row = TMEM lane
+    const int j0 = (warp >> 2) * CH;
+    const uint32_t tl = tbase + ((uint32_t)((warp & 3) * 32) << 16);
+    unsigned bk = 0;
+    bool ok = true;
+    for (int it = blockIdx.x; it < p.norder && ok; it += gridDim.x) {
+        if (tc_failed(&sm.fail)) break;
+        const TcItem q = tc_item_of(p, __ldg(&p.order[it]));
+        const int nfb = (q.nck + p.flush - 1) / p.flush;
+        for (int fb = 0; fb < nfb; ++fb, ++bk) {
+            const unsigned kb = bk & 1u;
+            const bool last = fb == nfb - 1;
+            if (!mbar_wait_warp(&sm.accFull[kb], (bk >> 1) & 1u, p.wait_ns)) { ok = false; break; }
+            tc_fence_after();
+            bool first = fb == 0;
+            if (last) {  // the correction sums first: the next item's products wait for their columns
+#pragma unroll 1
+                for (int e = 0; e < CH; ++e)
+#pragma unroll 1
+                    for (int col = 0; col < N; col += 32)
+                        fold32(&sm.acc[j0 + e][0][0], tl + (uint32_t)(C::COL_CORR + (j0 + e) * N + col), col, row, first);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm.corrEmpty);
+                first = false;
+            }
+#pragma unroll 1
+            for (int e = 0; e < CH; ++e)
+#pragma unroll 1
+                for (int col = 0; col < N; col += 32)
+                    fold32(&sm.acc[j0 + e][0][0], tl + (uint32_t)((kb * C::NG + j0 + e) * N + col), col, row, first);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.accEmpty[kb]);
+        }
+        if (!ok) break;
+        // the item's spectra for every map of the group (no representable term: exactly zero)
+#pragma unroll 1
+        for (int e = 0; e < CH; ++e) {
+            const int j = j0 + e, t = tc_ring<SPIN>(q.tile, j, row);
+            if (t >= p.T) continue;
+            for (int bm = 0; bm < nb; ++bm) {
+                double w[4];
 #pragma unroll
-            for (int e = 0; e < CH; ++e) {
-                const int t = tr[e];
-                if (t < p.T)
-                    for (int bm = 0; bm < nb; ++bm) tc_store_F<SPIN>(p, F_all, bm, SPIN ? j0 + e : 0, t, q.m, q.lmin, z);
+                for (int u = 0; u < 4; ++u) w[u] = nfb > 0 ? sm.acc[j][4 * bm + u][row] : 0.0;
+                tc_store_F<SPIN>(p, F_all, bm, SPIN ? j : 0, t, q.m, q.lmin, w);
             }
         }
     }
@@ -365,88 +421,105 @@ template <int SPIN, int BM>
 __device__ void tc_loader(const TcParams &p, TcSmem<SPIN, BM> &sm, int lane) {
     using C = TcCfg<SPIN, BM>;
     if (p.inject == kInjectStall) return;  // test hook: no stage is ever published
-    const int nitems = p.norder;
-    unsigned gc = 0;
-    bool ok = true;
-    for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
-        if (tc_failed(&sm.fail)) break;
-        const TcItem q = tc_item_of(p, __ldg(&p.order[it]));
-        const size_t base = (size_t)__ldg(&p.cbase[q.m]) + q.c0;
-        for (int c = 0; c < q.nck; ++c, ++gc) {
-            const int sB = gc % C::NSB;
-            if (gc >= (unsigned)C::NSB && !mbar_wait_warp(&sm.emptyB[sB], ((gc / C::NSB) - 1u) & 1u, p.wait_ns)) {
-                ok = false;
-                break;
-            }
-            if (lane == 0) {
+    if (lane == 0) {
+        unsigned gc = 0;
+        bool ok = true;
+        for (int it = blockIdx.x; it < p.norder && ok; it += gridDim.x) {
+            if (*(volatile int *)&sm.fail) break;
+            const TcItem q = tc_item_of(p, __ldg(&p.order[it]));
+            const size_t base = (size_t)__ldg(&p.cbase[q.m]) + q.c0;
+            for (int c = 0; c < q.nck; ++c, ++gc) {
+                const int sB = gc % C::NSB;
+                if (gc >= (unsigned)C::NSB && !mbar_wait(&sm.emptyB[sB], ((gc / C::NSB) - 1u) & 1u, p.wait_ns)) {
+                    ok = false;
+                    break;
+                }
                 mbar_arrive_tx(&sm.fullB[sB], C::BBYTES);
                 bulk_g2s(sm.B[sB], p.Bt + (base + c) * C::BBYTES, C::BBYTES, &sm.fullB[sB]);
             }
-            __syncwarp();
         }
+        if (!ok) tc_fail(&sm.fail, p.err);
     }
-    if (!ok) tc_fail(&sm.fail, p.err);
+    __syncwarp();
 }
 
 // ---------------------------------------------------------------------------------
-// MMA warp: one thread issues the split products and the commits
+// MMA warp: one thread issues the split products and the commits; stage indices and parities
+// are counters and the descriptors offsets from the first stage's, so that few instructions
+// stand between two products
 // ---------------------------------------------------------------------------------
 template <int SPIN, int BM>
 __device__ void tc_mma(const TcParams &p, TcSmem<SPIN, BM> &sm, uint32_t tbase, int lane) {
     using C = TcCfg<SPIN, BM>;
     constexpr int N = C::N;
     constexpr uint32_t IDESC = idesc_bf16(kTcRows, N);
-    const int nitems = p.norder;
-    unsigned gc = 0, bk = 0, ncorr = 0;
-    bool ok = true;
-    for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
-        if (tc_failed(&sm.fail)) break;
-        const TcItem q = tc_item_of(p, __ldg(&p.order[it]));
-        for (int c = 0; c < q.nck; ++c, ++gc) {
-            const int sA = gc % C::NSA, sB = gc % C::NSB;
-            const bool bstart = (c % p.flush) == 0;
-            const bool bend = (c % p.flush) == p.flush - 1 || c == q.nck - 1;
-            const unsigned kb = bk & 1u;
-            if (!mbar_wait_warp(&sm.fullA[sA], (gc / C::NSA) & 1u, p.wait_ns) ||
-                !mbar_wait_warp(&sm.fullB[sB], (gc / C::NSB) & 1u, p.wait_ns) ||
-                (bstart && bk >= 2 && !mbar_wait_warp(&sm.accEmpty[kb], ((bk >> 1) - 1u) & 1u, p.wait_ns)) ||
-                (c == 0 && ncorr > 0 && !mbar_wait_warp(&sm.corrEmpty, (ncorr - 1u) & 1u, p.wait_ns))) {
-                ok = false;
-                break;
-            }
-            tc_fence_after();
-            if (lane == 0) {
-#pragma unroll
-                for (int j = 0; j < C::NG; ++j) {
-                    const int jb = SPIN ? j : 0;
-                    const uint32_t d = tbase + (uint32_t)((kb * C::NG + j) * N);
-                    const uint32_t dc = tbase + (uint32_t)(C::COL_CORR + j * N);
-                    const uint32_t a0 = tbase + (uint32_t)(C::COL_A + (sA * C::NG + j) * 3 * C::ACOLS);
-                    const uint32_t a1 = a0 + C::ACOLS, a2 = a0 + 2 * C::ACOLS;
-                    const unsigned char *Bj = sm.B[sB] + jb * 3 * C::BTILE;
-                    const uint64_t c0 = smem_desc(Bj, 128, 256), c1 = smem_desc(Bj + C::BTILE, 128, 256),
-                                   c2 = smem_desc(Bj + 2 * C::BTILE, 128, 256);
-                    umma_f16_ts(d, a0, c0, IDESC, bstart ? 0u : 1u);  // hh
-                    umma_f16_ts(dc, a0, c1, IDESC, c == 0 ? 0u : 1u); // hm
-                    umma_f16_ts(dc, a1, c0, IDESC, 1u);               // mh
-                    umma_f16_ts(dc, a0, c2, IDESC, 1u);               // hl
-                    umma_f16_ts(dc, a2, c0, IDESC, 1u);               // lh
-                    umma_f16_ts(dc, a1, c1, IDESC, 1u);               // mm
+    if (lane == 0) {
+        unsigned bk = 0, ncorr = 0;
+        int sA = 0, sB = 0;
+        uint32_t phA = 0, phB = 0;
+        bool ok = true;
+        const uint64_t dB0 = smem_desc(sm.B[0], 128, 256);
+        for (int it = blockIdx.x; it < p.norder && ok; it += gridDim.x) {
+            if (*(volatile int *)&sm.fail) break;
+            const TcItem q = tc_item_of(p, __ldg(&p.order[it]));
+            int fcount = 0;  // chunks of the current FP32 accumulation block so far
+            for (int c = 0; c < q.nck; ++c) {
+                const bool bstart = fcount == 0;
+                const bool bend = fcount == p.flush - 1 || c == q.nck - 1;
+                const unsigned kb = bk & 1u;
+                if (!mbar_wait(&sm.fullB[sB], phB, p.wait_ns) || !mbar_wait(&sm.fullA[sA], phA, p.wait_ns) ||
+                    (bstart && bk >= 2 && !mbar_wait(&sm.accEmpty[kb], ((bk >> 1) - 1u) & 1u, p.wait_ns)) ||
+                    (c == 0 && ncorr > 0 && !mbar_wait(&sm.corrEmpty, (ncorr - 1u) & 1u, p.wait_ns))) {
+                    ok = false;
+                    break;
                 }
+                tc_fence_after();
+                const uint64_t dS = dB0 + (uint64_t)((sB * C::BSTRIDE) >> 4);
+                const uint32_t aS = tbase + (uint32_t)(C::COL_A + sA * C::NG * 3 * C::ACOLS);
+                const uint32_t dh = tbase + (uint32_t)(kb * C::NG * N), dc = tbase + (uint32_t)C::COL_CORR;
+                // the two GEMMs alternate, so that products into one accumulator do not follow one
+                // another directly (nside 1024 / lmax 2048, 16 maps: 16.9 -> 16.4 ms)
+                constexpr uint64_t T = C::BTILE >> 4;
+                const uint64_t dS1 = dS + (SPIN ? 3 * T : 0);
+                const uint32_t aT = aS + 3 * C::ACOLS, dh1 = dh + N, dc1 = dc + N;
+                constexpr uint32_t AM = C::ACOLS, AL = 2 * C::ACOLS;
+                const uint32_t zc = c == 0 ? 0u : 1u, zh = bstart ? 0u : 1u;
+                umma_f16_ts(dc, aS, dS + T, IDESC, zc);             // hm
+                umma_f16_ts(dc1, aT, dS1 + T, IDESC, zc);
+                umma_f16_ts(dh, aS, dS, IDESC, zh);                 // hh
+                umma_f16_ts(dc, aS + AM, dS, IDESC, 1u);            // mh
+                umma_f16_ts(dc1, aT + AM, dS1, IDESC, 1u);
+                umma_f16_ts(dh1, aT, dS1, IDESC, zh);
+                umma_f16_ts(dc, aS, dS + 2 * T, IDESC, 1u);         // hl
+                umma_f16_ts(dc1, aT, dS1 + 2 * T, IDESC, 1u);
+                umma_f16_ts(dc, aS + AL, dS, IDESC, 1u);            // lh
+                umma_f16_ts(dc1, aT + AL, dS1, IDESC, 1u);
+                umma_f16_ts(dc, aS + AM, dS + T, IDESC, 1u);        // mm
+                umma_f16_ts(dc1, aT + AM, dS1 + T, IDESC, 1u);
                 umma_commit(&sm.emptyA[sA]);
                 umma_commit(&sm.emptyB[sB]);
                 if (bend) umma_commit(&sm.accFull[kb]);
+                if (++sA == C::NSA) {
+                    sA = 0;
+                    phA ^= 1u;
+                }
+                if (++sB == C::NSB) {
+                    sB = 0;
+                    phB ^= 1u;
+                }
+                if (bend) {
+                    ++bk;
+                    fcount = 0;
+                } else {
+                    ++fcount;
+                }
             }
-            __syncwarp();
-            if (bend) ++bk;
+            if (ok && q.nck > 0) ++ncorr;
         }
-        if (ok && q.nck > 0) ++ncorr;
-    }
-    if (!ok) tc_fail(&sm.fail, p.err);
-    // every issued MMA has completed before tensor memory is released
-    if (lane == 0) {
+        if (!ok) tc_fail(&sm.fail, p.err);
+        // every issued MMA has completed before tensor memory is released
         umma_commit(&sm.fin);
-        if (!mbar_wait(&sm.fin, 0u, p.wait_ns)) tc_fail(&sm.fail, p.err);  // lane 0 alone
+        if (!mbar_wait(&sm.fin, 0u, p.wait_ns)) tc_fail(&sm.fail, p.err);
     }
     __syncwarp();
 }
@@ -468,6 +541,11 @@ __global__ void __launch_bounds__(TcCfg<SPIN, BM>::NTHREADS, 1)
             mbar_init(&sm.fullA[s], C::NPW);
             mbar_init(&sm.emptyA[s], 1);
         }
+        for (int s = 0; s < C::NSX; ++s)
+            for (int w = 0; w < C::NPW; ++w) {
+                mbar_init(&sm.fullX[s][w], 1);
+                mbar_init(&sm.emptyX[s][w], 1);
+            }
         for (int s = 0; s < C::NSB; ++s) {
             mbar_init(&sm.fullB[s], 1);
             mbar_init(&sm.emptyB[s], 1 + C::NPW);
@@ -486,7 +564,11 @@ __global__ void __launch_bounds__(TcCfg<SPIN, BM>::NTHREADS, 1)
     tc_fence_after();
     const uint32_t tbase = sm.taddr;
     if (warp < C::NPW) {
-        tc_producer<SPIN, BM>(p, sm, F_all, nb, tbase, warp, lane);
+        tc_recursion<SPIN, BM>(p, sm, warp, lane);
+    } else if (warp < 2 * C::NPW) {
+        tc_split<SPIN, BM>(p, sm, tbase, warp - C::NPW, lane);
+    } else if (warp < 3 * C::NPW) {
+        tc_fold<SPIN, BM>(p, sm, F_all, nb, tbase, warp - 2 * C::NPW, lane);
     } else if (warp == C::LOAD_WARP) {
         tc_loader<SPIN, BM>(p, sm, lane);
     } else {
