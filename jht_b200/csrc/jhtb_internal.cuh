@@ -64,7 +64,10 @@ constexpr long long kSmallAdjItems = 16384;
 constexpr int kTcMaps = JHTB_TC_MAPS;  // maps per tensor-core pass (N = 4 * maps per GEMM)
 
 // Azimuthal stage (ringfft.cu).
-constexpr int kTwLen = 32768;      // twiddle table length: every FFT length divides it
+// Twiddles of an FFT pass over blocks of 2^b points, 5 <= b <= 13: for each j < 2^b / 16 the four
+// entries e^{-2 pi i j a / 2^b}, a = 1, 4, 8, 12, next to one another.
+__host__ __device__ constexpr int tw_offset(int b) { return 4 * ((1 << (b - 4)) - 2); }
+constexpr int kTwLen = tw_offset(14);
 constexpr int kFftPiece = 4096;    // points of one FFT of the 256-thread kernels
 constexpr int kRingThreads = 256;  // threads of a ring CTA
 constexpr int kSmallRing = 128;    // rings up to this length run as a plain sum
@@ -124,7 +127,7 @@ struct Plan {
     double *d_logch;    // [T] log cos(theta/2)    (spin 2 seeds)
     double *d_logsh;    // [T] log sin(theta/2)
     RingDesc *d_rings;  // [nrings]
-    double2 *d_tw;      // [kTwLen] exp(-2 pi i k / kTwLen)
+    double2 *d_tw;      // [kTwLen] FFT pass twiddles (tw_offset)
     double2 *d_bh;      // chirp spectra, FFT_P(conj(w))/P, per distinct chirp length
     double2 *d_ctab;    // chirp, piece and ring-phase factors per distinct chirp length
     double2 *d_belt;    // [2 belt_n] e^{i pi a / belt_n} of a power-of-two belt

@@ -629,10 +629,13 @@ int build_plan(Plan *p, const jhtb_host_tables *ht) {
         if ((rc = build_ring_lists(p, bytes))) return rc;
 
         std::vector<double2> tw(kTwLen);
-        for (int k = 0; k < kTwLen; ++k) {
-            long double a = -2.0L * 3.14159265358979323846264338327950288L * (long double)k / (long double)kTwLen;
-            tw[k] = make_double2((double)cosl(a), (double)sinl(a));
-        }
+        for (int b = 5; b <= 13; ++b)
+            for (int j = 0; j < 1 << (b - 4); ++j)
+                for (int e = 0; e < 4; ++e) {
+                    const int k = j * (e ? 4 * e : 1);
+                    const long double a = -2.0L * 3.14159265358979323846264338327950288L * (long double)k / (long double)(1 << b);
+                    tw[tw_offset(b) + 4 * j + e] = make_double2((double)cosl(a), (double)sinl(a));
+                }
         if ((rc = upload(&p->d_tw, tw, bytes))) return rc;
         JHTB_CUDA_TRY(cudaMalloc((void **)&p->d_bh, sizeof(double2) * std::max(bo, 1LL)));
         JHTB_CUDA_TRY(cudaMalloc((void **)&p->d_ctab, sizeof(double2) * std::max(co, 1LL)));
