@@ -279,6 +279,22 @@ int jhtb_fft_c2c(const void *in, void *out, int n, int64_t howmany, int64_t inne
                  int64_t in_dist_outer, int64_t in_dist_inner, int64_t out_stride, int64_t out_dist_outer,
                  int64_t out_dist_inner, int sign, double scale, int64_t twiddle_n, const void *roots, void *stream);
 
+/* Off-grid transforms' torus grid (jht _nufft.py:164-191 and offgrid.py:126-139), in one call of
+ * batched FFTs.  F: [ncomp][ns][lmax + 1] complex FP64 ring coefficients (+spin, -spin) on ns
+ * equispaced colatitudes 0 .. pi; they are extended to the 2 ns - 2 samples of the full circle
+ * (times (-1)^(m + spin) across the poles), transformed in theta (scaled by 1 / (2 ns - 2)),
+ * multiplied by the deconvolution factors ick[2 ns - 2] x icm[2 lmax + 1] (centred), zero padded
+ * and transformed to the nk x nm grid (unscaled, sign +1).  The adjoint runs the transposes in
+ * reverse order and returns V in F's layout.  roots_n: e^{-2 pi i k / n} for k < n (n = 2 ns - 2,
+ * nk, nm) or NULL; work: (2 ns - 2) (2 lmax + 1 + nm) complex values.  Lengths must be
+ * 2,3,5-smooth and within jhtb_fft_c2c's limit. */
+int jhtb_torus_grid(const void *F, int ncomp, int lmax, int ns, int spin, int nk, int nm, const double *ick,
+                    const double *icm, const void *roots_nd, const void *roots_nk, const void *roots_nm, void *work,
+                    void *grid, void *stream);
+int jhtb_torus_grid_adjoint(const void *grid, int ncomp, int lmax, int ns, int spin, int nk, int nm, const double *ick,
+                            const double *icm, const void *roots_nd, const void *roots_nk, const void *roots_nm,
+                            void *work, void *V, void *stream);
+
 /* Bounds-check record of a debug library (no counterpart in jht; the replacement for a
  * memory checker on machines where none can run).  A library built with `make debug`
  * (jht_b200/_lib_debug/libjhtb.so, -DJHTB_DEBUG) tests every checked gather and scatter

@@ -57,6 +57,8 @@ EXPORTS = (
     "jhtb_nufft_spread_tiles",
     "jhtb_debug_bounds",
     "jhtb_fft_c2c",
+    "jhtb_torus_grid",
+    "jhtb_torus_grid_adjoint",
     "jhtb_real_to_alm",
     "jhtb_alm_to_real",
     "jhtb_synthesis_cotangent",
@@ -133,6 +135,8 @@ def load_library(path: str | os.PathLike | None = None):
             "jhtb_synthesis_cotangent": (i32, [i32, i32, i32, vp, vp]),
             "jhtb_fft_c2c": (i32, [vp, vp, i32, i64, i64, i64, i64, i64, i64, i64, i64, i32, ctypes.c_double, i64,
                                    vp, vp]),
+            "jhtb_torus_grid": (i32, [vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp]),
+            "jhtb_torus_grid_adjoint": (i32, [vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp]),
         }
         for name, (res, args) in sig.items():
             f = getattr(lib, name)

@@ -10,14 +10,15 @@ matches ducc's ``sphere_interpol``), mapped onto the device:
    kernels on a ring-set plan (``jhtb_plan_create_rings`` + ``jhtb_legendre_synthesis``);
 2. the double-Fourier-sphere extension to the 2 pi theta period and a theta FFT
    (offgrid.py:113-129), then the deconvolution by the kernel's Fourier transform and an
-   inverse 2D FFT onto the oversampled torus grid (_nufft.py:164-174) -- gathers and the
-   library's FFT kernel (``jhtb_fft_c2c``, 2,3,5-smooth lengths; the 2-D transform skips
-   the grid's all-zero rows);
+   inverse 2D FFT onto the oversampled torus grid (_nufft.py:164-174) -- one
+   library call (``jhtb_torus_grid``: three batched FFTs of 2,3,5-smooth lengths that
+   extend, centre and zero-pad where they read and write); lengths above the one-CTA
+   limit run as gathers around ``jhtb_fft_c2c``;
 3. the W x W exponential-of-semicircle window sums at the points
    (``jhtb_nufft_interp``, _nufft.py:150-178).
 
 The adjoint runs the transposes in reverse order (``jhtb_nufft_spread`` with FP64
-atomics, forward FFT, transposed extension, ``jhtb_legendre_adjoint``).
+atomics, ``jhtb_torus_grid_adjoint``, ``jhtb_legendre_adjoint``).
 
 Accuracy is set by ``epsilon`` through jht's kernel table (W = 14 at the default 1e-10);
 torch autograd gives the alm gradient (the adjoint, jht's VJP convention) and the
@@ -99,13 +100,15 @@ class _Geometry:
         dev = torch.device("cuda", device)
         ck = _kernel_ft(self.nd, self.nk, self.W, self.beta)
         cm = _kernel_ft(self.Nm, self.nm, self.W, self.beta)
-        self.inv_corr = torch.as_tensor(1.0 / np.outer(ck, cm), device=dev)  # (nd, Nm) centered
+        self.ick, self.icm = (torch.as_tensor(1.0 / c, device=dev) for c in (ck, cm))  # centred
         self.kpos = torch.as_tensor(np.arange(-(self.nd // 2), -(self.nd // 2) + self.nd) % self.nk, device=dev)
         self.mpos = torch.as_tensor(np.arange(-lmax, lmax + 1) % self.nm, device=dev)
         mv = np.arange(-lmax, lmax + 1)
         self.sign_m = torch.as_tensor(((-1.0) ** np.abs(mv)) * ((-1.0) ** spin), device=dev)
         self.south = torch.arange(self.ns, self.nd, device=dev)
         self.refl = self.nd - self.south
+        # every length within one CTA's FFT: the torus grid is one library call
+        self.one_call = max(self.nd, self.nk, self.nm) <= _fft.SM_MAX
         self.metric = torch.as_tensor(np.array(alm_metric_weight(lmax)), device=dev)
         with torch.cuda.device(device):
             self.plan = _lib.Plan(0, lmax, spin, "fp64", 1, device=device, rings=(self.ns, x))
@@ -171,9 +174,21 @@ def _ring_coeffs(g: _Geometry, alm: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def _torus_args(g: _Geometry, device: torch.device):
+    """The arguments that the two torus grid calls share, with a fresh workspace."""
+    work = torch.empty(g.nd * (g.Nm + g.nm), dtype=torch.complex128, device=device)
+    roots = [_fft._roots(n, device.index).data_ptr() for n in (g.nd, g.nk, g.nm)]
+    return (g.ncomp, g.lmax, g.ns, g.spin, g.nk, g.nm, g.ick.data_ptr(), g.icm.data_ptr(), *roots, work.data_ptr()), work
+
+
 def _torus_grid(g: _Geometry, F: torch.Tensor) -> torch.Tensor:
     """Ring coefficients -> samples of the field's torus extension on the nk x nm grid,
     deconvolved by the window's transform (offgrid.py:126-139, _nufft.py:164-174)."""
+    if g.one_call:
+        grid = torch.empty((g.nk, g.nm), dtype=torch.complex128, device=F.device)
+        args, work = _torus_args(g, F.device)
+        _lib.check(g.plan.lib.jhtb_torus_grid(F.data_ptr(), *args, grid.data_ptr(), _stream()), "jhtb_torus_grid")
+        return grid
     L, ns, nd = g.lmax, g.ns, g.nd
     Fp, Fm = F[0], F[-1]
     cols = torch.zeros((nd, g.Nm), dtype=torch.complex128, device=F.device)
@@ -185,7 +200,7 @@ def _torus_grid(g: _Geometry, F: torch.Tensor) -> torch.Tensor:
     # the unscaled inverse 2-D FFT of the zero-padded grid: rows first, only the nd non-zero
     # rows (the other rows stay zero), then every column
     Crow = torch.zeros((nd, g.nm), dtype=torch.complex128, device=F.device)
-    Crow[:, g.mpos] = Fk * g.inv_corr
+    Crow[:, g.mpos] = Fk * g.ick[:, None] * g.icm
     C = torch.zeros((g.nk, g.nm), dtype=torch.complex128, device=F.device)
     C[g.kpos] = _fft.fft(Crow, 1, +1)
     return _fft.fft(C, 0, +1)
@@ -232,10 +247,35 @@ def _field_of(g: _Geometry, f: torch.Tensor) -> torch.Tensor:
 # ---------------------------------------------------------------------------------------
 # adjoint: points -> grid -> ring coefficients -> alm
 # ---------------------------------------------------------------------------------------
+def _torus_grid_adjoint(g: _Geometry, grid: torch.Tensor) -> torch.Tensor:
+    """The transpose of _torus_grid: (ncomp, ns, lmax + 1) ring coefficients."""
+    L, ns, nd = g.lmax, g.ns, g.nd
+    if g.one_call:
+        V = torch.empty((g.ncomp, ns, L + 1), dtype=torch.complex128, device=grid.device)
+        args, work = _torus_args(g, grid.device)
+        _lib.check(g.plan.lib.jhtb_torus_grid_adjoint(grid.data_ptr(), *args, V.data_ptr(), _stream()),
+                   "jhtb_torus_grid_adjoint")
+        return V
+    # the forward 2-D FFT restricted to the nd x Nm centred modes: every column, then the
+    # nd rows that are kept; then the scaled inverse theta FFT of the uncentred columns
+    G = _fft.fft(_fft.fft(grid, 0, -1)[g.kpos], 1, -1)[:, g.mpos] * g.ick[:, None] * g.icm
+    d = _fft.fft(torch.roll(G, -(nd // 2), dims=0), 0, +1, 1.0 / nd)
+    top = d[:ns].clone()
+    top.index_add_(0, g.refl, g.sign_m[None, :] * d[g.south])
+    V = torch.zeros((g.ncomp, ns, L + 1), dtype=torch.complex128, device=grid.device)
+    Vm = torch.zeros((ns, L + 1), dtype=torch.complex128, device=grid.device)
+    Vm[:, 1:] = torch.conj(torch.flip(top[:, :L], dims=(1,)))
+    if g.spin == 0:
+        V[0] = top[:, L:] + Vm
+    else:
+        V[0] = top[:, L:]
+        V[1] = Vm
+    return V
+
+
 def _adjoint(g: _Geometry, fc: torch.Tensor, theta: torch.Tensor, phi: torch.Tensor) -> torch.Tensor:
     """Complex point values -> (ncomp, K) alm, the transpose of _forward's value path
     divided by the metric (offgrid.py:223-243)."""
-    L, ns, nd = g.lmax, g.ns, g.nd
     grid = torch.zeros((g.nk, g.nm), dtype=torch.complex128, device=fc.device)
     po = _point_order(g, theta, phi)
     if po is not None:
@@ -251,21 +291,8 @@ def _adjoint(g: _Geometry, fc: torch.Tensor, theta: torch.Tensor, phi: torch.Ten
         st = g.plan.lib.jhtb_nufft_spread(fc.contiguous().data_ptr(), theta.data_ptr(), phi.data_ptr(), theta.numel(),
                                           g.nk, g.nm, g.W, ctypes.c_double(g.beta), grid.data_ptr(), _stream())
         _lib.check(st, "jhtb_nufft_spread")
-    # the forward 2-D FFT restricted to the nd x Nm centred modes: every column, then the
-    # nd rows that are kept; then the scaled inverse theta FFT of the uncentred columns
-    G = _fft.fft(_fft.fft(grid, 0, -1)[g.kpos], 1, -1)[:, g.mpos] * g.inv_corr
-    d = _fft.fft(torch.roll(G, -(nd // 2), dims=0), 0, +1, 1.0 / nd)
-    top = d[:ns].clone()
-    top.index_add_(0, g.refl, g.sign_m[None, :] * d[g.south])
-    V = torch.zeros((g.ncomp, ns, L + 1), dtype=torch.complex128, device=fc.device)
-    Vm = torch.zeros((ns, L + 1), dtype=torch.complex128, device=fc.device)
-    Vm[:, 1:] = torch.conj(torch.flip(top[:, :L], dims=(1,)))
-    if g.spin == 0:
-        V[0] = top[:, L:] + Vm
-    else:
-        V[0] = top[:, L:]
-        V[1] = Vm
-    a = torch.empty((g.ncomp, alm_size(L)), dtype=torch.complex128, device=fc.device)
+    V = _torus_grid_adjoint(g, grid)
+    a = torch.empty((g.ncomp, alm_size(g.lmax)), dtype=torch.complex128, device=fc.device)
     st = g.plan.lib.jhtb_legendre_adjoint(g.plan.handle, V.data_ptr(), a.data_ptr(), 1, _stream())
     _lib.check(st, "jhtb_legendre_adjoint")
     # the library's spin-2 form is (1/2)(-p - n), (i/2)(p - n); jht's off-grid one has no 1/2
