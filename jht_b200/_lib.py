@@ -341,6 +341,9 @@ def get_plan(nside: int, lmax: int, spin: int, precision: str = "fp64", batch: i
     import torch
 
     dev = torch.cuda.current_device()
+    plan = _plans.get((dev, nside, lmax, spin, precision))
+    if plan is not None and plan.max_batch >= batch:  # holds the batch: no budget to work out
+        return plan
     per = workspace_bytes_per_map(nside, lmax, spin)
     if precision == "bf16x3":
         # the tensor-core path shares one recursion among the maps of a pass: hold whole
@@ -384,4 +387,5 @@ def clear_plans() -> None:
 def stream_ptr():
     import torch
 
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the handle of torch.cuda.current_stream(), without building a Stream object
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))

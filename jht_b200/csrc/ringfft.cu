@@ -859,18 +859,15 @@ JHTB_DEBUG_ACCESSOR(ringfft)
 
 int launch_ring_synth(const Plan &p, const double2 *F, double *maps, int nb, cudaStream_t s) {
     if (nb <= 0) return JHTB_OK;
-    int rc;
     RingArgs a = make_args(p);
     const size_t fmap = (size_t)p.ncomp * p.nrings * p.M;
     const long long pmap = (long long)p.ncomp * p.npix;
     if (p.nunit_long > 0) {
-        if ((rc = ensure_smem(ring_long_kernel<false>, kLongSmem))) return rc;
         a.units = p.d_ring_units + p.nunit;
         ring_long_kernel<false><<<dim3(p.nunit_long, nb), 512, kLongSmem, s>>>(a, F, nullptr, nullptr, maps, fmap, pmap);
         JHTB_CUDA_TRY(cudaGetLastError());
     }
     if (p.nunit > 0) {
-        if ((rc = ensure_smem(ring_synth_kernel, kRingSmem))) return rc;
         a.units = p.d_ring_units;
         ring_synth_kernel<<<dim3(p.nunit, nb), kRingThreads, kRingSmem, s>>>(a, F, maps, fmap, pmap);
         JHTB_CUDA_TRY(cudaGetLastError());
@@ -880,18 +877,15 @@ int launch_ring_synth(const Plan &p, const double2 *F, double *maps, int nb, cud
 
 int launch_ring_adjoint(const Plan &p, const double *maps, double2 *V, int nb, cudaStream_t s) {
     if (nb <= 0) return JHTB_OK;
-    int rc;
     RingArgs a = make_args(p);
     const size_t fmap = (size_t)p.ncomp * p.nrings * p.M;
     const long long pmap = (long long)p.ncomp * p.npix;
     if (p.nunit_long > 0) {
-        if ((rc = ensure_smem(ring_long_kernel<true>, kLongSmem))) return rc;
         a.units = p.d_ring_units + p.nunit;
         ring_long_kernel<true><<<dim3(p.nunit_long, nb), 512, kLongSmem, s>>>(a, nullptr, V, maps, nullptr, fmap, pmap);
         JHTB_CUDA_TRY(cudaGetLastError());
     }
     if (p.nunit > 0) {
-        if ((rc = ensure_smem(ring_adjoint_kernel, kRingSmem))) return rc;
         a.units = p.d_ring_units;
         ring_adjoint_kernel<<<dim3(p.nunit, nb), kRingThreads, kRingSmem, s>>>(a, maps, V, fmap, pmap);
         JHTB_CUDA_TRY(cudaGetLastError());
@@ -901,6 +895,11 @@ int launch_ring_adjoint(const Plan &p, const double *maps, double2 *V, int nb, c
 
 int launch_ring_tables(const Plan &p, const int *lens, const long long *ctab_offs, const long long *bh_offs,
                        const int (&count)[14], cudaStream_t s) {
+    int rc;
+    // the kernels' shared-memory limits, once per plan (on its device) instead of at each launch
+    if ((rc = ensure_smem(ring_synth_kernel, kRingSmem)) || (rc = ensure_smem(ring_adjoint_kernel, kRingSmem)) ||
+        (rc = ensure_smem(ring_long_kernel<false>, kLongSmem)) || (rc = ensure_smem(ring_long_kernel<true>, kLongSmem)))
+        return rc;
     if (p.belt_n > 0) {
         belt_table_kernel<<<(2 * p.belt_n + 255) / 256, 256, 0, s>>>(p.belt_n, p.d_belt);
         JHTB_CUDA_TRY(cudaGetLastError());
@@ -911,7 +910,7 @@ int launch_ring_tables(const Plan &p, const int *lens, const long long *ctab_off
     ring_table_kernel<<<dim3(n, kRingCols), 128, 0, s>>>(lens, ctab_offs, p.d_ctab);
     JHTB_CUDA_TRY(cudaGetLastError());
     // the lengths are sorted by their P: count[log2 P] of each
-    int rc, o = 0;
+    int o = 0;
 #define JHTB_SPECTRUM(L)                                                                                   \
     if ((rc = launch_spectrum<L>(lens + o, bh_offs + o, count[L], p.d_tw, p.d_bh, s))) return rc; \
     o += count[L];

@@ -126,6 +126,8 @@ def _host_tensor(x) -> torch.Tensor:
 
 def _as_alm(alm) -> torch.Tensor:
     t = _host_tensor(alm)
+    if t.is_cuda and t.dtype == torch.complex128 and t.device.index == torch.cuda.current_device():
+        return t  # what the conversions below return, unasked
     if not t.is_complex():
         t = t.to(torch.float64)
     return t.to(device=_device(), dtype=torch.complex128)
@@ -133,6 +135,8 @@ def _as_alm(alm) -> torch.Tensor:
 
 def _as_map(m) -> torch.Tensor:
     t = _host_tensor(m)
+    if t.is_cuda and t.dtype == torch.float64 and t.device.index == torch.cuda.current_device():
+        return t
     if t.is_complex():
         raise TypeError("maps must be real")
     return t.to(device=_device(), dtype=torch.float64)
