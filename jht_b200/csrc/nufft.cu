@@ -13,8 +13,16 @@
 //   spread (type 1):  grid[ik_a][im_b] += wk_a wm_b v_j for every point (FP64 atomic
 //                     adds: the summation order over points is not fixed).
 //
-// One thread per point; its 2 W weights stay in registers (W is a template parameter).
-// The grid of a typical case (lmax <= 2048: <= 8640^2 cells) is read through L2.
+// Interpolation: eight lanes per point, a lane for columns b and b + 8 of the window.  A window
+// row is then one or two contiguous reads of 128 bytes and the eight lanes share the window
+// weights' exponentials; with a thread per point a warp read 32 scattered cells at a time and the
+// L1 took one after the other.  3 million points of W = 14 on 4320 x 4320 cells: 1201 us with a
+// thread per point, 784 us now; 20000 points on 864 x 810: 33 and 13 us.  (Sixteen lanes per
+// point: 1292 us, 336 warp instructions per point, most of them row addresses and window starts.)
+// What is left is the instructions: about 60 of each weight's exp and sqrt.
+//
+// Direct spread: a lane for each of the 2 W doubles of a window row, so that a row's additions
+// leave as one request of whole sectors (20000 points: 70 us with a thread per point, now 18 us).
 #include <cuda_runtime.h>
 
 #include "jhtb_internal.cuh"
@@ -25,111 +33,215 @@ namespace {
 constexpr int kNuThreads = 256;
 constexpr double kTwoPi = 6.283185307179586476925286766559;
 
-// Window start and weights (and derivative weights d psi / d u) of one coordinate.
-template <int W, bool DERIV>
-__device__ __forceinline__ void window(double coord, int n, double beta, long long &first, double (&w)[W],
-                                       double (&dw)[W]) {
-    const double u = coord * (double)n / kTwoPi;
-    const double f = ceil(u - 0.5 * W);
-    // far outside any sensible range (or NaN) the start saturates; every index is then
-    // still reduced into [0, n) by wrap
+// Window start of one coordinate: u is the position in cells, f the first cell, first f as an
+// integer.  Far outside any sensible range (or NaN) the start saturates; every index is still
+// reduced into [0, n) by wrap.
+template <int W>
+__device__ __forceinline__ void window_start(double coord, int n, double &u, double &f, long long &first) {
+    u = coord * (double)n / kTwoPi;
+    f = ceil(u - 0.5 * W);
     first = (f > -4.0e18 && f < 4.0e18) ? (long long)f : 0;
-    const double inv_half = 2.0 / W;
-#pragma unroll
-    for (int a = 0; a < W; ++a) {
-        const double t = u - (f + a);
-        const double z = t * inv_half;
-        const double z2 = z * z;
-        if (z2 < 1.0) {
-            const double r = sqrt(1.0 - z2);
-            const double v = exp(beta * (r - 1.0));
-            w[a] = v;
-            if (DERIV) dw[a] = -v * beta * z * inv_half / r;
-        } else {
-            w[a] = 0.0;
-            if (DERIV) dw[a] = 0.0;
-        }
+}
+
+// Weight a of the window that starts at f, and its derivative d psi / d u.
+template <int W, bool DERIV>
+__device__ __forceinline__ double window_at(double u, double f, int a, double beta, double &dw) {
+    const double t = u - (f + a);
+    const double z = t * (2.0 / W);
+    const double z2 = z * z;
+    double w = 0.0;
+    dw = 0.0;
+    if (z2 < 1.0) {
+        const double r = sqrt(1.0 - z2);
+        w = exp(beta * (r - 1.0));
+        if (DERIV) dw = -w * beta * z * (2.0 / W) / r;
     }
+    return w;
+}
+template <int W>
+__device__ __forceinline__ double window_at(double u, double f, int a, double beta) {
+    const double t = u - (f + a);
+    const double z = t * (2.0 / W);
+    const double z2 = z * z;
+    return z2 < 1.0 ? exp(beta * (sqrt(1.0 - z2) - 1.0)) : 0.0;
 }
 
 __device__ __forceinline__ int wrap(long long i, int n) {
+    if (i == (int)i) {  // the ordinary case: 32-bit remainder
+        const int r = (int)i % n;
+        return r < 0 ? r + n : r;
+    }
     const long long r = i % n;
     return (int)(r < 0 ? r + n : r);
 }
+// base + a reduced into [0, n), base already there.
+__device__ __forceinline__ unsigned step_wrap(int base, int a, int n) {
+    const unsigned r = (unsigned)base + (unsigned)a;
+    return r < (unsigned)n ? r : r % (unsigned)n;
+}
 
+template <int L>
+__device__ __forceinline__ double2 lane_sum(double2 v) {
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+    }
+    return v;
+}
+
+constexpr int kInterpLanes = 8;                    // lanes of a point
+constexpr int kInterpPts = kNuThreads / kInterpLanes;  // points of a CTA at a time
+constexpr int kWinStride = 18;                     // of a point's row weights: 16-byte reads, points in other banks
+
+// A warp takes `batch` points at a time: a lane per point finds the windows' starts (divisions,
+// remainders), then the points go by four.  Lane b of a point has columns b and b + 8.
 template <int W, bool DERIV>
 __global__ void __launch_bounds__(kNuThreads) interp_kernel(const double2 *__restrict__ grid, int nk, int nm,
                                                             double beta, const double *__restrict__ theta,
-                                                            const double *__restrict__ phi, long long npts,
+                                                            const double *__restrict__ phi, long long npts, int batch,
                                                             double2 *__restrict__ out, double2 *__restrict__ dth,
                                                             double2 *__restrict__ dph) {
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < npts;
-         j += (long long)gridDim.x * blockDim.x) {
-        long long k0, m0;
-        double wk[W], wm[W], dk[W], dm[W];
-        window<W, DERIV>(theta[j], nk, beta, k0, wk, dk);
-        window<W, DERIV>(phi[j], nm, beta, m0, wm, dm);
-        int mi[W];
+    constexpr int L = kInterpLanes, PER = 32 / L, WARPS = kNuThreads / 32, NC = (W + L - 1) / L, ND = DERIV ? 2 : 1;
+    static_assert(W % 2 == 0 && W <= 16, "rows in pairs, two columns a lane");
+    __shared__ __align__(16) double sk[kInterpPts][ND][kWinStride];  // row weights (and derivatives) of each point
+    __shared__ double2 su[WARPS][32], sf[WARPS][32];                 // (theta, phi) u and f of the batch
+    __shared__ int2 sbase[WARPS][32];
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int b = lane % L, sub = lane / L, slot = threadIdx.x / L;
+    // A CTA takes consecutive points, which the caller may have grouped by tiles of the grid: their
+    // windows overlap in its L1.
+    const long long batches = (npts + batch - 1) / batch;
+    const long long b0 = batches * blockIdx.x / gridDim.x, b1 = batches * (blockIdx.x + 1) / gridDim.x;
+    for (long long bi = b0 + warp; bi < b1; bi += WARPS) {
+        const long long first = bi * batch;
+        const int count = (int)min((long long)batch, npts - first);
+        __syncwarp();  // the batch before is done
+        bool inside = true;  // no row of this lane's point wraps
+        if (lane < count) {
+            double2 u, f;
+            long long k0, m0;
+            window_start<W>(theta[first + lane], nk, u.x, f.x, k0);
+            window_start<W>(phi[first + lane], nm, u.y, f.y, m0);
+            const int2 base = make_int2(wrap(k0, nk), wrap(m0, nm));
+            su[warp][lane] = u;
+            sf[warp][lane] = f;
+            sbase[warp][lane] = base;
+            inside = base.x <= nk - W;
+        }
+        inside = __all_sync(0xffffffffu, inside);
+        for (int i0 = 0; i0 < count; i0 += PER) {
+            const int i = min(i0 + sub, count - 1);  // the last points' partners repeat the last point
+            const double2 u = su[warp][i], f0 = sf[warp][i];
+            const int2 base = sbase[warp][i];
+            double wm[NC], dm[NC];
+            __syncwarp();  // the points before are read
 #pragma unroll
-        for (int b = 0; b < W; ++b) mi[b] = wrap(m0 + b, nm);
-        double2 f = make_double2(0.0, 0.0), gk = make_double2(0.0, 0.0), gm = make_double2(0.0, 0.0);
-#pragma unroll 2
-        for (int a = 0; a < W; ++a) {
-            const double2 *row = grid + (size_t)wrap(k0 + a, nk) * nm;
-            double2 s = make_double2(0.0, 0.0), sd = make_double2(0.0, 0.0);
+            for (int c = 0; c < NC; ++c) {
+                double dk;
+                const double wk = window_at<W, DERIV>(u.x, f0.x, b + L * c, beta, dk);
+                sk[slot][0][b + L * c] = wk;
+                if (DERIV) sk[slot][ND - 1][b + L * c] = dk;
+                wm[c] = window_at<W, DERIV>(u.y, f0.y, b + L * c, beta, dm[c]);
+            }
+            __syncwarp();
+            double2 s[NC], sd[NC];
+            const double2 *col[NC];
 #pragma unroll
-            for (int b = 0; b < W; ++b) {
-                const double2 g = __ldg(&row[mi[b]]);
-                s.x = fma(wm[b], g.x, s.x);
-                s.y = fma(wm[b], g.y, s.y);
+            for (int c = 0; c < NC; ++c) {
+                s[c] = sd[c] = make_double2(0.0, 0.0);
+                col[c] = grid + step_wrap(base.y, b + L * c, nm);
+            }
+            auto rows = [&](auto row_of) {
+#pragma unroll
+                for (int a = 0; a < W; a += 2) {
+                    const double2 wk = *reinterpret_cast<const double2 *>(&sk[slot][0][a]);
+                    double2 wd;
+                    if (DERIV) wd = *reinterpret_cast<const double2 *>(&sk[slot][ND - 1][a]);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const size_t r = row_of(a + h);
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) {
+                            if (b + L * c >= W) continue;
+                            const double2 g = __ldg(col[c] + r);
+                            const double w = h ? wk.y : wk.x;
+                            s[c].x = fma(w, g.x, s[c].x);
+                            s[c].y = fma(w, g.y, s[c].y);
+                            if (DERIV) {
+                                const double d = h ? wd.y : wd.x;
+                                sd[c].x = fma(d, g.x, sd[c].x);
+                                sd[c].y = fma(d, g.y, sd[c].y);
+                            }
+                        }
+                    }
+                }
+            };
+            if (inside) {
+                const size_t r0 = (size_t)base.x * nm;
+                rows([&](int a) { return r0 + (size_t)a * nm; });
+            } else {
+                rows([&](int a) { return (size_t)step_wrap(base.x, a, nk) * nm; });
+            }
+            // columns past the window hold zeros, whatever their weight
+            double2 f = make_double2(0.0, 0.0), gk = f, gm = f;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                if (b + L * c >= W) continue;
+                f = make_double2(fma(wm[c], s[c].x, f.x), fma(wm[c], s[c].y, f.y));
                 if (DERIV) {
-                    sd.x = fma(dm[b], g.x, sd.x);
-                    sd.y = fma(dm[b], g.y, sd.y);
+                    gk = make_double2(fma(wm[c], sd[c].x, gk.x), fma(wm[c], sd[c].y, gk.y));
+                    gm = make_double2(fma(dm[c], s[c].x, gm.x), fma(dm[c], s[c].y, gm.y));
                 }
             }
-            f.x = fma(wk[a], s.x, f.x);
-            f.y = fma(wk[a], s.y, f.y);
+            f = lane_sum<L>(f);
             if (DERIV) {
-                gk.x = fma(dk[a], s.x, gk.x);
-                gk.y = fma(dk[a], s.y, gk.y);
-                gm.x = fma(wk[a], sd.x, gm.x);
-                gm.y = fma(wk[a], sd.y, gm.y);
+                gk = lane_sum<L>(gk);
+                gm = lane_sum<L>(gm);
             }
-        }
-        out[j] = f;
-        if (DERIV) {
-            // d/dcoord = (n / 2 pi) d/du
-            const double ck = (double)nk / kTwoPi, cm = (double)nm / kTwoPi;
-            dth[j] = make_double2(ck * gk.x, ck * gk.y);
-            dph[j] = make_double2(cm * gm.x, cm * gm.y);
+            if (b == 0 && i0 + sub < count) {
+                const long long j = first + i;
+                out[j] = f;
+                if (DERIV) {
+                    // d/dcoord = (n / 2 pi) d/du
+                    const double ck = (double)nk / kTwoPi, cm = (double)nm / kTwoPi;
+                    dth[j] = make_double2(ck * gk.x, ck * gk.y);
+                    dph[j] = make_double2(cm * gm.x, cm * gm.y);
+                }
+            }
         }
     }
 }
+
+template <int W>
+constexpr int kSpreadLanes = W <= 8 ? 16 : 32;  // lanes of a point: 2 W doubles of a row
 
 template <int W>
 __global__ void __launch_bounds__(kNuThreads) spread_kernel(const double2 *__restrict__ vals,
                                                             const double *__restrict__ theta,
                                                             const double *__restrict__ phi, long long npts, int nk,
                                                             int nm, double beta, double2 *__restrict__ grid) {
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < npts;
-         j += (long long)gridDim.x * blockDim.x) {
+    constexpr int L = kSpreadLanes<W>, H = L / 2, PER = 32 / L;
+    const int l = threadIdx.x % L, slot = threadIdx.x / L;
+    const long long step = (long long)gridDim.x * (kNuThreads / L);
+    for (long long j0 = (long long)blockIdx.x * (kNuThreads / L) + slot / PER * PER; j0 < npts; j0 += step) {
+        const long long jj = j0 + slot % PER, j = jj < npts ? jj : npts - 1;
+        double uk, fk, um, fm;
         long long k0, m0;
-        double wk[W], wm[W], unused[W];
-        window<W, false>(theta[j], nk, beta, k0, wk, unused);
-        window<W, false>(phi[j], nm, beta, m0, wm, unused);
-        const double2 v = vals[j];
-        int mi[W];
-#pragma unroll
-        for (int b = 0; b < W; ++b) mi[b] = wrap(m0 + b, nm);
-#pragma unroll 1
+        window_start<W>(theta[j], nk, uk, fk, k0);
+        window_start<W>(phi[j], nm, um, fm, m0);
+        // row weights in the lower lanes, column weights in the upper ones
+        const double w = l < H ? window_at<W>(uk, fk, l, beta) : window_at<W>(um, fm, l - H, beta);
+        const double wm = __shfl_sync(0xffffffffu, w, H + l / 2, L);
+        const double2 v2 = vals[j];
+        const double v = l & 1 ? v2.y : v2.x;
+        const bool on = l < 2 * W && jj < npts;
+        const int kb = wrap(k0, nk);
+        double *col = reinterpret_cast<double *>(grid + wrap(m0 + l / 2, nm)) + (l & 1);
+#pragma unroll 2
         for (int a = 0; a < W; ++a) {
-            double *row = reinterpret_cast<double *>(grid + (size_t)wrap(k0 + a, nk) * nm);
-            const double vx = wk[a] * v.x, vy = wk[a] * v.y;
-#pragma unroll
-            for (int b = 0; b < W; ++b) {
-                atomicAdd(row + 2 * mi[b], wm[b] * vx);
-                atomicAdd(row + 2 * mi[b] + 1, wm[b] * vy);
-            }
+            const double wk = __shfl_sync(0xffffffffu, w, a, L);
+            if (on) atomicAdd(col + (size_t)step_wrap(kb, a, nk) * 2 * nm, wm * (wk * v));
         }
     }
 }
@@ -154,15 +266,6 @@ constexpr int kSA = kBlkCells + 4, kSB = 2 * kBlkCells + 4;  // strides = 4 mod 
 
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
     asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
-}
-
-// Weight a of the window of one coordinate (the value window() gives at index a).
-template <int W>
-__device__ __forceinline__ double window_at(double u, double f, int a, double beta) {
-    const double t = u - (f + a);
-    const double z = t * (2.0 / W);
-    const double z2 = z * z;
-    return z2 < 1.0 ? exp(beta * (sqrt(1.0 - z2) - 1.0)) : 0.0;
 }
 
 template <int W>
@@ -255,12 +358,15 @@ __global__ void __launch_bounds__(kSpreadThreads, 3) spread_tiles_kernel(
     }
 }
 
-int grid_blocks(long long npts) {
+int sm_count() {
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const long long need = (npts + kNuThreads - 1) / kNuThreads;
-    return (int)std::max<long long>(1, std::min<long long>(need, (long long)nsm * 16));
+    return nsm;
+}
+// CTAs for `groups` units of work of a CTA each
+int grid_blocks(long long groups) {
+    return (int)std::max<long long>(1, std::min<long long>(groups, 16LL * sm_count()));
 }
 
 int check_args(int nk, int nm, int W, long long npts, const char *who) {
@@ -274,16 +380,21 @@ int check_args(int nk, int nm, int W, long long npts, const char *who) {
 template <int W>
 void launch_interp(const double2 *g, int nk, int nm, double beta, const double *th, const double *ph, long long n,
                    double2 *out, double2 *dth, double2 *dph, cudaStream_t s) {
+    // points of a warp's batch: up to a lane each, while every SM has 32 warps' worth
+    constexpr int per = 32 / kInterpLanes, warps = kNuThreads / 32;
+    const int batch = (int)std::max<long long>(per, std::min<long long>(32, n / (32 * sm_count()) / per * per));
+    const int blocks = grid_blocks((n + (long long)batch * warps - 1) / ((long long)batch * warps));
     if (dth && dph)
-        interp_kernel<W, true><<<grid_blocks(n), kNuThreads, 0, s>>>(g, nk, nm, beta, th, ph, n, out, dth, dph);
+        interp_kernel<W, true><<<blocks, kNuThreads, 0, s>>>(g, nk, nm, beta, th, ph, n, batch, out, dth, dph);
     else
-        interp_kernel<W, false><<<grid_blocks(n), kNuThreads, 0, s>>>(g, nk, nm, beta, th, ph, n, out, nullptr, nullptr);
+        interp_kernel<W, false><<<blocks, kNuThreads, 0, s>>>(g, nk, nm, beta, th, ph, n, batch, out, nullptr, nullptr);
 }
 
 template <int W>
 void launch_spread(const double2 *v, const double *th, const double *ph, long long n, int nk, int nm, double beta,
                    double2 *g, cudaStream_t s) {
-    spread_kernel<W><<<grid_blocks(n), kNuThreads, 0, s>>>(v, th, ph, n, nk, nm, beta, g);
+    constexpr int per = kNuThreads / kSpreadLanes<W>;
+    spread_kernel<W><<<grid_blocks((n + per - 1) / per), kNuThreads, 0, s>>>(v, th, ph, n, nk, nm, beta, g);
 }
 
 template <int W>
