@@ -27,7 +27,8 @@
  *   jhtb_legendre_adjoint   offgrid.py:163-168 (adjoint_contract at those rings)
  *   jhtb_nufft_interp       _nufft.py:164-178 (nufft2d2's window sums)
  *   jhtb_nufft_spread       _nufft.py:181-188 (nufft2d1's scatter-add)
- *   jhtb_nufft_spread_tiles _nufft.py:181-188 (the same, for points grouped by grid tile)
+ *   jhtb_nufft_spread_tiles _nufft.py:181-188 (the same, for points grouped by grid tile;
+ *                           jhtb_nufft_group_points groups them)
  */
 #ifndef JHTB_H
 #define JHTB_H
@@ -189,6 +190,20 @@ int jhtb_nufft_spread_tiles(const void *vals, const double *theta, const double 
                             int64_t nseg, const int64_t *seg_start, const int *seg_count,
                             const int64_t *seg_tile, int tiles_m, int nk, int nm, int W, double beta,
                             void *grid, void *stream);
+/* Group points by 32 x 32-cell tiles of the grid (tiles_k >= nk / 32 + 1 rows of tiles_m >=
+ * nm / 32 + 1 tiles, at most 2^20 of them): point order[p] of the input goes to place p of theta_s,
+ * phi_s and vals_s (complex; vals may be NULL).  Segments of at most 1024 points of one tile, in
+ * the form jhtb_nufft_spread_tiles takes: nseg = tiles_k tiles_m + npts / 1024 of them, those not
+ * needed with count 0.  work: 16 tiles_k tiles_m + 8192 + 2 npts ints, 16-byte aligned.  No
+ * synchronisation; npts < 2^31 - 1024.  The order of a tile's points is not fixed. */
+int jhtb_nufft_group_points(const double *theta, const double *phi, const void *vals, int64_t npts,
+                            int nk, int nm, int tiles_k, int tiles_m, int *work, int *order,
+                            double *theta_s, double *phi_s, void *vals_s, int *seg_count,
+                            int64_t *seg_start, int64_t *seg_tile, void *stream);
+/* jhtb_nufft_interp of grouped points: the value at place p goes to out[order[p]] (order NULL: p). */
+int jhtb_nufft_interp_grouped(const void *grid, int nk, int nm, int W, double beta, const double *theta,
+                              const double *phi, const int *order, int64_t npts, void *out,
+                              void *dtheta, void *dphi, void *stream);
 
 /* ---- coefficient layouts (masked.py:117-175, healpix.py:58-74) ----
  * One launch each for what jht writes as gathers and concatenations.  alm: device

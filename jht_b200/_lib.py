@@ -57,6 +57,8 @@ EXPORTS = (
     "jhtb_nufft_spread_tiles",
     "jhtb_debug_bounds",
     "jhtb_fft_c2c",
+    "jhtb_nufft_group_points",
+    "jhtb_nufft_interp_grouped",
     "jhtb_torus_grid",
     "jhtb_torus_grid_adjoint",
     "jhtb_real_to_alm",
@@ -135,6 +137,8 @@ def load_library(path: str | os.PathLike | None = None):
             "jhtb_synthesis_cotangent": (i32, [i32, i32, i32, vp, vp]),
             "jhtb_fft_c2c": (i32, [vp, vp, i32, i64, i64, i64, i64, i64, i64, i64, i64, i32, ctypes.c_double, i64,
                                    vp, vp]),
+            "jhtb_nufft_group_points": (i32, [vp, vp, vp, i64, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
+            "jhtb_nufft_interp_grouped": (i32, [vp, i32, i32, i32, ctypes.c_double, vp, vp, vp, i64, vp, vp, vp, vp]),
             "jhtb_torus_grid": (i32, [vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp]),
             "jhtb_torus_grid_adjoint": (i32, [vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp]),
         }

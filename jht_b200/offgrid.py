@@ -96,7 +96,7 @@ class _Geometry:
         self.Nm = 2 * lmax + 1
         self.nk, self.nm = _fft_size(sigma * self.nd), _fft_size(sigma * self.Nm)
         self.beta = float(np.pi * self.W * (1.0 - 0.5 / sigma))
-        self.tiles_m = self.nm // _TILE + 2
+        self.tiles_k, self.tiles_m = self.nk // _TILE + 2, self.nm // _TILE + 2
         dev = torch.device("cuda", device)
         ck = _kernel_ft(self.nd, self.nk, self.W, self.beta)
         cm = _kernel_ft(self.Nm, self.nm, self.W, self.beta)
@@ -163,6 +163,33 @@ def _segments(sorted_keys: torch.Tensor):
     return seg_start.contiguous(), seg_count.contiguous(), seg_tile.contiguous()
 
 
+_GROUP_MAX_TILES = 1 << 20  # of jhtb_nufft_group_points: grids of 32768 x 32768 cells
+
+
+class _Grouped:
+    """Point sets of _SORT_MIN_POINTS and more grouped by tiles in one library call (a counting
+    sort): the sorted coordinates (and values), the input place of each, and the spread's segments."""
+
+    def __init__(self, g: "_Geometry", theta: torch.Tensor, phi: torch.Tensor, vals: torch.Tensor | None = None):
+        n, dev, tiles = theta.numel(), theta.device, g.tiles_k * g.tiles_m
+        self.theta, self.phi = torch.empty((2, n), dtype=torch.float64, device=dev)
+        self.vals = None if vals is None else torch.empty_like(vals)
+        self.nseg = tiles + n // _SEG_POINTS
+        self.seg_start, self.seg_tile = torch.empty((2, self.nseg), dtype=torch.int64, device=dev)
+        self.seg_count = torch.empty(self.nseg, dtype=torch.int32, device=dev)
+        self.order = torch.empty(n, dtype=torch.int32, device=dev)
+        work = torch.empty(16 * tiles + 8192 + 2 * n, dtype=torch.int32, device=dev)
+        _lib.check(g.plan.lib.jhtb_nufft_group_points(
+            theta.data_ptr(), phi.data_ptr(), None if vals is None else vals.data_ptr(), n, g.nk, g.nm, g.tiles_k,
+            g.tiles_m, work.data_ptr(), self.order.data_ptr(), self.theta.data_ptr(), self.phi.data_ptr(),
+            None if vals is None else self.vals.data_ptr(), self.seg_count.data_ptr(), self.seg_start.data_ptr(),
+            self.seg_tile.data_ptr(), _stream()), "jhtb_nufft_group_points")
+
+    @staticmethod
+    def takes(g: "_Geometry", n: int) -> bool:
+        return _SORT_MIN_POINTS <= n < 2**31 - 1024 and g.tiles_k * g.tiles_m <= _GROUP_MAX_TILES
+
+
 # ---------------------------------------------------------------------------------------
 # forward: alm -> oversampled grid -> points
 # ---------------------------------------------------------------------------------------
@@ -207,30 +234,25 @@ def _torus_grid(g: _Geometry, F: torch.Tensor) -> torch.Tensor:
 
 
 def _interp(g: _Geometry, grid: torch.Tensor, theta: torch.Tensor, phi: torch.Tensor, deriv: bool):
+    if _Grouped.takes(g, theta.numel()):
+        p = _Grouped(g, theta, phi)
+        return _interp_raw(g, grid, p.theta, p.phi, deriv, p.order)
     po = _point_order(g, theta, phi)
     if po is not None:
-        order = po[0]
-        out = _interp_raw(g, grid, theta[order], phi[order], deriv)
-        res = []
-        for t in out:
-            if t is None:
-                res.append(None)
-                continue
-            r = torch.empty_like(t)
-            r[order] = t
-            res.append(r)
-        return tuple(res)
-    return _interp_raw(g, grid, theta, phi, deriv)
+        order = po[0].to(torch.int32)
+        return _interp_raw(g, grid, theta[po[0]], phi[po[0]], deriv, order)
+    return _interp_raw(g, grid, theta, phi, deriv, None)
 
 
-def _interp_raw(g: _Geometry, grid: torch.Tensor, theta: torch.Tensor, phi: torch.Tensor, deriv: bool):
+def _interp_raw(g: _Geometry, grid: torch.Tensor, theta: torch.Tensor, phi: torch.Tensor, deriv: bool, order):
     n = theta.numel()
     out = torch.empty(n, dtype=torch.complex128, device=theta.device)
     dth = torch.empty_like(out) if deriv else None
     dph = torch.empty_like(out) if deriv else None
-    st = g.plan.lib.jhtb_nufft_interp(
-        grid.contiguous().data_ptr(), g.nk, g.nm, g.W, ctypes.c_double(g.beta), theta.data_ptr(), phi.data_ptr(), n,
-        out.data_ptr(), dth.data_ptr() if deriv else None, dph.data_ptr() if deriv else None, _stream())
+    st = g.plan.lib.jhtb_nufft_interp_grouped(
+        grid.contiguous().data_ptr(), g.nk, g.nm, g.W, ctypes.c_double(g.beta), theta.data_ptr(), phi.data_ptr(),
+        None if order is None else order.data_ptr(), n, out.data_ptr(), dth.data_ptr() if deriv else None,
+        dph.data_ptr() if deriv else None, _stream())
     _lib.check(st, "jhtb_nufft_interp")
     return out, dth, dph
 
@@ -277,15 +299,22 @@ def _adjoint(g: _Geometry, fc: torch.Tensor, theta: torch.Tensor, phi: torch.Ten
     """Complex point values -> (ncomp, K) alm, the transpose of _forward's value path
     divided by the metric (offgrid.py:223-243)."""
     grid = torch.zeros((g.nk, g.nm), dtype=torch.complex128, device=fc.device)
-    po = _point_order(g, theta, phi)
-    if po is not None:
-        order, keys = po
-        fc, theta, phi = fc[order].contiguous(), theta[order].contiguous(), phi[order].contiguous()
-        seg_start, seg_count, seg_tile = _segments(keys)
+    segments = None
+    if _Grouped.takes(g, theta.numel()):
+        p = _Grouped(g, theta, phi, fc.contiguous())
+        fc, theta, phi, segments = p.vals, p.theta, p.phi, (p.seg_start, p.seg_count, p.seg_tile)
+    else:
+        po = _point_order(g, theta, phi)
+        if po is not None:
+            order, keys = po
+            fc, theta, phi = fc[order].contiguous(), theta[order].contiguous(), phi[order].contiguous()
+            segments = _segments(keys)
+    if segments is not None:
+        start, count, tile = segments
         st = g.plan.lib.jhtb_nufft_spread_tiles(
-            fc.data_ptr(), theta.data_ptr(), phi.data_ptr(), theta.numel(), seg_start.numel(), seg_start.data_ptr(),
-            seg_count.data_ptr(), seg_tile.data_ptr(), g.tiles_m, g.nk, g.nm, g.W, ctypes.c_double(g.beta),
-            grid.data_ptr(), _stream())
+            fc.data_ptr(), theta.data_ptr(), phi.data_ptr(), theta.numel(), start.numel(), start.data_ptr(),
+            count.data_ptr(), tile.data_ptr(), g.tiles_m, g.nk, g.nm, g.W, ctypes.c_double(g.beta), grid.data_ptr(),
+            _stream())
         _lib.check(st, "jhtb_nufft_spread_tiles")
     else:
         st = g.plan.lib.jhtb_nufft_spread(fc.contiguous().data_ptr(), theta.data_ptr(), phi.data_ptr(), theta.numel(),
