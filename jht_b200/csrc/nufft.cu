@@ -256,8 +256,10 @@ __global__ void __launch_bounds__(kNuThreads) spread_kernel(const double2 *__res
 // pairs), so it runs on the FP64 matrix unit: 9 of the block's 6 x 12 products of 8 x 8 per warp,
 // four points per step, accumulators in registers.  Products of blocks that none of the four points
 // touches are left out: points grouped by the part of the tile their window starts in need about a
-// third of them (3 million points of W = 14: all products 1417 us, those touched 1271 us; the window
-// weights, their staging and the additions to the grid are now the larger part).  Adding the windows
+// third of them (3 million points of W = 14: all products 1417 us, those touched 1271 us, with the
+// next round's points fetched a round ahead 1210 us; the window weights, their staging and the
+// additions to the grid are now the larger part, and three CTAs an SM hide only some of their
+// latency: two took 1561 us, four, with spills, 1240 us).  Adding the windows
 // into shared memory took 392 shared FP64 atomics per point (compare-and-swap loops).  A point whose
 // window leaves the block (a coordinate outside the tile its key named) is added straight to the grid.
 constexpr int kTile = 32;
@@ -297,6 +299,18 @@ __global__ void __launch_bounds__(kSpreadThreads, 3) spread_tiles_kernel(
 #pragma unroll
         for (int c = 0; c < 3; ++c) acc[r][c][0] = acc[r][c][1] = 0.0;
     const int pt = threadIdx.x >> 3, sub = threadIdx.x & 7;  // eight threads stage a point
+    // this thread's point of the next round, fetched while one runs
+    double th = 0.0, ph = 0.0;
+    double2 v = make_double2(0.0, 0.0);
+    auto fetch = [&](int q0) {
+        const long long j = p0 + q0 + pt;
+        if (q0 + pt < cnt && j >= 0 && j < npts) {
+            th = theta[j];
+            ph = phi[j];
+            v = vals[j];
+        }
+    };
+    fetch(0);
     for (int q0 = 0; q0 < cnt; q0 += kSpreadPts) {
         __syncthreads();  // the round before is read
         for (int i = threadIdx.x; i < kSpreadPts * (kSA + kSB) / 2; i += kSpreadThreads) {
@@ -308,11 +322,10 @@ __global__ void __launch_bounds__(kSpreadThreads, 3) spread_tiles_kernel(
         const long long j = p0 + q0 + pt;
         unsigned mask = 0;
         if (q0 + pt < cnt && j >= 0 && j < npts) {
-            const double uk = theta[j] * (double)nk / kTwoPi, um = phi[j] * (double)nm / kTwoPi;
+            const double uk = th * (double)nk / kTwoPi, um = ph * (double)nm / kTwoPi;
             const double fk = ceil(uk - 0.5 * W), fm = ceil(um - 0.5 * W);
             const long long k0 = (fk > -4.0e18 && fk < 4.0e18) ? (long long)fk : 0;
             const long long m0 = (fm > -4.0e18 && fm < 4.0e18) ? (long long)fm : 0;
-            const double2 v = vals[j];
             const long long bk = k0 - k_org, bm = m0 - m_org;
             // an infinite value would reach the block's other cells as 0 x inf
             if (bk >= 0 && bk + W <= B && bm >= 0 && bm + W <= B && isfinite(v.x) && isfinite(v.y)) {
@@ -335,6 +348,7 @@ __global__ void __launch_bounds__(kSpreadThreads, 3) spread_tiles_kernel(
                 }
             }
         }
+        fetch(q0 + kSpreadPts);
         mask = __reduce_or_sync(0xffffffffu, mask);  // a warp stages the four points of a step
         if (lane == 0) smask[warp] = mask;
         __syncthreads();
