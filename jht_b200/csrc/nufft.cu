@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(kNuThreads) interp_kernel(const double2 *__res
             inside = base.x <= nk - W;
         }
         inside = __all_sync(0xffffffffu, inside);
+        __syncwarp();  // the batch's starts are written: a vote alone orders no memory
         for (int i0 = 0; i0 < count; i0 += PER) {
             const int i = min(i0 + sub, count - 1);  // the last points' partners repeat the last point
             const double2 u = su[warp][i], f0 = sf[warp][i];
