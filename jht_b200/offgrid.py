@@ -164,6 +164,8 @@ def _segments(sorted_keys: torch.Tensor):
 
 
 _GROUP_MAX_TILES = 1 << 20  # of jhtb_nufft_group_points: grids of 32768 x 32768 cells
+_ORDER_MAX = 2**31 - 1024  # points whose order fits 32 bits, the limit of jhtb_nufft_group_points
+_ORDER_PART = 1 << 28  # points of a part where there are more: 4 GB per complex output
 
 
 class _Grouped:
@@ -187,7 +189,7 @@ class _Grouped:
 
     @staticmethod
     def takes(g: "_Geometry", n: int) -> bool:
-        return _SORT_MIN_POINTS <= n < 2**31 - 1024 and g.tiles_k * g.tiles_m <= _GROUP_MAX_TILES
+        return _SORT_MIN_POINTS <= n < _ORDER_MAX and g.tiles_k * g.tiles_m <= _GROUP_MAX_TILES
 
 
 # ---------------------------------------------------------------------------------------
@@ -234,6 +236,20 @@ def _torus_grid(g: _Geometry, F: torch.Tensor) -> torch.Tensor:
 
 
 def _interp(g: _Geometry, grid: torch.Tensor, theta: torch.Tensor, phi: torch.Tensor, deriv: bool):
+    n = theta.numel()
+    if n < _ORDER_MAX:
+        return _interp_part(g, grid, theta, phi, deriv)
+    # the library's point order is 32 bits wide: longer sets go part by part
+    outs = [torch.empty(n, dtype=torch.complex128, device=theta.device) if k == 0 or deriv else None for k in range(3)]
+    for p0 in range(0, n, _ORDER_PART):
+        p1 = min(p0 + _ORDER_PART, n)
+        for out, part in zip(outs, _interp_part(g, grid, theta[p0:p1], phi[p0:p1], deriv)):
+            if out is not None:
+                out[p0:p1] = part
+    return tuple(outs)
+
+
+def _interp_part(g: _Geometry, grid: torch.Tensor, theta: torch.Tensor, phi: torch.Tensor, deriv: bool):
     if _Grouped.takes(g, theta.numel()):
         p = _Grouped(g, theta, phi)
         return _interp_raw(g, grid, p.theta, p.phi, deriv, p.order)
