@@ -48,6 +48,7 @@ def _weighted(maps: torch.Tensor, synth: torch.Tensor | None, nside: int, lmax: 
               use_weights: bool) -> torch.Tensor:
     """W (maps - synth) through the C ABI (no autograd); shapes (B, ncomp, npix)."""
     plan = _lib.get_plan(nside, lmax, spin, "fp64", maps.shape[0])
+    maps = _lib.dense(maps)
     out = torch.empty_like(maps)
     rw = _ring_w_device(nside, maps.device.index).data_ptr() if use_weights else None
     st = plan.lib.jhtb_weighted_residual(

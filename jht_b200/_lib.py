@@ -388,6 +388,13 @@ def clear_plans() -> None:
         _plans.clear()
 
 
+def dense(t):
+    """``t`` contiguous and with torch's lazy conjugation and negation carried out: the values
+    that a kernel finds behind ``data_ptr()`` (contiguous() alone keeps a lazy bit)."""
+    t = t.contiguous()
+    return t.resolve_conj().resolve_neg() if t.is_conj() or t.is_neg() else t
+
+
 def stream_ptr():
     import torch
 

@@ -165,7 +165,7 @@ class ShardedTransform:
 
     def _batched(self, x, last: int):
         t = x if x.dim() == 3 else x.reshape(1, self.ncomp, last)
-        return t.contiguous()
+        return _lib.dense(t)
 
     def synthesis(self, alm: torch.Tensor, gather: bool = True) -> torch.Tensor:
         """Map (B, ncomp, npix) of this rank's rings (zeros elsewhere), or with `gather` the whole

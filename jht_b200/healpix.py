@@ -149,7 +149,7 @@ def _synth_raw(alm: torch.Tensor, nside: int, lmax: int, spin: int, precision: s
     """alm (B, ncomp, K) complex128 contiguous -> maps (B, ncomp, npix) float64."""
     B = alm.shape[0]
     plan = _lib.get_plan(nside, lmax, spin, precision, B)
-    alm = alm.contiguous()
+    alm = _lib.dense(alm)
     out = torch.empty((B, plan.ncomp, plan.npix), dtype=torch.float64, device=alm.device)
     if B:
         st = plan.lib.jhtb_synthesis(plan.handle, alm.data_ptr(), out.data_ptr(), B, _lib.stream_ptr())
@@ -161,7 +161,7 @@ def _adjoint_raw(maps: torch.Tensor, nside: int, lmax: int, spin: int, precision
     """maps (B, ncomp, npix) float64 contiguous -> alm (B, ncomp, K) complex128."""
     B = maps.shape[0]
     plan = _lib.get_plan(nside, lmax, spin, precision, B)
-    maps = maps.contiguous()
+    maps = _lib.dense(maps)
     out = torch.empty((B, plan.ncomp, plan.K), dtype=torch.complex128, device=maps.device)
     if B:
         st = plan.lib.jhtb_adjoint_synthesis(plan.handle, maps.data_ptr(), out.data_ptr(), B, _lib.stream_ptr())

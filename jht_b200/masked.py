@@ -105,7 +105,7 @@ def _one_launch(t: torch.Tensor, dtype: torch.dtype, shape: tuple) -> bool:
 def _real_batch(a: torch.Tensor, lmax: int, spin: int) -> torch.Tensor:
     """(B, ncomp, K) complex -> (B, n_dof) real."""
     if _one_launch(a, torch.complex128, (1 if spin == 0 else 2, alm_size(lmax))):
-        a = a.contiguous()
+        a = _lib.dense(a)
         x = torch.empty((a.shape[0], n_dof(lmax, spin)), dtype=torch.float64, device=a.device)
         if x.numel():
             _lib.check(_lib.load_library().jhtb_alm_to_real(lmax, spin, a.shape[0], a.data_ptr(), x.data_ptr(),
@@ -122,7 +122,7 @@ def _real_batch(a: torch.Tensor, lmax: int, spin: int) -> torch.Tensor:
 def _alm_batch(x: torch.Tensor, lmax: int, spin: int) -> torch.Tensor:
     """(B, n_dof) real -> (B, ncomp, K) complex."""
     if _one_launch(x, torch.float64, (n_dof(lmax, spin),)):
-        x = x.contiguous()
+        x = _lib.dense(x)
         a = torch.empty((x.shape[0], 1 if spin == 0 else 2, alm_size(lmax)), dtype=torch.complex128, device=x.device)
         if a.numel():
             _lib.check(_lib.load_library().jhtb_real_to_alm(lmax, spin, x.shape[0], x.data_ptr(), a.data_ptr(),

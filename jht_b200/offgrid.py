@@ -198,7 +198,7 @@ class _Grouped:
 def _ring_coeffs(g: _Geometry, alm: torch.Tensor) -> torch.Tensor:
     """(ncomp, K) alm -> (ncomp, ns, lmax+1) ring coefficients (+spin, -spin channels)."""
     out = torch.empty((g.ncomp, g.ns, g.lmax + 1), dtype=torch.complex128, device=alm.device)
-    st = g.plan.lib.jhtb_legendre_synthesis(g.plan.handle, alm.contiguous().data_ptr(), out.data_ptr(), 1, _stream())
+    st = g.plan.lib.jhtb_legendre_synthesis(g.plan.handle, _lib.dense(alm).data_ptr(), out.data_ptr(), 1, _stream())
     _lib.check(st, "jhtb_legendre_synthesis")
     return out
 
@@ -436,7 +436,7 @@ def synthesis_general(alm, loc, *, spin: int = 0, lmax: int, epsilon: float = 1e
     a = _as_alm(a)
     t = t.to(device=a.device, dtype=torch.float64)
     g = _geometry(int(lmax), int(spin), float(epsilon), a.device.index)
-    theta, phi = t[:, 0].contiguous(), t[:, 1].contiguous()
+    theta, phi = _lib.dense(t[:, 0]), _lib.dense(t[:, 1])
     return _SynthesisGeneral.apply(a.reshape(g.ncomp, -1), theta, phi, g)
 
 
@@ -458,6 +458,6 @@ def adjoint_synthesis_general(field, loc, *, spin: int = 0, lmax: int, epsilon: 
     t = t.to(device=_device(), dtype=torch.float64)
     f = f.to(device=t.device, dtype=torch.float64).contiguous()
     g = _geometry(int(lmax), int(spin), float(epsilon), t.device.index)
-    theta, phi = t[:, 0].contiguous(), t[:, 1].contiguous()
+    theta, phi = _lib.dense(t[:, 0]), _lib.dense(t[:, 1])
     out = _AdjointGeneral.apply(f, theta, phi, g)
     return out.reshape(-1) if spin == 0 else out
