@@ -87,7 +87,7 @@ def fft(x: torch.Tensor, dim: int, sign: int, scale: float = 1.0) -> torch.Tenso
         raise ValueError("fft: expects a 2-D complex128 CUDA tensor")
     if dim not in (0, 1) or sign not in (1, -1):
         raise ValueError("fft: dim must be 0 or 1 and sign +1 or -1")
-    x = _lib.dense(x)
+    x = x.contiguous()
     rows, cols = x.shape
     out = torch.empty_like(x)
     n = x.shape[dim]

@@ -17,7 +17,7 @@ if not torch.cuda.is_available():  # pragma: no cover - CPU hosts
     pytest.skip("no CUDA device", allow_module_level=True)
 
 import jht_b200 as jhtb  # noqa: E402
-from jht_b200 import _fft, distributed, masked  # noqa: E402
+from jht_b200 import distributed, masked  # noqa: E402
 
 NSIDE, LMAX = 8, 12
 NPIX, K = 12 * NSIDE**2, jhtb.alm_size(LMAX)
@@ -100,7 +100,3 @@ def test_offgrid(spin, gen):
     for got, ref in zip(both(a, f, loc), both(_plain(a), _plain(f), _plain(loc))):
         assert torch.equal(got, ref)
 
-
-def test_fft(gen):
-    x = _conj(gen, 4, 60)
-    assert torch.equal(_fft.fft(x, 1, -1), _fft.fft(_plain(x), 1, -1))
