@@ -345,15 +345,16 @@ def get_plan(nside: int, lmax: int, spin: int, precision: str = "fp64", batch: i
     import torch
 
     dev = torch.cuda.current_device()
-    plan = _plans.get((dev, nside, lmax, spin, precision))
+    key = (dev, nside, lmax, spin, precision)
+    with _plans_lock:
+        plan = _plans.get(key)
     if plan is not None and plan.max_batch >= batch:  # holds the batch: no budget to work out
         return plan
     per = workspace_bytes_per_map(nside, lmax, spin)
     if precision == "bf16x3":
         # the tensor-core path shares one recursion among the maps of a pass: hold whole
         # groups of TC_MAPS maps when device memory allows
-        cached = _plans.get((dev, nside, lmax, spin, precision))
-        if cached is None or cached.max_batch < min(batch, 64):
+        if plan is None or plan.max_batch < min(batch, 64):
             torch.cuda.empty_cache()  # a new plan: return torch's idle cached blocks first
         free, _ = torch.cuda.mem_get_info(dev)
         budget = min(64 << 30, max(free // 2, free - (24 << 30)))
@@ -365,12 +366,13 @@ def get_plan(nside: int, lmax: int, spin: int, precision: str = "fp64", batch: i
     else:
         cap = max(1, min(64, (4 << 30) // per))
     want = max(1, min(batch, cap))
-    key = (dev, nside, lmax, spin, precision)
     with _plans_lock:
         plan = _plans.get(key)
         if plan is None or plan.max_batch < want:
-            if plan is not None:
-                plan.close()
+            # the smaller plan leaves the cache first (its workspace goes with the last reference,
+            # so a thread that still launches with it keeps it): no call finds it half closed
+            plan = None
+            _plans.pop(key, None)
             plan = Plan(nside, lmax, spin, precision, max_batch=want, device=dev)
             from .autotune import lookup  # the tuned knobs of this configuration, if any
 
