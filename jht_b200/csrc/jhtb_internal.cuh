@@ -130,6 +130,7 @@ struct Plan {
     double2 *d_tw;      // [kTwLen] FFT pass twiddles (tw_offset)
     double2 *d_bh;      // chirp spectra, FFT_P(conj(w))/P, per distinct chirp length
     double2 *d_ctab;    // chirp, piece and ring-phase factors per distinct chirp length
+    long long bh_len, ctab_len;  // entries of the two
     double2 *d_belt;    // [2 belt_n] e^{i pi a / belt_n} of a power-of-two belt
     int belt_n;         // points of the belt rings where they run as power-of-two FFTs, else 0
 

@@ -612,6 +612,8 @@ int build_plan(Plan *p, const jhtb_host_tables *ht) {
             co += (long long)kRingCols * i;
             bo += 1LL << lg;
         }
+        p->bh_len = bo;
+        p->ctab_len = co;
         p->h_ring_n.resize(nr);
         for (int r = 0; r < nr; ++r) {
             RingDesc &d = rings[r];

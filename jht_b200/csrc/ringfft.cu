@@ -188,7 +188,9 @@ struct Fft {
     template <int PASS, bool PLUS>
     static __device__ __forceinline__ void twiddle(double2 (&v)[16], int t, const double2 *__restrict__ tw) {
         constexpr int BLOG = LOGP - 4 * PASS, SLOG = BLOG - 4;
-        const double2 *T = tw + tw_offset(BLOG) + 4 * (t & ((1 << SLOG) - 1));  // e^{-2 pi i j {1, 4, 8, 12} / B}
+        const int at = tw_offset(BLOG) + 4 * (t & ((1 << SLOG) - 1));
+        if (!JHTB_IN(at + 3, kTwLen, 107)) return;
+        const double2 *T = tw + at;  // e^{-2 pi i j {1, 4, 8, 12} / B}
         const double2 w1 = __ldg(&T[0]);
         const double2 w2 = cmul(w1, w1), w3 = cmul(w2, w1);
         v[1] = PLUS ? cmulc(v[1], w1) : cmul(v[1], w1);
@@ -207,12 +209,13 @@ struct Fft {
     template <int PASS>
     static __device__ __forceinline__ void put(const double2 (&v)[16], double2 *buf, int t) {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) buf[pos<PASS>(t, q)] = v[q];
+        for (int q = 0; q < 16; ++q)
+            if (JHTB_IN(pos<PASS>(t, q), LEN, 106)) buf[pos<PASS>(t, q)] = v[q];
     }
     template <int PASS>
     static __device__ __forceinline__ void get(double2 (&v)[16], const double2 *buf, int t) {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) v[q] = buf[pos<PASS>(t, q)];
+        for (int q = 0; q < 16; ++q) v[q] = JHTB_IN(pos<PASS>(t, q), LEN, 106) ? buf[pos<PASS>(t, q)] : zero2();
     }
     // forward, e^{+}: v[q] = x[t + TP q] in, v[g RLAST + q] = X[out_index(t, g RLAST + q)] out.
     // The buffer must be free on entry; `on` is false for idle threads, which only meet the barriers.
@@ -326,6 +329,7 @@ struct RingArgs {
     const double2 *tw;     // twiddles of the FFT passes (tw_offset)
     const double2 *bh;     // chirp spectra
     const double2 *ctab;   // per chirp length i: kRingCols columns of i factors
+    long long bh_len, ctab_len;
     const double2 *belt;   // e^{i pi a / Nb}, a < 2 Nb, of the power-of-two belt
     int belt_n;            // Nb
 };
@@ -396,15 +400,24 @@ __device__ __forceinline__ void gather_orders(double2 *Pr, double2 *Mr, bool sto
     }
 }
 
+// a staged point in a unit's `len` slots of shared memory
+__device__ __forceinline__ double2 staged(const double2 *buf, int i, int len) { return JHTB_IN(i, len, 106) ? buf[i] : zero2(); }
+__device__ __forceinline__ void stage(double2 *buf, int i, int len, double2 v) {
+    if (JHTB_IN(i, len, 106)) buf[i] = v;
+}
+// factor k of a chirp length's column that starts at table entry `col`
+__device__ __forceinline__ double2 chirp_factor(const RingArgs &a, long long col, int k) {
+    return JHTB_IN(col + k, a.ctab_len, 110) ? __ldg(&a.ctab[col + k]) : zero2();
+}
+
 __device__ __forceinline__ double2 load_pixel(const double *map, const Streams &s, long long npix, int nstream, int j) {
     const double x = JHTB_IN(s.offX + j, npix * nstream, 103) ? map[s.offX + j] : 0.0;
-    const double y = s.offY >= 0 ? map[s.offY + j] : 0.0;
+    const double y = s.offY >= 0 && JHTB_IN(s.offY + j, npix * nstream, 103) ? map[s.offY + j] : 0.0;
     return make_double2(x, y);
 }
 __device__ __forceinline__ void store_pixel(double *map, const Streams &s, long long npix, int nstream, int j, double2 v) {
-    if (!JHTB_IN(s.offX + j, npix * nstream, 104)) return;
-    map[s.offX + j] = v.x;
-    if (s.offY >= 0) map[s.offY + j] = v.y;
+    if (JHTB_IN(s.offX + j, npix * nstream, 104)) map[s.offX + j] = v.x;
+    if (s.offY >= 0 && JHTB_IN(s.offY + j, npix * nstream, 104)) map[s.offY + j] = v.y;
 }
 
 // ---------------------------------------------------------------------------------
@@ -451,10 +464,10 @@ __device__ __forceinline__ void direct_unit(const RingArgs &a, const RingUnit &u
 #pragma unroll 1
                     for (int k2 = 1; k2 < Q; ++k2)
                         d = cadd(d, cmul(fold_sum(Pr, Mr, k1 + X::P * k2, N, a.lmax, sh), root8((4 / Q) * c * k2)));
-                    fb[X::template pos<0>(t, q)] = d;
+                    stage(fb, X::template pos<0>(t, q), X::LEN, d);
                 }
 #pragma unroll
-                for (int q = 0; q < 16; ++q) v[q] = fb[X::template pos<0>(t, q)];
+                for (int q = 0; q < 16; ++q) v[q] = staged(fb, X::template pos<0>(t, q), X::LEN);
             }
             if (c) {
 #pragma unroll
@@ -515,7 +528,7 @@ __device__ __forceinline__ void chirp_unit(const RingArgs &a, const RingUnit &u,
     const Streams st = streams_of(a, r, rd);
     const int N = rd.N, i = N >> 2, nstream = a.spin ? 2 : 1;
     const bool sh = rd.shifted;
-    const double2 *ct = a.ctab + rd.ctab_off;
+    constexpr int RB = PPC * X::LEN;  // slots of one ring
     double2 *rb = buf + g * PPC * X::LEN;  // this ring's part of the buffer
     const double2 *Pr = F + st.rowP, *Mr = F + st.rowM;
     // e^{i pi k2 / 4}: the part of the ring phase that depends on the quarter
@@ -530,7 +543,7 @@ __device__ __forceinline__ void chirp_unit(const RingArgs &a, const RingUnit &u,
             if (!ADJ && N <= a.lmax) {
 #pragma unroll 1
                 for (int k = tg; k < N; k += GT)
-                    rb[k] = quarter(fold_sum(Pr, Mr, k, N, a.lmax, sh), (k >= i) + (k >= 2 * i) + (k >= 3 * i));
+                    stage(rb, k, RB, quarter(fold_sum(Pr, Mr, k, N, a.lmax, sh), (k >= i) + (k >= 2 * i) + (k >= 3 * i)));
             } else for (int k0 = tg; k0 < N; k0 += U * GT) {
                 double2 d[U];
                 if (ADJ) {
@@ -545,14 +558,14 @@ __device__ __forceinline__ void chirp_unit(const RingArgs &a, const RingUnit &u,
 #pragma unroll
                 for (int e = 0; e < U; ++e) {
                     const int k = k0 + e * GT;
-                    if (k < N) rb[k] = quarter(d[e], (k >= i) + (k >= 2 * i) + (k >= 3 * i));
+                    if (k < N) stage(rb, k, RB, quarter(d[e], (k >= i) + (k >= 2 * i) + (k >= 3 * i)));
                 }
             }
         }
         __syncthreads();
     }
     double2 v[16];
-    const double2 *win = ct + (ADJ ? (size_t)(kColAdjIn + s) : (size_t)((sh ? kColSynth : kColAdjIn) + s)) * i;
+    const long long win = rd.ctab_off + (ADJ ? (long long)(kColAdjIn + s) : (long long)((sh ? kColSynth : kColAdjIn) + s)) * i;
     double2 *fb = rb + (tg / X::TP) * X::LEN;
     if (on) {
         const bool odd = s & 1;
@@ -577,7 +590,7 @@ __device__ __forceinline__ void chirp_unit(const RingArgs &a, const RingUnit &u,
                     else if (k2 == 1) d[1] = f;
                     else d[0] = f;
                 }
-                fb[X::template pos<0>(t, q)] = combine(d);
+                stage(fb, X::template pos<0>(t, q), X::LEN, combine(d));
             }
         }
 #pragma unroll
@@ -586,19 +599,19 @@ __device__ __forceinline__ void chirp_unit(const RingArgs &a, const RingUnit &u,
             if (k1 < i) {
                 double2 x;
                 if (PPC == 1 && !ADJ && N <= a.lmax) {
-                    x = fb[X::template pos<0>(t, q)];
+                    x = staged(fb, X::template pos<0>(t, q), X::LEN);
                 } else {
                     double2 d[4];
 #pragma unroll
                     for (int k2 = 0; k2 < 4; ++k2) {
                         const int k = k1 + i * k2;
-                        if (PPC >= 2) d[k2] = rb[k];
+                        if (PPC >= 2) d[k2] = staged(rb, k, RB);
                         else if (ADJ) d[k2] = conjd(load_pixel(in, st, a.npix, nstream, k));
                         else d[k2] = quarter(fold_one(Pr, Mr, k, N, a.lmax, sh), k2);
                     }
                     x = combine(d);
                 }
-                v[q] = cmul(x, __ldg(&win[k1]));
+                v[q] = cmul(x, chirp_factor(a, win, k1));
             } else {
                 v[q] = zero2();
             }
@@ -607,13 +620,15 @@ __device__ __forceinline__ void chirp_unit(const RingArgs &a, const RingUnit &u,
     if (PPC >= 2) __syncthreads();  // the staged points are read: the buffer is free
     X::template forward<true>(v, fb, t, on, a.tw);
     if (on) {
-        const double2 *B = a.bh + rd.bh_off;
 #pragma unroll
-        for (int q = 0; q < 16; ++q) v[q] = cmul(v[q], __ldg(&B[X::out_index(t, q)]));
+        for (int q = 0; q < 16; ++q) {
+            const long long b = rd.bh_off + X::out_index(t, q);
+            v[q] = cmul(v[q], JHTB_IN(b, a.bh_len, 108) ? __ldg(&a.bh[b]) : zero2());
+        }
     }
     X::backward(v, fb, t, on, a.tw);
     // y[j] times the last chirp factor: pixel 4 j + s, or conj -> W'[4 j + s]
-    const double2 *wout = ct + (ADJ ? (size_t)(sh ? kColAdjOut + s : kColAdjIn) : (size_t)kColAdjIn) * i;
+    const long long wout = rd.ctab_off + (ADJ ? (long long)(sh ? kColAdjOut + s : kColAdjIn) : (long long)kColAdjIn) * i;
     if (PPC == 4) {
         __syncthreads();  // every thread has read its last points
         if (on) {
@@ -621,18 +636,18 @@ __device__ __forceinline__ void chirp_unit(const RingArgs &a, const RingUnit &u,
             for (int q = 0; q < 8; ++q) {
                 const int j = t + X::TP * q;
                 if (j < i) {
-                    const double2 w = cmul(v[q], __ldg(&wout[j]));
-                    rb[s * cs + j] = ADJ ? conjd(w) : w;
+                    const double2 w = cmul(v[q], chirp_factor(a, wout, j));
+                    stage(rb, s * cs + j, RB, ADJ ? conjd(w) : w);
                 }
             }
         }
         __syncthreads();
         if (!on) return;
         if (!ADJ) {
-            for (int j = tg; j < N; j += GT) store_pixel(out, st, a.npix, nstream, j, rb[(j & 3) * cs + (j >> 2)]);
+            for (int j = tg; j < N; j += GT) store_pixel(out, st, a.npix, nstream, j, staged(rb, (j & 3) * cs + (j >> 2), RB));
         } else {
             gather_orders(V + st.rowP, V + st.rowM, st.rowM != st.rowP, N, a.lmax, sh, tg, GT,
-                          [&](int k) { return rb[(k & 3) * cs + (k >> 2)]; });
+                          [&](int k) { return staged(rb, (k & 3) * cs + (k >> 2), RB); });
         }
         return;
     }
@@ -641,7 +656,7 @@ __device__ __forceinline__ void chirp_unit(const RingArgs &a, const RingUnit &u,
     for (int q = 0; q < 8; ++q) {
         const int j = t + X::TP * q;
         if (j >= i) continue;
-        const double2 w = cmul(v[q], __ldg(&wout[j]));
+        const double2 w = cmul(v[q], chirp_factor(a, wout, j));
         if (!ADJ) store_pixel(out, st, a.npix, nstream, 4 * j + s, w);
         else scatter_orders(V + st.rowP, V + st.rowM, st.rowM != st.rowP, conjd(w), 4 * j + s, N, a.lmax, sh);
     }
@@ -686,7 +701,7 @@ __device__ __forceinline__ void small_unit(const RingArgs &a, const RingUnit &u,
         int idx = (int)((long long)step1 * p % n2);
         const int step = (int)((long long)step1 * parts % n2);
         for (int e = p; e < N; e += parts) {
-            const double2 d = D[e], w = root[idx];
+            const double2 d = staged(D, e, kSmallRing), w = staged(root, idx, 2 * kSmallRing);
             acc.x = fma(d.x, w.x, fma(-d.y, w.y, acc.x));
             acc.y = fma(d.x, w.y, fma(d.y, w.x, acc.y));
             idx += step;
@@ -703,7 +718,7 @@ __device__ __forceinline__ void small_unit(const RingArgs &a, const RingUnit &u,
     }
     if (!ADJ) return;
     __syncthreads();
-    gather_orders(V + st.rowP, V + st.rowM, st.rowM != st.rowP, N, a.lmax, sh, threadIdx.x, NT, [&](int q) { return D[q]; });
+    gather_orders(V + st.rowP, V + st.rowM, st.rowM != st.rowP, N, a.lmax, sh, threadIdx.x, NT, [&](int q) { return staged(D, q, kSmallRing); });
 }
 
 template <bool ADJ>
@@ -828,6 +843,8 @@ RingArgs make_args(const Plan &p) {
     a.tw = p.d_tw;
     a.bh = p.d_bh;
     a.ctab = p.d_ctab;
+    a.bh_len = p.bh_len;
+    a.ctab_len = p.ctab_len;
     a.belt = p.d_belt;
     a.belt_n = p.belt_n;
     return a;
