@@ -262,7 +262,8 @@ __global__ void __launch_bounds__(kNuThreads) spread_kernel(const double2 *__res
 // additions to the grid are now the larger part, and three CTAs an SM hide only some of their
 // latency: two took 1561 us, four, with spills, 1240 us).  Adding the windows
 // into shared memory took 392 shared FP64 atomics per point (compare-and-swap loops).  A point whose
-// window leaves the block (a coordinate outside the tile its key named) is added straight to the grid.
+// window leaves the block (it lies in another tile than its segment's, whole periods aside) and
+// one with an infinite or NaN value is added straight to the grid.
 constexpr int kTile = 32;
 constexpr int kSpreadThreads = 256;
 constexpr int kSpreadPts = 32;                    // points staged per round
@@ -327,9 +328,12 @@ __global__ void __launch_bounds__(kSpreadThreads, 3) spread_tiles_kernel(
             const double fk = ceil(uk - 0.5 * W), fm = ceil(um - 0.5 * W);
             const long long k0 = (fk > -4.0e18 && fk < 4.0e18) ? (long long)fk : 0;
             const long long m0 = (fm > -4.0e18 && fm < 4.0e18) ? (long long)fm : 0;
-            const long long bk = k0 - k_org, bm = m0 - m_org;
+            // a coordinate outside [0, 2 pi) lies whole periods from the tile that its key named
+            long long bk = k0 - k_org, bm = m0 - m_org;
+            if (bk < 0 || bk + W > B) bk = wrap(bk, nk);
+            if (bm < 0 || bm + W > B) bm = wrap(bm, nm);
             // an infinite value would reach the block's other cells as 0 x inf
-            if (bk >= 0 && bk + W <= B && bm >= 0 && bm + W <= B && isfinite(v.x) && isfinite(v.y)) {
+            if (bk + W <= B && bm + W <= B && isfinite(v.x) && isfinite(v.y)) {
                 mask = (2u << (bk + W - 1) / 8) - (1u << bk / 8) | ((2u << (bm + W - 1) / 4) - (1u << bm / 4)) << 6;
                 for (int a = sub; a < W; a += 8) {
                     sa[pt][bk + a] = window_at<W>(uk, fk, a, beta);
@@ -337,11 +341,15 @@ __global__ void __launch_bounds__(kSpreadThreads, 3) spread_tiles_kernel(
                     *reinterpret_cast<double2 *>(&sb[pt][2 * (bm + a)]) = make_double2(wm * v.x, wm * v.y);
                 }
             } else {
+                // the point's column weights once, in its own staged row: its row weights stay
+                // zero, so nothing of them reaches the products
+                for (int b = sub; b < W; b += 8) sb[pt][b] = window_at<W>(um, fm, b, beta);
+                __syncwarp(0xffu << (lane & 24));  // the point's eight threads, which all came this way
                 for (int a = sub; a < W; a += 8) {
                     double *row = reinterpret_cast<double *>(grid + (size_t)wrap(k0 + a, nk) * nm);
                     const double wk = window_at<W>(uk, fk, a, beta);
                     for (int b = 0; b < W; ++b) {
-                        const double wm = window_at<W>(um, fm, b, beta);
+                        const double wm = sb[pt][b];
                         const int mi = wrap(m0 + b, nm);
                         atomicAdd(row + 2 * mi, wm * (wk * v.x));
                         atomicAdd(row + 2 * mi + 1, wm * (wk * v.y));
