@@ -1073,9 +1073,14 @@ int launch_seg_states(const Plan &p, cudaStream_t s) {
 // (1028 items), nside 256 / lmax 512 spin 0 53 -> 30 (2052), spin 2 86 -> 73 (4104), but nside 400 /
 // lmax 800 spin 0 103 -> 113 (5607).  Adjoint nside 128 spin 2 78 -> 22 (514), nside 300 / lmax 641
 // spin 2 356 -> 179 (3210), nside 512 / lmax 1024 spin 0 288 -> 256 and spin 2 657 -> 615 (8200), but
-// nside 1024 / lmax 2048 spin 2 4073 -> 4179 (32784).
-static bool small_synth(const Plan &p, int nb) { return (long long)nb * p.M * p.ntiles <= kSmallSynthItems; }
-static bool small_adj(const Plan &p, int nb) { return p.d_sg_st && (long long)nb * p.M * p.a_ntiles <= kSmallAdjItems; }
+// nside 1024 / lmax 2048 spin 2 4073 -> 4179 (32784).  A tuned CTA count is one of the plain forms'
+// persistent grids.
+static bool small_synth(const Plan &p, int nb) {
+    return p.leg_ctas == 0 && (long long)nb * p.M * p.ntiles <= kSmallSynthItems;
+}
+static bool small_adj(const Plan &p, int nb) {
+    return p.leg_ctas == 0 && p.d_sg_st && (long long)nb * p.M * p.a_ntiles <= kSmallAdjItems;
+}
 
 // Several maps share one recursion on the matrix unit (legendre_batch.cu, with the rule); a
 // left-over single map, and batches below one wave of items, run here.

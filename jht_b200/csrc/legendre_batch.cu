@@ -512,12 +512,13 @@ BatchParams make_batch(const Plan &p, bool paired) {
     return q;
 }
 
-// persistent grid: the resident CTAs, or fewer where the items do not fill them
+// persistent grid: the resident CTAs or the plan's tuned count, or fewer where the items do not fill them
 template <typename K>
-int batch_grid(K k, int threads, int smem, long long items, int *grid) {
+int batch_grid(const Plan &p, K k, int threads, int smem, long long items, int *grid) {
     JHTB_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads, smem) != cudaSuccess || n < 1) n = 1;
+    if (p.leg_ctas > 0) n = std::min(n, p.leg_ctas);
     *grid = (int)std::max<long long>(1, std::min<long long>((long long)n * sm_count(), items));
     return JHTB_OK;
 }
@@ -528,7 +529,7 @@ int synth_groups(const Plan &p, BatchParams q, const double2 *alm, double2 *F, i
     auto k = synth_batch_kernel<SPIN, NB>;
     const int smem = (int)sizeof(SynSmem<SPIN, NB>), groups = (nb + MAPS - 1) / MAPS;
     int rc, grid;
-    if ((rc = batch_grid(k, kSynWarps * 32, smem, (long long)q.nitems * groups, &grid))) return rc;
+    if ((rc = batch_grid(p, k, kSynWarps * 32, smem, (long long)q.nitems * groups, &grid))) return rc;
     JHTB_CUDA_TRY(cudaMemsetAsync(p.d_counter, 0, sizeof(unsigned), s));
     k<<<grid, kSynWarps * 32, smem, s>>>(q, alm, F, nb, groups);
     JHTB_CUDA_TRY(cudaGetLastError());
@@ -541,7 +542,7 @@ int adj_groups(const Plan &p, BatchParams q, const double2 *V, double2 *part, in
     auto k = adj_batch_kernel<SPIN, NB>;
     const int smem = (int)sizeof(AdjBSmem<SPIN, NB>), groups = (nb + MAPS - 1) / MAPS;
     int rc, grid;
-    if ((rc = batch_grid(k, kAdjWarps * 32, smem, (long long)q.nitems * groups, &grid))) return rc;
+    if ((rc = batch_grid(p, k, kAdjWarps * 32, smem, (long long)q.nitems * groups, &grid))) return rc;
     JHTB_CUDA_TRY(cudaMemsetAsync(p.d_counter, 0, sizeof(unsigned), s));
     k<<<grid, kAdjWarps * 32, smem, s>>>(q, V, part, nb, groups);
     JHTB_CUDA_TRY(cudaGetLastError());
