@@ -267,7 +267,8 @@ int jhtb_plan_set_watchdog(jhtb_plan *plan, int64_t timeout_ns);
  *   JHTB_TUNE_TCA_FOLD  rings per FP32 accumulation block of the tensor-core adjoint
  *                       (multiple of 32, default 256);
  *   JHTB_TUNE_TC_GROUP  maps per tensor-core synthesis group, 8 or 16 (default 16);
- *   JHTB_TUNE_LEG_CTAS  CTAs per SM of the FP64 Legendre kernels, 0 = all that fit (default). */
+ *   JHTB_TUNE_LEG_CTAS  CTAs per SM of the FP64 Legendre kernels, 0 = all that fit (default; a set
+ *                       count also keeps small problems on the persistent kernels). */
 #define JHTB_TUNE_TC_FOLD 1
 #define JHTB_TUNE_TCA_FOLD 2
 #define JHTB_TUNE_TC_GROUP 3

@@ -335,6 +335,8 @@ _plans_lock = threading.Lock()
 
 
 def workspace_bytes_per_map(nside: int, lmax: int, spin: int) -> int:
+    """What a map takes while it is transformed: ring spectra, four partial coefficient rows and
+    twice its pixels (an allowance for the caller's maps); the plan's own tables are not in it."""
     ncomp = 1 if spin == 0 else 2
     K = (lmax + 1) * (lmax + 2) // 2
     return 16 * (ncomp * (4 * nside - 1) * (lmax + 1) + 2 * 12 * nside * nside + 4 * ncomp * K)

@@ -3,8 +3,8 @@
 // A plan holds, on the device, everything that depends only on (nside, lmax,
 // spin): the RING geometry (jht healpix.py:107-140), per-m recursion seeds
 // (_recursion.py:53-56, :166-188), the normalised three-term recursion
-// coefficients, the per-ring FFT descriptors with Bluestein chirp spectra, and
-// the ring-spectrum workspace.  It replaces jht's lru-cached _prepare
+// coefficients, the ring descriptors and work units with the chirp spectra and factors
+// of each distinct ring length, and the ring-spectrum workspace.  It replaces jht's lru-cached _prepare
 // (healpix.py:184-357), which builds the same information as NumPy constants.
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>

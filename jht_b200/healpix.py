@@ -291,7 +291,9 @@ def adjoint_synthesis(m, nside: int, lmax: int, spin: int = 0, *, precision: str
 def synthesis_batch(alm, nside: int, lmax: int, spin: int = 0, *, precision: str = "fp64") -> torch.Tensor:
     """Batched :func:`synthesis`: alm ``(B, K)`` or ``(B, 2, K)`` -> ``(B, Npix)`` / ``(B, 2, Npix)``.
 
-    One launch for the whole batch (jht reaches the same result with ``jax.vmap``).
+    One call for the whole batch (jht reaches the same result with ``jax.vmap``).  Large FP64
+    batches share one recursion per group of maps, so a map's last bits can differ from
+    :func:`synthesis` of that map alone, and with its place in the batch.
     """
     a = _as_alm(alm)
     K = alm_size(lmax)
