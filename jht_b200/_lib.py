@@ -348,8 +348,7 @@ def get_plan(nside: int, lmax: int, spin: int, precision: str = "fp64", batch: i
 
     dev = torch.cuda.current_device()
     key = (dev, nside, lmax, spin, precision)
-    with _plans_lock:
-        plan = _plans.get(key)
+    plan = _plans.get(key)  # no lock: a plan in the cache is open, and stays so while it is referenced
     if plan is not None and plan.max_batch >= batch:  # holds the batch: no budget to work out
         return plan
     per = workspace_bytes_per_map(nside, lmax, spin)
@@ -387,9 +386,7 @@ def get_plan(nside: int, lmax: int, spin: int, precision: str = "fp64", batch: i
 
 def clear_plans() -> None:
     with _plans_lock:
-        for p in _plans.values():
-            p.close()
-        _plans.clear()
+        _plans.clear()  # each is closed with its last reference
 
 
 def dense(t):

@@ -93,3 +93,13 @@ def test_a_failed_creation_leaves_no_closed_plan(cache):
         _lib.get_plan(*KEY, batch=4)
     FakePlan.fail = False
     assert _lib.get_plan(*KEY, batch=1).handle is not None
+
+
+def test_clearing_the_cache_leaves_a_plan_in_use_open(cache):
+    held, _ = _lib.get_plan(*KEY, batch=1), _lib.get_plan(16, 24, 0, "fp64")
+    del _
+    _lib.clear_plans()
+    assert FakePlan.closed == 1 and held.handle is not None
+    assert _lib.get_plan(*KEY, batch=1) is not held
+    del held
+    assert FakePlan.closed == 2
