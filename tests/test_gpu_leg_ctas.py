@@ -36,6 +36,8 @@ def _legendre_grids(call, path):
         call()
     p.export_chrome_trace(str(path))
     kernels = [e for e in json.loads(path.read_text())["traceEvents"] if e.get("cat") == "kernel"]
+    if not kernels:
+        pytest.skip("no kernel trace on this machine")
     return [e["args"]["grid"][0] for e in kernels if any(k in e["name"] for k in (
         "synth0_kernel", "synth2_kernel", "synth_batch_kernel", "adj0_kernel", "adj2_kernel", "adj_batch_kernel"))]
 
